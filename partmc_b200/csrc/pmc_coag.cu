@@ -1905,7 +1905,7 @@ void launch_pp(Ctx& c, int kt, long long Q, bool grouped) {
   }
   with_kt(c, kt, [&](auto ktc, auto) {
     constexpr int KT = decltype(ktc)::value;
-    k_pp_ops<KT><<<blocks, 128, 0, c.stream>>>(c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p,
+    k_pp_ops<KT><<<grid_for(32 * Q, 32 * kPPWarps), 32 * kPPWarps, 0, c.stream>>>(c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p,
                                                c.op_key.p, c.n_dev.p + 0, c.pp_res.p, c.pp_vol.p, c.pp_rm_off.p,
                                                c.pp_rm_pool.p, (long long)c.pp_rm_pool.n);
   });
