@@ -14,7 +14,7 @@ OUT = os.path.join(HERE, "libpmc_coag_gpu.so")
 BUILD = os.path.join(HERE, "_build")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"] + ARCH
+COMMON = ["-std=c++17", "-O3", "--split-compile=0", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"] + ARCH
 
 UNITS = [
     ("pmc_coag.cu", []),
