@@ -2087,14 +2087,13 @@ __global__ void k_step_reset(PopCtr* ctrs, int n_pop) {
   ctrs[k].cap_site = 0;
 }
 
+// every slot, those above n_slots included: a slot that an earlier, larger
+// population used keeps its claim word, and a word of an old generation is
+// below every word of a restarted one
 __global__ void k_fill_claims(const PopDev* pops) {
   const PopDev& P = pops[blockIdx.y];
-  int n = P.ctr->n_slots;
-  if (n > P.cap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) bad_index(P.ctr, kBadSlotCount, n);
-    n = P.cap;
-  }
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  if (P.ctr->n_slots > P.cap && blockIdx.x == 0 && threadIdx.x == 0) bad_index(P.ctr, kBadSlotCount, P.ctr->n_slots);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.cap; i += gridDim.x * blockDim.x) {
     P.claim[i] = ~0ULL;
     P.rclaim[i] = ~0ULL;
     P.touched[i] = ~0u;

@@ -77,3 +77,28 @@ def test_batched_step_graph(gpu_lib):
     assert res[0][0] == res[1][0]
     for a, b in zip(res[0][1], res[1][1]):
         same(a, b)
+
+
+def test_claim_generations_restart_after_a_smaller_upload(gpu_lib):
+    """Claim generations restart after about 2000 rounds.  A population
+    uploaded again starts with fewer slots than it ended with, so slots above
+    them hold claims of old generations when that happens; events on those
+    slots must not lose to them."""
+    import partmc_b200 as pm
+    from partmc_b200 import aero_dist
+    pop = aero_dist.brown_20spec(2500, seed=6)
+    st = pm.AeroState(pop.aero_data, pop.awa, seed=5)
+    env = pm.EnvState(288.0, 1e5)
+    first, rounds = None, 0
+    while rounds < 5000:  # at least two restarts
+        st.set_next_id(1)
+        st.add_particles(pop.vol, pop.group)
+        st.set_seed(9)
+        for _ in range(12):
+            pm.mc_coag(pm.COAG_KERNEL_TYPE_BROWN, env, pop.aero_data, st, 600.0)
+            rounds += st.stats()["rounds"]
+        got = st.particles()
+        if first is None:
+            first = got
+            assert got["id"].max() > pop.n_part  # new slots were made
+        same(first, got)
