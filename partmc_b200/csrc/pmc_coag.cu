@@ -951,7 +951,7 @@ struct Ctx {
   DevBuf<uint8_t> it_flag, it_done;
   DevBuf<unsigned long long> it_key;
   DevBuf<int2> it_c;
-  DevBuf<int> it_gp, it_len, it_head;
+  DevBuf<int> it_gp, it_len, it_head, it_start;
   DevBuf<float> it_pos;
   DevBuf<uint32_t> it_dec, it_gused;
   DevBuf<int4> it_term, ev_term;  // pending tests where chains stopped (kPendingTerm)
@@ -1754,32 +1754,67 @@ ChainPool chain_pool(Ctx& c) {
   return pool;
 }
 
+// blocks of tb threads for a warp per item of a later round, at most 2 x 256
+// threads per SM, which is what its registers let it hold (the kernels fall
+// back to a thread per item beyond that)
+int grid_warps(const Ctx& c, long long W, int tb) {
+  return (int)std::min<long long>((long long)c.n_sm * 2 * 256 / tb, std::max<long long>(1, (32 * W + tb - 1) / tb));
+}
+
 // a later round's items: the events of the round before, n_items =
 // round_dev[2] on the device, W bounds it
 void launch_items_kt(Ctx& c, int kt, bool flat, int n_gpairs, long long W, cudaStream_t st) {
   const int ti = c.tune.threads[kTuneItems], tc = c.tune.threads[kTuneChain];
-  int blocks = grid_for(W, ti);
-  const long long* n_items = c.round_dev.p + 2;
   ChainPool pool = chain_pool(c);
+  ItemArgs A;
+  A.pops = c.d_pops;
+  A.gpair_pop = c.gpair_pop.p;
+  A.gpair_local = c.gpair_local.p;
+  A.pop_pair_base = c.pop_pair_base.p;
+  A.n_gpairs = n_gpairs;
+  A.n_items = c.round_dev.p + 2;
+  A.n_items_ev = c.round_dev.p + 6;
+  A.ppw_slot = c.ppw_slot_in.p;
+  A.ppw_gp = c.ppw_gp_in.p;
+  A.op_pop = c.op_pop.p;
+  A.op_pair = c.op_pair.p;
+  A.op_slot = c.op_slot.p;
+  A.op_k = c.op_k.p;
+  A.op_key = c.op_key.p;
+  A.n_ops = c.n_dev.p;
+  A.op_cap = c.op_cap;
+  A.win = c.win_set.p;
+  A.dest = c.ev_dest.p;
+  A.ev_key = c.ev_key.p;
+  A.ev_c = c.ev_c.p;
+  A.gp_c = c.gp_c.p;
+  A.ev_pos = c.ev_pos.p;
+  A.dec = c.dec_set.p;
+  A.it_flag = c.it_flag.p;
+  A.it_key = c.it_key.p;
+  A.it_c = c.it_c.p;
+  A.it_gp = c.it_gp.p;
+  A.it_pos = c.it_pos.p;
+  A.it_len = c.it_len.p;
+  A.it_head = c.it_head.p;
+  A.it_done = c.it_done.p;
+  A.it_dec = c.it_dec.p;
+  A.it_gused = c.it_gused.p;
+  A.it_term = c.it_term.p;
+  A.start_list = c.it_start.p;
+  A.n_start = c.round_dev.p + 10;
   with_kt(c, kt, [&](auto ktc, auto tt) {
     constexpr int KT = decltype(ktc)::value;
     using T = decltype(tt);
     auto k = flat ? k_items<KT, T, true> : k_items<KT, T, false>;
     {
       TuneScope ts_items(c, kTuneItems, st);
-      k<<<blocks, ti, 0, st>>>(c.d_pops, c.gpair_pop.p, c.gpair_local.p, c.pop_pair_base.p, n_gpairs, n_items,
-                                c.round_dev.p + 6, c.ppw_slot_in.p, c.ppw_gp_in.p, c.op_pop.p, c.op_pair.p,
-                                c.op_slot.p, c.op_k.p, c.op_key.p, c.n_dev.p, c.op_cap,
-                                c.win_set.p, c.ev_dest.p, c.ev_key.p, c.ev_c.p, c.gp_c.p, c.ev_pos.p, c.dec_set.p,
-                                c.it_flag.p, c.it_key.p, c.it_c.p, c.it_gp.p, c.it_pos.p, c.it_len.p, c.it_head.p,
-                                c.it_done.p, c.it_dec.p, c.it_gused.p, c.it_term.p);
+      k<<<grid_warps(c, W, ti), ti, 0, st>>>(A);
     }
     auto kc = flat ? k_chain<KT, T, true> : k_chain<KT, T, false>;
     {
       TuneScope ts_chain(c, kTuneChain, st);
-      kc<<<grid_for(W, tc), tc, 0, st>>>(c.d_pops, c.gpair_pop.p, n_items, c.it_flag.p, c.it_key.p, c.it_c.p,
-                                           c.it_gp.p, c.it_pos.p, c.it_dec.p, c.it_gused.p, pool, c.it_len.p,
-                                           c.it_head.p, c.it_done.p, c.it_term.p);
+      kc<<<grid_warps(c, W, tc), tc, 0, st>>>(A, pool);
     }
   });
   note_launch();
@@ -2141,6 +2176,7 @@ __global__ void k_round_begin(uint32_t* d_round, long long* round_dev, int* per_
     round_dev[4] = 0;
     round_dev[5] = 0;
     round_dev[8] = 0;
+    round_dev[10] = 0;
   }
   for (int k = threadIdx.x; k < n_per_pop; k += blockDim.x) per_pop[k] = 0;
 }
@@ -2197,7 +2233,7 @@ __global__ void k_step_begin(PopDev* pops, PopCtr* ctrs, int n_pop, uint32_t* d_
     pops[i].step += 1u;
   }
   if (i < 4 * n_pop) per_pop[i] = 0;
-  if (i < 10) round_dev[i] = 0;
+  if (i < 12) round_dev[i] = 0;
   if (i < kStatWords) stat[i] = 0;
   const int gp = (int)pop_pair_base[n_pop] + i;  // the places past the last pair
   if (gp < n_gp) nwork_set[gp] = nwork_pp[gp] = 0;
@@ -2383,7 +2419,7 @@ std::vector<long long> round_graph_key(const Ctx& c, const RoundBounds& b) {
           (long long)c.ev_pos.p, (long long)c.ev_dest.p, (long long)c.ev_len.p, (long long)c.ev_head.p,
           (long long)c.ev_app.p, (long long)c.ev_done.p, (long long)c.chain_list.p, (long long)c.it_flag.p, (long long)c.it_key.p,
           (long long)c.it_c.p, (long long)c.it_gp.p, (long long)c.it_pos.p, (long long)c.it_len.p,
-          (long long)c.it_head.p, (long long)c.it_done.p, (long long)c.it_dec.p, (long long)c.it_gused.p, (long long)c.it_off.p,
+          (long long)c.it_head.p, (long long)c.it_start.p, (long long)c.it_done.p, (long long)c.it_dec.p, (long long)c.it_gused.p, (long long)c.it_off.p,
           (long long)c.it_term.p, (long long)c.ev_term.p, (long long)c.ppw_slot.p, (long long)c.ppw_gp.p,
           (long long)c.ch_y.p,
           (long long)c.ch_q.p, (long long)c.ch_pos.p, (long long)c.need_slot_set.p, (long long)c.need_id_set.p,
@@ -2446,7 +2482,7 @@ bool events_fit(const Ctx& c, long long W) {
 void reserve_round(Ctx& c, long long W) {
   size_t w = (size_t)std::max<long long>(W, 1);
   c.it_flag.reserve(w + 1); c.it_key.reserve(w + 1); c.it_c.reserve(w + 1); c.it_gp.reserve(w + 1);
-  c.it_pos.reserve(w + 1); c.it_len.reserve(w + 1); c.it_head.reserve(w + 1); c.it_done.reserve(w + 1);
+  c.it_pos.reserve(w + 1); c.it_len.reserve(w + 1); c.it_head.reserve(w + 1); c.it_done.reserve(w + 1); c.it_start.reserve(w + 1);
   c.it_dec.reserve(w + 1); c.it_gused.reserve(w + 1); c.it_term.reserve(w + 1);
   c.it_off.reserve(w + 2);
 }
@@ -2883,8 +2919,9 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
   c.n_dev.reserve(4 + 2 * (size_t)c.n_pop);
   // round_dev: [0] losers, [1] events, [2] items, [3] chain chunks, [4] chains,
   // [5] walkers of target operations, [6] items that are events, [7] items
-  // that are such walkers, [8] target operations that lost a claim
-  c.round_dev.reserve(10);
+  // that are such walkers, [8] target operations that lost a claim,
+  // [9] places of their walkers, [10] chains that k_chain carries on
+  c.round_dev.reserve(12);
   int max_pairs = 1, nb_max = 1, max_cap = 1;
   for (int k = 0; k < c.n_pop; k++) {
     max_pairs = std::max(max_pairs, c.pops[k].h.n_pairs);
@@ -3007,7 +3044,7 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
     c.lost_off.reserve(Q + 2); c.rank_slot_pp.reserve(Q + 2); c.rank_id_pp.reserve(Q + 2);
   }
   if (c.dirty) push_pops(c);
-  CK(cudaMemsetAsync(c.round_dev.p, 0, sizeof(long long) * 10, c.stream));
+  CK(cudaMemsetAsync(c.round_dev.p, 0, sizeof(long long) * 12, c.stream));
   CK(cudaMemsetAsync(c.per_pop_i.p, 0, sizeof(int) * 4 * c.n_pop, c.stream));
   if (W > 0) {
     ProfScope ps(c, 0, W);
@@ -3306,7 +3343,7 @@ int pmc_coag_gpu_destroy(pmc_coag_gpu_ctx* x) {
   DevBuf<int>* bi[] = {&c.gpair_pop, &c.gpair_local, &c.need_slot_set, &c.need_id_set, &c.need_slot_pp,
                        &c.need_id_pp, &c.lost_pp, &c.op_pop, &c.op_pair, &c.op_slot, &c.op_k, &c.r_pop,
                        &c.r_pair, &c.r_slot, &c.r_k, &c.per_pop_i, &c.slot_base_set, &c.slot_base_pp,
-                       &c.ev_dest, &c.ev_len, &c.ev_head, &c.ev_app, &c.it_gp, &c.it_len, &c.it_head,
+                       &c.ev_dest, &c.ev_len, &c.ev_head, &c.ev_app, &c.it_gp, &c.it_len, &c.it_head, &c.it_start,
                        &c.ch_y, &c.ch_q};
   for (auto* b : bi) b->release();
   DevBuf<long long>* bl[] = {&c.pop_pair_base, &c.nwork_set, &c.nwork_pp, &c.work_off, &c.pp_off, &c.flag_off,

@@ -147,8 +147,10 @@ __device__ int block_excl_scan(int v, int* total) {
   return pre;
 }
 
-// pair-test record of a particle of radius r, total volume v, mass m and
-// class cls (1-based) (see RecD)
+// pair-test record of a particle of radius r (vol2rad(v)), total volume v,
+// mass m and class cls (1-based) (see RecD).  A sphere's mobility radius is r:
+// taking it saves two of the record's three FP64 pow calls, each about half a
+// microsecond where one thread's chain of merges waits for it.
 __device__ __forceinline__ RecD make_rec_v(const PopDev& P, double r, double v, double m, int cls) {
   RecD q;
   const Fractal& F = P.benv.frac;
@@ -160,13 +162,13 @@ __device__ __forceinline__ RecD make_rec_v(const PopDev& P, double r, double v, 
   switch (P.kernel_type) {
     case kKernelAdditive: q.a = v; break;
     case kKernelBrown: {
-      BrownPart bp = brown_part(P.benv, v, m / v, &ok);
+      BrownPart bp = brown_part(P.benv, r, v, m / v, &ok);
       q.a = bp.diffus;
       q.b = bp.speedsq;
       q.c = bp.deltasq;
       break;
     }
-    case kKernelSedi: q.a = fall_g(mobility_rad(F, v, P.benv.fp, &ok)); break;
+    case kKernelSedi: q.a = fall_g(F.spherical ? r : mobility_rad(F, v, P.benv.fp, &ok)); break;
     case kKernelBrownFree: {
       q.a = v;
       q.b = m / v;
@@ -602,21 +604,24 @@ __device__ __forceinline__ bool f32_decides(float pf, double u) {
 }
 
 // u < k / k_max in FP64 from the slots' FP64 records, for the pair p's
-// orientation (first cell's particle first); counts k > k_max as the
-// reference's warn_assert_msg does (coagulation.F90:749-751)
+// orientation (first cell's particle first); *warn if k > k_max, which the
+// reference warns of (warn_assert_msg, coagulation.F90:749-751)
 template <int KT, bool FLAT>
 __device__ __forceinline__ bool accept_f64_rec(const PopDev& P, const RecD& a, const RecD& b, const PairDesc& d,
-                                               int cc, double fflat, double inv_k_max, double u) {
+                                               int cc, double fflat, double inv_k_max, double u, bool* warn) {
   const double k = pair_kernel<KT, double, FLAT>(P, (const double*)&a, (const double*)&b, d.c1, d.c2, cc, fflat,
                                                  P.coeff);
   const double prob = k * inv_k_max;
-  if (!(prob <= 1.0)) add_ll(&P.ctr->kmax_warn, 1LL);
+  *warn = !(prob <= 1.0);
   return u < prob;
 }
 template <int KT, bool FLAT>
 __device__ __forceinline__ bool accept_f64(const PopDev& P, int s1, int s2, const PairDesc& d, const PairState& S,
                                            double u) {
-  return accept_f64_rec<KT, FLAT>(P, P.recd[s1], P.recd[s2], d, S.cc, S.fflat, S.inv_k_max, u);
+  bool warn;
+  const bool acc = accept_f64_rec<KT, FLAT>(P, P.recd[s1], P.recd[s2], d, S.cc, S.fflat, S.inv_k_max, u, &warn);
+  if (warn) add_ll(&P.ctr->kmax_warn, 1LL);
+  return acc;
 }
 
 __device__ __forceinline__ int find_pair(const long long* off, int n, long long w) {
@@ -636,14 +641,32 @@ struct MergeDecision {
   int new_group;  // 1-based
 };
 
+// one flat weight: every number concentration is the same, so every draw of
+// coagulate_weighting is below its ratio of 1 whatever its value
+__device__ __forceinline__ bool one_flat_weight(const PopDev& P) {
+  return P.flat && P.n_group == 1 && P.n_class == 1 && P.w.mag[0] > 0.0 && P.w.mag[0] < 1e300;
+}
+
+// volume whose radius merge_decide_rc takes
+__device__ __forceinline__ double merge_vol(const PopDev& P, double r1, double r2) {
+  return rad2vol(P.benv.frac, r1) + rad2vol(P.benv.frac, r2);
+}
+
 // particle 1 (radius r1, total volume vt1) from the pair's first cell,
-// particle 2 from its second
+// particle 2 from its second; rc: the radius of merge_vol (not read under one
+// flat weight)
 template <class R>
-__device__ MergeDecision merge_decide_v(const PopDev& P, R& g, double r1, double vt1, double r2, double vt2, int c1,
-                                        int c2, int cc) {
+__device__ MergeDecision merge_decide_rc(const PopDev& P, R& g, double r1, double vt1, double r2, double vt2, int c1,
+                                         int c2, int cc, double rc) {
   MergeDecision d;
-  const Fractal& F = P.benv.frac;
-  double rc = vol2rad(F, rad2vol(F, r1) + rad2vol(F, r2));
+  if (one_flat_weight(P)) {
+    g.seek(g.used() + 5u);  // the group's two draws and the three ratios'
+    d.new_group = 1;
+    d.rm1 = d.rm2 = d.create = true;
+    d.lost2 = vt1 > vt2;
+    d.lost1 = !d.lost2;
+    return d;
+  }
   double nc1 = num_conc_at_radius<double>(P.w, c1, r1);
   double nc2 = num_conc_at_radius<double>(P.w, c2, r2);
   double ncc = num_conc_at_radius<double>(P.w, cc, rc);
@@ -665,6 +688,13 @@ __device__ MergeDecision merge_decide_v(const PopDev& P, R& g, double r1, double
     d.lost2 = d.rm2;
   }
   return d;
+}
+
+template <class R>
+__device__ MergeDecision merge_decide_v(const PopDev& P, R& g, double r1, double vt1, double r2, double vt2, int c1,
+                                        int c2, int cc) {
+  const double rc = one_flat_weight(P) ? 0.0 : vol2rad(P.benv.frac, merge_vol(P, r1, r2));
+  return merge_decide_rc(P, g, r1, vt1, r2, vt2, c1, c2, cc, rc);
 }
 
 template <class R>

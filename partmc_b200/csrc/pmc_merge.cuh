@@ -9,6 +9,8 @@
 // k_items) in the next round.
 #pragma once
 
+#include <type_traits>
+
 #include "pmc_kernels.cuh"
 #include "pmc_particle.cuh"
 
@@ -432,9 +434,8 @@ struct WalkOut {
   bool stop = false;        // the walk reached a per-particle pair (q) whose target cell is its cell
 };
 
-// true if this round's claim on slot y is the chain of walker x
-__device__ __forceinline__ bool claimed_by_walk(const PopDev& P, int y, int x) {
-  unsigned long long w = P.claim[y];
+// true if claim word w is this round's claim of the chain of walker x
+__device__ __forceinline__ bool is_walk_claim(const PopDev& P, unsigned long long w, int x) {
   return (w >> 53) == (unsigned long long)(~*P.gen_p & kGenLimit) && ((w >> 32) & 1ULL) &&
          (uint32_t)w == (uint32_t)x;
 }
@@ -531,8 +532,34 @@ __device__ __forceinline__ int walk_pair(const Stretch& s, double at) {
 // Partner draws of a chain's test t after the first: the walk stream's
 // block (x, t + r * 2^26) for the r-th redraw (t stays below 2^26).
 constexpr uint32_t kChainRedraws = 64;
+constexpr int kRedrawBatch = 4;
 __device__ __forceinline__ uint32_t walk_redraw(const PopDev& P, int x, uint32_t t, uint32_t r) {
   return walk_draws(P, x, t | (r << 26)).x;
+}
+
+// The first of the redraws r = 1, 2, ... of a test whose partner is no
+// absorbed member, -2 if every one is.  A collector that has emptied most of
+// a cell redraws tens of times, so the redraws go kRedrawBatch at a time with
+// their loads in flight together.
+__device__ __noinline__ int redraw_partner(const PopDev& P, int x, uint32_t t, int o_start, int n_o) {
+  for (uint32_t r0 = 1; r0 < kChainRedraws; r0 += kRedrawBatch) {
+    int y[kRedrawBatch];
+    unsigned long long w[kRedrawBatch];
+#pragma unroll
+    for (int k = 0; k < kRedrawBatch; k++) {
+      int i = (int)(u32d(walk_redraw(P, x, t, r0 + k)) * (double)n_o);
+      if (i >= n_o) i = n_o - 1;
+      y[k] = P.list[o_start + i];
+    }
+#pragma unroll
+    for (int k = 0; k < kRedrawBatch; k++) w[k] = y[k] >= 0 && y[k] < P.cap ? __ldcg(&P.claim[y[k]]) : 0ULL;
+#pragma unroll
+    for (int k = 0; k < kRedrawBatch; k++) {
+      if (r0 + k >= kChainRedraws) break;
+      if (!(y[k] >= 0 && y[k] < P.cap && is_walk_claim(P, w[k], x))) return y[k];
+    }
+  }
+  return -2;
 }
 
 // One walk test t of particle x (records qxd/qxf) at running position at of
@@ -545,12 +572,16 @@ __device__ __forceinline__ uint32_t walk_redraw(const PopDev& P, int x, uint32_t
 // coagulation.F90:628-638); a test whose kChainRedraws draws all land on
 // absorbed members counts as that exit.  Returns 0 for no test (no member,
 // itself, a dead or moved member, the exit), 1 for a rejected test, 2 for an
-// accepted one, -1 for a failed bounds check.
+// accepted one, -1 for a failed bounds check.  *side gets kSideExact if the
+// test was decided in FP64 and kSideWarn if k > k_max: the caller counts them,
+// as a test drawn ahead of an accepted one never happens.
+constexpr uint32_t kSideExact = 1u, kSideWarn = 2u;
 template <int KT, class T, bool FLAT>
 __device__ __forceinline__ int walk_test(const PopDev& P, int x, const Stretch& s, int j, double at, uint32_t t,
                                          uint32_t pick, uint32_t accu, const RecD& qxd, const RecF& qxf, bool chain,
                                          int* y_out, float* pos_out, int* q_out, bool* first_out, double* ry_out,
-                                         double* vty_out) {
+                                         double* vty_out, uint32_t* side) {
+  *side = 0u;
   const double c0 = s.cum[j], c1 = s.cum[j + 1];
   const int4 ent = P.cp_ent[j];
   double lam = c1 - c0;
@@ -565,13 +596,9 @@ __device__ __forceinline__ int walk_test(const PopDev& P, int x, const Stretch& 
   int i = (int)(u32d(pick) * (double)n_o);
   if (i >= n_o) i = n_o - 1;
   int y = P.list[o_start + i];
-  if (chain) {
-    for (uint32_t r = 1; y >= 0 && y < P.cap && claimed_by_walk(P, y, x); r++) {
-      if (r >= kChainRedraws) return 0;
-      i = (int)(u32d(walk_redraw(P, x, t, r)) * (double)n_o);
-      if (i >= n_o) i = n_o - 1;
-      y = P.list[o_start + i];
-    }
+  if (chain && y >= 0 && y < P.cap && is_walk_claim(P, __ldcg(&P.claim[y]), x)) {
+    y = redraw_partner(P, x, t, o_start, n_o);
+    if (y == -2) return 0;
   }
   const PairDesc d = P.pair_desc[q];
   const PairState& S = P.pair[q];
@@ -586,10 +613,10 @@ __device__ __forceinline__ int walk_test(const PopDev& P, int x, const Stretch& 
   const double ry = P.rad[y], vty = P.vtot[y];  // for the merge decision if the test accepts
   if (y == x || !alive || cell_y != O) return 0;
   const double u = u32d(accu);
-  bool acc;
+  bool acc, warn = false;
   if constexpr (sizeof(T) == 8) {
     const RecD qy = P.recd[y];
-    acc = accept_f64_rec<KT, FLAT>(P, first ? qxd : qy, first ? qy : qxd, d, cc, fflat, inv_k_max, u);
+    acc = accept_f64_rec<KT, FLAT>(P, first ? qxd : qy, first ? qy : qxd, d, cc, fflat, inv_k_max, u, &warn);
   } else {
     const RecF qy = P.recf[y];
     const float* qw = (const float*)&qxf;
@@ -601,10 +628,11 @@ __device__ __forceinline__ int walk_test(const PopDev& P, int x, const Stretch& 
       acc = u < (double)pf;
     } else {  // decided in FP64 (see f32_decides)
       const RecD qy = P.recd[y];
-      acc = accept_f64_rec<KT, FLAT>(P, first ? qxd : qy, first ? qy : qxd, d, cc, fflat, inv_k_max, u);
-      add_ll(&P.ctr->exact_tests, 1LL);
+      acc = accept_f64_rec<KT, FLAT>(P, first ? qxd : qy, first ? qy : qxd, d, cc, fflat, inv_k_max, u, &warn);
+      *side = kSideExact;
     }
   }
+  if (warn) *side |= kSideWarn;
   *y_out = y;
   *pos_out = (float)((at - c0) / lam);
   *q_out = q;
@@ -641,7 +669,10 @@ __device__ __forceinline__ int walk_next(const PopDev& P, int x, Stretch& s, uin
     int j = walk_pair(s, at);
     s.j = j;
     s.at = at;
-    int r = walk_test<KT, T, FLAT>(P, x, s, j, at, t, u.z, u.w, qxd, qxf, chain, y, pos, q, first, ry, vty);
+    uint32_t side;
+    int r = walk_test<KT, T, FLAT>(P, x, s, j, at, t, u.z, u.w, qxd, qxf, chain, y, pos, q, first, ry, vty, &side);
+    if (side & kSideExact) add_ll(&P.ctr->exact_tests, 1LL);
+    if (side & kSideWarn) add_ll(&P.ctr->kmax_warn, 1LL);
     if (r < 0) return -1;
     if (r == 0) continue;
     (*n_tests)++;
@@ -649,12 +680,211 @@ __device__ __forceinline__ int walk_next(const PopDev& P, int x, Stretch& s, uin
   }
 }
 
+// The next 32 tests of one walker, one a lane (every lane of the warp takes
+// the same walker).  What a test reads of the walker's cell, its pair and its
+// partner does not depend on the walking particle's size, so a chain that
+// stays in its cell goes on with the same tests after an absorb and evaluates
+// only their acceptance again.
+template <class T>
+struct WalkBatch {
+  using Rec = typename std::conditional<sizeof(T) == 8, RecD, RecF>::type;
+  int n_in;     // tests before the end of the stretch
+  double end;   // position after the last of the 32 gaps drawn
+  // the lane's test
+  uint32_t t;
+  double at;    // position and list entry
+  int j;
+  int state;    // 1: a test, 0: no partner, -1: a failed check
+  int y, q, O, o_start, n_o, c1, c2, cc;
+  bool first;
+  float pos;
+  double ry, vty, inv_k_max, fflat, u;
+  Rec rec;
+};
+
+// the lane's partner B.y: its state and values
+template <class T>
+__device__ __forceinline__ void batch_partner(const PopDev& P, int x, WalkBatch<T>& B) {
+  const int y = B.y;
+  if (y < 0 || y >= P.cap) {
+    bad_index(P.ctr, kBadTestSlot, y);
+    B.state = -1;
+    return;
+  }
+  const uint8_t alive = P.alive[y];
+  const int cell_y = P.cell[y];
+  B.ry = P.rad[y];
+  B.vty = P.vtot[y];
+  if constexpr (sizeof(T) == 8) B.rec = P.recd[y];
+  else B.rec = P.recf[y];
+  B.state = y == x || !alive || cell_y != B.O ? 0 : 1;
+}
+
+// a partner that the chain has absorbed is drawn again (see walk_test)
+template <class T>
+__device__ __forceinline__ void batch_redraw(const PopDev& P, int x, WalkBatch<T>& B) {
+  if (!(B.y >= 0 && B.y < P.cap && is_walk_claim(P, __ldcg(&P.claim[B.y]), x))) return;
+  B.y = redraw_partner(P, x, B.t, B.o_start, B.n_o);
+  if (B.y == -2) B.state = 0;
+  else batch_partner(P, x, B);
+}
+
+template <class T>
+__device__ __forceinline__ void batch_draw(const PopDev& P, int x, const Stretch& s, uint32_t t_next, bool chain,
+                                           WalkBatch<T>& B) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  B.t = t_next + (uint32_t)lane;
+  const U4 u = walk_draws(P, x, B.t);
+  const double gap = -log(u53(u.x, u.y));
+  // positions summed in test order
+  double acc = s.at;
+  B.n_in = 32;
+  B.at = 0.0;
+#pragma unroll 1
+  for (int k0 = 0; k0 < 32 && B.n_in == 32; k0 += 8) {
+    double g8[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) g8[k] = __shfl_sync(kFull, gap, k0 + k);
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (B.n_in == 32) {
+        acc = acc + g8[k];
+        if (lane == k0 + k) B.at = acc;
+        if (!(acc < s.total)) B.n_in = k0 + k;
+      }
+  }
+  B.end = acc;
+  B.j = s.j;
+  B.state = 0;
+  B.y = -1;
+  if (lane >= B.n_in) return;
+  if (B.t >= (1u << 26)) {  // far past any mean the step can ask for
+    set_status(P.ctr, kErrTimeout);
+    B.state = -1;
+    return;
+  }
+  B.j = walk_pair(s, B.at);
+  const double c0 = s.cum[B.j], c1 = s.cum[B.j + 1];
+  const int4 ent = P.cp_ent[B.j];
+  const double lam = c1 - c0;
+  B.n_o = ent.w;
+  B.o_start = ent.z;
+  if (!(lam > 0.0) || B.n_o < 1) return;
+  if (B.o_start < 0 || (long long)B.o_start + B.n_o > P.cap || ent.x < 0 || ent.x >= P.n_pairs) {
+    bad_index(P.ctr, kBadPairCells, ent.x);
+    B.state = -1;
+    return;
+  }
+  B.q = ent.x;
+  B.O = ent.y & ((1 << 30) - 1);
+  B.first = (ent.y >> 30) & 1;
+  B.pos = (float)((B.at - c0) / lam);
+  B.u = u32d(u.w);
+  int i = (int)(u32d(u.z) * (double)B.n_o);
+  if (i >= B.n_o) i = B.n_o - 1;
+  B.y = P.list[B.o_start + i];
+  const PairDesc d = P.pair_desc[B.q];
+  const PairState& S = P.pair[B.q];
+  B.c1 = d.c1;
+  B.c2 = d.c2;
+  B.inv_k_max = S.inv_k_max;
+  B.fflat = S.fflat;
+  B.cc = S.cc;
+  batch_partner(P, x, B);
+  if (chain) batch_redraw(P, x, B);
+}
+
+// The first accepted test at or after lane `from` for the walking particle
+// (records qxd/qxf): its lane, 32 if none is accepted (or -1 - lane for a
+// failed check).  *n_tests counts the tests up to it.
+template <int KT, class T, bool FLAT>
+__device__ __forceinline__ int batch_first(const PopDev& P, const WalkBatch<T>& B, int from, const RecD& qxd,
+                                           const RecF& qxf, long long* n_tests) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  bool acc = false, warn = false, exact = false;
+  const bool on = lane >= from && lane < B.n_in && B.state == 1;
+  if (on) {
+    PairDesc d;
+    d.c1 = (int8_t)B.c1;
+    d.c2 = (int8_t)B.c2;
+    if constexpr (sizeof(T) == 8) {
+      acc = accept_f64_rec<KT, FLAT>(P, B.first ? qxd : B.rec, B.first ? B.rec : qxd, d, B.cc, B.fflat, B.inv_k_max,
+                                     B.u, &warn);
+    } else {
+      const float* qw = (const float*)&qxf;
+      const float* py = (const float*)&B.rec;
+      const float pf = pair_kernel<KT, float, FLAT>(P, B.first ? qw : py, B.first ? py : qw, B.c1, B.c2, B.cc,
+                                                    (float)B.fflat, (float)P.coeff) *
+                       (float)B.inv_k_max;
+      if (f32_decides(pf, B.u)) {
+        acc = B.u < (double)pf;
+      } else {  // decided in FP64 (see f32_decides)
+        const RecD qy = P.recd[B.y];
+        acc = accept_f64_rec<KT, FLAT>(P, B.first ? qxd : qy, B.first ? qy : qxd, d, B.cc, B.fflat, B.inv_k_max, B.u,
+                                       &warn);
+        exact = true;
+      }
+    }
+  }
+  const unsigned m_end = __ballot_sync(kFull, acc || (lane >= from && lane < B.n_in && B.state < 0));
+  const int stop = m_end ? __ffs(m_end) - 1 : 32;
+  // the tests after the accepted one have not happened yet
+  const unsigned m_cnt = __ballot_sync(kFull, on && lane <= stop);
+  const unsigned m_ex = __ballot_sync(kFull, exact && lane <= stop), m_wa = __ballot_sync(kFull, warn && lane <= stop);
+  *n_tests += __popc(m_cnt);
+  if (lane == 0) {
+    if (m_ex) add_ll(&P.ctr->exact_tests, (long long)__popc(m_ex));
+    if (m_wa) add_ll(&P.ctr->kmax_warn, (long long)__popc(m_wa));
+  }
+  if (stop == 32) return 32;
+  return __shfl_sync(kFull, B.state, stop) < 0 ? -1 - stop : stop;
+}
+
+// walk_next by a warp for one walker: the tests 32 at a time, those up to the
+// first accepted one stand.  A test is a chain of about six dependent loads
+// and, for some kernels, as much arithmetic (2 to 3 us), and most reject.
+template <int KT, class T, bool FLAT>
+__device__ __forceinline__ int walk_next_warp(const PopDev& P, int x, Stretch& s, uint32_t& t_next, const RecD& qxd,
+                                              const RecF& qxf, long long* n_tests, int* y, float* pos, int* q,
+                                              bool* first, double* ry, double* vty) {
+  constexpr unsigned kFull = 0xffffffffu;
+  for (;;) {
+    WalkBatch<T> B;
+    batch_draw(P, x, s, t_next, false, B);
+    const int at = batch_first<KT, T, FLAT>(P, B, 0, qxd, qxf, n_tests);
+    if (at < 0) return -1;
+    if (at < 32) {
+      t_next += (uint32_t)at + 1u;
+      *y = __shfl_sync(kFull, B.y, at);
+      *q = __shfl_sync(kFull, B.q, at);
+      *pos = __shfl_sync(kFull, B.pos, at);
+      *first = __shfl_sync(kFull, B.first ? 1 : 0, at) != 0;
+      *ry = __shfl_sync(kFull, B.ry, at);
+      *vty = __shfl_sync(kFull, B.vty, at);
+      return 1;
+    }
+    if (B.n_in < 32) {
+      if (s.stop >= 0) {  // a per-particle pair that takes the particle as a target
+        *q = P.cp_list[s.stop];
+        return 3;
+      }
+      return 0;  // no test left in the cell's later pairs
+    }
+    s.at = B.end;
+    s.j = __shfl_sync(kFull, B.j, 31);
+    t_next += 32u;
+  }
+}
+
 // The first event of walker x from (p0, pos0): the first accepted test,
 // claimed by its merge decision; an absorb (the walking particle is replaced
 // by the coagulated one) is carried on as a chain by k_chain from the next
-// test on.
-template <int KT, class T, bool FLAT>
+// test on.  WARP: by a warp, every lane with the same arguments.
+template <int KT, class T, bool FLAT, bool WARP>
 __device__ void walk(const PopDev& P, int x, int p0, float pos0, WalkOut* out) {
+  const bool lead = !WARP || (threadIdx.x & 31) == 0;
   if (x < 0 || x >= P.cap || !P.alive[x]) return;
   const int C = P.cell[x];
   if (C < 0 || C >= P.n_cells) return;
@@ -668,7 +898,11 @@ __device__ void walk(const PopDev& P, int x, int p0, float pos0, WalkOut* out) {
   float pos;
   bool first;
   double ry, vty;
-  int r = walk_next<KT, T, FLAT>(P, x, s, t_next, qxd, qxf, false, &n_tests, &y, &pos, &q, &first, &ry, &vty);
+  int r;
+  if constexpr (WARP)
+    r = walk_next_warp<KT, T, FLAT>(P, x, s, t_next, qxd, qxf, &n_tests, &y, &pos, &q, &first, &ry, &vty);
+  else
+    r = walk_next<KT, T, FLAT>(P, x, s, t_next, qxd, qxf, false, &n_tests, &y, &pos, &q, &first, &ry, &vty);
   if (r == 0) out->done = true;
   if (r == 3) {
     out->stop = true;
@@ -681,8 +915,8 @@ __device__ void walk(const PopDev& P, int x, int p0, float pos0, WalkOut* out) {
     unsigned long long ck = claim_key(P, key);
     Rng gm = merge_rng(P, key);
     double rx = P.rad[x], vtx = P.vtot[x];
-    MergeDecision m = first ? merge_decide_v(P, gm, rx, vtx, ry, vty, d.c1, d.c2, S.cc)
-                            : merge_decide_v(P, gm, ry, vty, rx, vtx, d.c1, d.c2, S.cc);
+    const MergeDecision m = merge_decide_v(P, gm, first ? rx : ry, first ? vtx : vty, first ? ry : rx,
+                                           first ? vty : vtx, d.c1, d.c2, S.cc);
     bool rm_x = first ? m.rm1 : m.rm2, rm_y = first ? m.rm2 : m.rm1;
     out->found = true;
     out->q = q;
@@ -690,13 +924,15 @@ __device__ void walk(const PopDev& P, int x, int p0, float pos0, WalkOut* out) {
     out->pos = pos;
     out->first_cell1 = first;
     out->dec = pack_decision(m, gm.used());
-    if (m.new_group == 0) set_status(P.ctr, kErrTimeout);
-    claim_slot(P, x, ck, rm_x);
-    claim_slot(P, y, ck, rm_y);
+    if (lead) {
+      if (m.new_group == 0) set_status(P.ctr, kErrTimeout);
+      claim_slot(P, x, ck, rm_x);
+      claim_slot(P, y, ck, rm_y);
+    }
     out->cont = m.create && rm_x && m.new_group != 0;
     out->g_used = t_next;
   }
-  if (n_tests) {
+  if (n_tests && lead) {
     add_ll_warp(&P.ctr->tot_samp, (int)n_tests);
     add_ll_warp(&P.ctr->walk_tests, (int)n_tests);
   }
@@ -715,8 +951,8 @@ __device__ __noinline__ uint32_t chain_event_decision(const PopDev& P, unsigned 
   const PairDesc d = P.pair_desc[q];
   const PairState& S = P.pair[q];
   Rng g = make_rng(P, kStreamChain, i + 1u, (uint32_t)x);
-  MergeDecision m = sl.x == x ? merge_decide_v(P, g, P.rad[x], P.vtot[x], P.rad[y], P.vtot[y], d.c1, d.c2, S.cc)
-                              : merge_decide_v(P, g, P.rad[y], P.vtot[y], P.rad[x], P.vtot[x], d.c1, d.c2, S.cc);
+  const int s1 = sl.x == x ? x : y, s2 = sl.x == x ? y : x;
+  MergeDecision m = merge_decide_v(P, g, P.rad[s1], P.vtot[s1], P.rad[s2], P.vtot[s2], d.c1, d.c2, S.cc);
   if (m.new_group == 0) set_status(P.ctr, kErrTimeout);
   return pack_decision(m, g.used());
 }
@@ -741,7 +977,46 @@ __device__ __noinline__ void add_target_op(const PopDev& P, int pop, int q, int 
   op_key[k] = make_key((uint32_t)q, 1u, (uint32_t)x);
 }
 
-// The work of a later round, one thread per event e of the round before:
+// Walks, or chains, per warp of the launch up to which each takes a warp; with
+// more, each takes a thread.  A launch ends with its longest walk, and a
+// warp's takes about as long as two tests of a thread's; but a warp each in
+// several waves (4 walks a warp: 25 us for the first later round of 1e6
+// particles) is slower than 32 walks a warp (22 us).
+constexpr int kWarpShare = 1;
+
+// what a later round's kernels read of the round before and write for this one
+struct ItemArgs {
+  const PopDev* pops;
+  const int *gpair_pop, *gpair_local;
+  const long long* pop_pair_base;
+  int n_gpairs;
+  const long long *n_items, *n_items_ev;
+  const int *ppw_slot, *ppw_gp;
+  int *op_pop, *op_pair, *op_slot, *op_k;
+  unsigned long long* op_key;
+  const long long* n_ops;
+  long long op_cap;
+  const uint8_t* win;
+  const int* dest;
+  const unsigned long long* ev_key;
+  const int2* ev_c;
+  const int* gp_c;
+  const float* ev_pos;
+  const uint32_t* dec;
+  uint8_t* it_flag;
+  unsigned long long* it_key;
+  int2* it_c;
+  int* it_gp;
+  float* it_pos;
+  int *it_len, *it_head;
+  uint8_t* it_done;
+  uint32_t *it_dec, *it_gused;
+  int4* it_term;
+  int* start_list;      // items whose walk k_chain carries on
+  long long* n_start;
+};
+
+// The work of a later round, per event e of the round before:
 //   - a winner that created or changed a particle (dest[e] >= 0): that
 //     particle walks from the event's pair and position (for a chain, its
 //     last applied event's);
@@ -754,135 +1029,150 @@ __device__ __noinline__ void add_target_op(const PopDev& P, int pop, int q, int 
 // Output per e: flag, and key, slots, global pair and position of the new
 // event (for a chain its first event) with the chain's length and head; the
 // new event holds claims on its slots.
-template <int KT, class T, bool FLAT>
-__global__ void __launch_bounds__(256) k_items(const PopDev* pops, const int* gpair_pop, const int* gpair_local,
-                                               const long long* pop_pair_base, int n_gpairs, const long long* n_items,
-                                               const long long* n_items_ev, const int* ppw_slot, const int* ppw_gp,
-                                               int* op_pop, int* op_pair, int* op_slot, int* op_k,
-                                               unsigned long long* op_key, long long* n_ops, long long op_cap,
-                                               const uint8_t* win, const int* dest,
-                                               const unsigned long long* ev_key, const int2* ev_c,
-                                               const int* gp_c, const float* ev_pos, const uint32_t* dec,
-                                               uint8_t* it_flag, unsigned long long* it_key,
-                                               int2* it_c, int* it_gp, float* it_pos, int* it_len, int* it_head,
-                                               uint8_t* it_done, uint32_t* it_dec, uint32_t* it_gused, int4* it_term) {
-  long long n = *n_items, n_ev = *n_items_ev;
-  const long long op_base = op_cap > 0 ? *n_ops : 0;  // the redone operations come first
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    it_flag[e] = 0;
-    it_term[e] = no_term();
-    if (op_cap > 0 && op_base + e < op_cap) op_pop[op_base + e] = -1;
-    int gp, walker = -1, p0 = 0;
-    float pos0 = 1.0f;
-    unsigned long long key = 0;
-    int2 sl = make_int2(-1, -1);
-    uint32_t dc = 0;
-    if (e >= n_ev) {
-      // a particle that a target operation of the round before made or
-      // changed walks from the end of that operation's pair
-      gp = ppw_gp[e - n_ev];
-      if (gp < 0 || gp >= n_gpairs) {
-        bad_index(pops[0].ctr, kBadEventSlot, gp);
-        continue;
+template <int KT, class T, bool FLAT, bool WARP>
+__device__ __forceinline__ void do_item(const ItemArgs& A, long long e, long long n_ev, long long op_base) {
+  const bool lead = !WARP || (threadIdx.x & 31) == 0;
+  if (lead) {
+    A.it_flag[e] = 0;
+    A.it_term[e] = no_term();
+    if (A.op_cap > 0 && op_base + e < A.op_cap) A.op_pop[op_base + e] = -1;
+  }
+  int gp, walker = -1, p0 = 0;
+  float pos0 = 1.0f;
+  unsigned long long key = 0;
+  int2 sl = make_int2(-1, -1);
+  uint32_t dc = 0;
+  if (e >= n_ev) {
+    // a particle that a target operation of the round before made or
+    // changed walks from the end of that operation's pair
+    gp = A.ppw_gp[e - n_ev];
+    if (gp < 0 || gp >= A.n_gpairs) {
+      if (lead) bad_index(A.pops[0].ctr, kBadEventSlot, gp);
+      return;
+    }
+    walker = A.ppw_slot[e - n_ev];
+    p0 = A.gpair_local[gp];
+  } else {
+    gp = A.gp_c[e];
+    if (gp < 0 || gp >= A.n_gpairs) {
+      if (lead) bad_index(A.pops[0].ctr, kBadEventSlot, gp);
+      return;
+    }
+    const PopDev& P = A.pops[A.gpair_pop[gp]];
+    uint32_t pend_dec = 0xffffffffu;  // a pending chain event's recomputed decision
+    pos0 = A.ev_pos[e];
+    key = A.ev_key[e];
+    sl = A.ev_c[e];
+    const bool won = A.win[e] != 0;
+    const int dst = A.dest[e];
+    const bool in = !(sl.x < 0 || sl.x >= P.cap || sl.y < 0 || sl.y >= P.cap);
+    if (won && (dst == kPendingTerm || dst == kPendingChain)) {
+      // the test where the previous round's chain stopped, with its
+      // decision: the walker was rewritten by its own chain, so only its
+      // death counts; a partner consumed in that round is no member now,
+      // and the walk goes on after the test
+      if (!in) {
+        if (lead) bad_index(P.ctr, kBadEventSlot, sl.x < 0 || sl.x >= P.cap ? sl.x : sl.y);
+        return;
       }
-      walker = ppw_slot[e - n_ev];
-      p0 = gpair_local[gp];
+      const int x = (int)key_idx(key), y = x == sl.x ? sl.y : sl.x;
+      if (!P.alive[x]) return;
+      if (P.touched[y] == *P.gen_p - 1u || !P.alive[y]) {
+        walker = x;
+        p0 = (int)key_pair(key);
+      } else if (dst == kPendingChain) {
+        pend_dec = chain_event_decision(P, key, sl, x, y, A.dec[e]);
+        if (pend_dec == 0xffffffffu) return;
+      }
+    } else if (won) {
+      walker = dst;
+      p0 = A.gpair_local[gp];
+      if (walker < 0) return;
     } else {
-      gp = gp_c[e];
-      if (gp < 0 || gp >= n_gpairs) {
-        bad_index(pops[0].ctr, kBadEventSlot, gp);
-        continue;
+      if (!in) {
+        if (lead) bad_index(P.ctr, kBadEventSlot, sl.x < 0 || sl.x >= P.cap ? sl.x : sl.y);
+        return;
       }
-      const PopDev& P = pops[gpair_pop[gp]];
-      uint32_t pend_dec = 0xffffffffu;  // a pending chain event's recomputed decision
-      pos0 = ev_pos[e];
-      key = ev_key[e];
-      sl = ev_c[e];
-      if (win[e] && (dest[e] == kPendingTerm || dest[e] == kPendingChain)) {
-        // the test where the previous round's chain stopped, with its
-        // decision: the walker was rewritten by its own chain, so only its
-        // death counts; a partner consumed in that round is no member now,
-        // and the walk goes on after the test
-        if (sl.x < 0 || sl.x >= P.cap || sl.y < 0 || sl.y >= P.cap) {
-          bad_index(P.ctr, kBadEventSlot, sl.x < 0 || sl.x >= P.cap ? sl.x : sl.y);
-          continue;
-        }
-        const int x = (int)key_idx(key), y = x == sl.x ? sl.y : sl.x;
-        if (!P.alive[x]) continue;
-        if (P.touched[y] == *P.gen_p - 1u || !P.alive[y]) {
+      uint32_t gen_prev = *P.gen_p - 1u;
+      bool c1 = P.touched[sl.x] == gen_prev || !P.alive[sl.x];
+      bool c2 = P.touched[sl.y] == gen_prev || !P.alive[sl.y];
+      if (key_kind(key) == 0u) {
+        if (c1 || c2) return;
+      } else {
+        int x = (int)key_idx(key);
+        bool cx = x == sl.x ? c1 : c2, cy = x == sl.x ? c2 : c1;
+        if (cx) return;
+        if (cy) {
           walker = x;
           p0 = (int)key_pair(key);
-        } else if (dest[e] == kPendingChain) {
-          pend_dec = chain_event_decision(P, key, sl, x, y, dec[e]);
-          if (pend_dec == 0xffffffffu) continue;
-        }
-      } else if (win[e]) {
-        walker = dest[e];
-        p0 = gpair_local[gp];
-        if (walker < 0) continue;
-      } else {
-        if (sl.x < 0 || sl.x >= P.cap || sl.y < 0 || sl.y >= P.cap) {
-          bad_index(P.ctr, kBadEventSlot, sl.x < 0 || sl.x >= P.cap ? sl.x : sl.y);
-          continue;
-        }
-        uint32_t gen_prev = *P.gen_p - 1u;
-        bool c1 = P.touched[sl.x] == gen_prev || !P.alive[sl.x];
-        bool c2 = P.touched[sl.y] == gen_prev || !P.alive[sl.y];
-        if (key_kind(key) == 0u) {
-          if (c1 || c2) continue;
-        } else {
-          int x = (int)key_idx(key);
-          bool cx = x == sl.x ? c1 : c2, cy = x == sl.x ? c2 : c1;
-          if (cx) continue;
-          if (cy) {
-            walker = x;
-            p0 = (int)key_pair(key);
-          }
         }
       }
-      dc = pend_dec != 0xffffffffu ? pend_dec : dec[e];
     }
-    const int pop = gpair_pop[gp];
-    const PopDev& P = pops[pop];
-    int len = 0, head = -1;
-    bool done = false;
-    if (walker >= 0) {
-      WalkOut w;
-      walk<KT, T, FLAT>(P, walker, p0, pos0, &w);
-      if (w.stop) add_target_op(P, pop, w.q, walker, op_pop, op_pair, op_slot, op_k, op_key, op_base + e, op_cap);
-      if (!w.found) continue;
-      key = make_key((uint32_t)w.q, 1u, (uint32_t)walker);
-      sl = w.first_cell1 ? make_int2(walker, w.y) : make_int2(w.y, walker);
-      gp = (int)(pop_pair_base[pop] + w.q);
-      pos0 = w.pos;
-      len = w.cont ? -1 : 0;  // -1: k_chain carries the walk on
-      done = w.done;
-      dc = w.dec;
-      it_gused[e] = w.g_used;
-    } else {
-      // a retry keeps its merge decision and claims by it
-      uint32_t used;
-      MergeDecision m = unpack_decision(dc, &used);
-      unsigned long long ck = claim_key(P, key);
-      claim_slot(P, sl.x, ck, m.rm1);
-      claim_slot(P, sl.y, ck, m.rm2);
+    dc = pend_dec != 0xffffffffu ? pend_dec : A.dec[e];
+  }
+  const int pop = A.gpair_pop[gp];
+  const PopDev& P = A.pops[pop];
+  int len = 0;
+  bool done = false;
+  if (walker >= 0) {
+    WalkOut w;
+    walk<KT, T, FLAT, WARP>(P, walker, p0, pos0, &w);
+    if (w.stop && lead)
+      add_target_op(P, pop, w.q, walker, A.op_pop, A.op_pair, A.op_slot, A.op_k, A.op_key, op_base + e, A.op_cap);
+    if (!w.found) return;
+    key = make_key((uint32_t)w.q, 1u, (uint32_t)walker);
+    sl = w.first_cell1 ? make_int2(walker, w.y) : make_int2(w.y, walker);
+    gp = (int)(A.pop_pair_base[pop] + w.q);
+    pos0 = w.pos;
+    done = w.done;
+    dc = w.dec;
+    if (w.cont) {
+      len = -1;  // k_chain carries the walk on
+      if (lead) {
+        A.it_gused[e] = w.g_used;
+        A.start_list[inc_warp((unsigned long long*)A.n_start)] = (int)e;
+      }
     }
-    it_flag[e] = 1;
-    it_key[e] = key;
-    it_c[e] = sl;
-    it_gp[e] = gp;
-    it_pos[e] = pos0;
-    it_len[e] = len;
-    it_head[e] = head;
-    it_done[e] = done ? 1 : 0;
-    it_dec[e] = dc;
+  } else if (lead) {
+    // a retry keeps its merge decision and claims by it
+    uint32_t used;
+    MergeDecision m = unpack_decision(dc, &used);
+    unsigned long long ck = claim_key(P, key);
+    claim_slot(P, sl.x, ck, m.rm1);
+    claim_slot(P, sl.y, ck, m.rm2);
+  }
+  if (lead) {
+    A.it_flag[e] = 1;
+    A.it_key[e] = key;
+    A.it_c[e] = sl;
+    A.it_gp[e] = gp;
+    A.it_pos[e] = pos0;
+    A.it_len[e] = len;
+    A.it_head[e] = -1;
+    A.it_done[e] = done ? 1 : 0;
+    A.it_dec[e] = dc;
   }
 }
 
-// Chains, after k_items: an item whose first event is an absorb (it_len -1)
-// carries its walk on from that event with the coagulated particle, one
-// thread per chain, drawing the walk's tests on from where k_items stopped.
+// A warp per item while the launch has the warps for it, else a thread.  Bound
+// by the longest walk's tests, one after another (57 us a launch for 4000
+// sedimenting drops in FP64, now 20), and below about 7 us by the item's own
+// dependent loads and the kernel's cold instructions.
+template <int KT, class T, bool FLAT>
+__global__ void __launch_bounds__(256) k_items(ItemArgs A) {
+  const long long n = *A.n_items, n_ev = *A.n_items_ev;
+  const long long op_base = A.op_cap > 0 ? *A.n_ops : 0;  // the redone operations come first
+  const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+  if (n <= kWarpShare * (nt >> 5)) {
+    for (long long e = tid >> 5; e < n; e += nt >> 5) do_item<KT, T, FLAT, true>(A, e, n_ev, op_base);
+  } else {
+    for (long long e = tid; e < n; e += nt) do_item<KT, T, FLAT, false>(A, e, n_ev, op_base);
+  }
+}
+
+// Chains, after k_items: an item whose first event is an absorb (it_len -1,
+// listed) carries its walk on from that event with the coagulated particle,
+// drawing the walk's tests on from where k_items stopped.
 // The coagulated particle's volumes are summed per species over the events,
 // then over the species, as k_apply_chain sums them, so its decisions are
 // the apply's.  While the particle stays in the cell it walked, the walk goes
@@ -893,84 +1183,242 @@ __global__ void __launch_bounds__(256) k_items(const PopDev* pops, const int* gp
 // the item gets the chain's length and head, or length 0 (the first event
 // alone) if the pool is full.
 template <int KT, class T, bool FLAT>
-__global__ void __launch_bounds__(128) k_chain(const PopDev* pops, const int* gpair_pop, const long long* n_items,
-                                               const uint8_t* it_flag, const unsigned long long* it_key,
-                                               const int2* it_c, const int* it_gp, const float* it_pos,
-                                               const uint32_t* it_dec, const uint32_t* it_gused, ChainPool pool,
-                                               int* it_len, int* it_head, uint8_t* it_done, int4* it_term) {
-  long long n = *n_items;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    if (!it_flag[e] || it_len[e] != -1) continue;
-    const PopDev& P = pops[gpair_pop[it_gp[e]]];
-    unsigned long long key = it_key[e];
-    const int x = (int)key_idx(key);
-    int q = (int)key_pair(key);
-    int2 sl = it_c[e];
-    int y = sl.x == x ? sl.y : sl.x;
-    uint32_t used;
-    MergeDecision m1 = unpack_decision(it_dec[e], &used);
-    bool rm_y1 = sl.x == x ? m1.rm2 : m1.rm1;
-    it_len[e] = 0;
-    if (x < 0 || x >= P.cap || y < 0 || y >= P.cap || q >= P.n_pairs) continue;
-    ChainWriter cw;
-    float pos = it_pos[e];
-    if (!cw.append(pool, y, q | (rm_y1 ? kChainRemoves : 0), pos)) continue;
-    uint32_t t_next = it_gused[e];
-    long long n_tests = 0;
-    bool done = false;
-    const int ns = P.n_spec;
-    double vcur[kMaxSpec];
-    for (int sp = 0; sp < ns; sp++) vcur[sp] = P.vol[vol_at(P, x, sp)];
-    int cls = P.pair[q].cc + 1;
-    Stretch s;
-    s.C = -1;
+__device__ __forceinline__ void do_chain(const ItemArgs& A, const ChainPool& pool, long long e) {
+  if (!A.it_flag[e] || A.it_len[e] != -1) return;
+  const PopDev& P = A.pops[A.gpair_pop[A.it_gp[e]]];
+  unsigned long long key = A.it_key[e];
+  const int x = (int)key_idx(key);
+  int q = (int)key_pair(key);
+  int2 sl = A.it_c[e];
+  int y = sl.x == x ? sl.y : sl.x;
+  uint32_t used;
+  MergeDecision m1 = unpack_decision(A.it_dec[e], &used);
+  bool rm_y1 = sl.x == x ? m1.rm2 : m1.rm1;
+  A.it_len[e] = 0;
+  if (x < 0 || x >= P.cap || y < 0 || y >= P.cap || q >= P.n_pairs) return;
+  ChainWriter cw;
+  float pos = A.it_pos[e];
+  if (!cw.append(pool, y, q | (rm_y1 ? kChainRemoves : 0), pos)) return;
+  uint32_t t_next = A.it_gused[e];
+  long long n_tests = 0;
+  bool done = false;
+  const int ns = P.n_spec;
+  double vcur[kMaxSpec];
+  for (int sp = 0; sp < ns; sp++) vcur[sp] = P.vol[vol_at(P, x, sp)];
+  int cls = P.pair[q].cc + 1;
+  Stretch s;
+  s.C = -1;
+  for (;;) {
+    // absorb y: the coagulated particle's volumes, radius, class, record
+    for (int sp = 0; sp < ns; sp++) vcur[sp] = vcur[sp] + P.vol[vol_at(P, y, sp)];
+    double s_v = 0.0, s_m = 0.0;
+    for (int sp = 0; sp < ns; sp++) s_v = s_v + vcur[sp];
+    for (int sp = 0; sp < ns; sp++) s_m = s_m + vcur[sp] * P.density[sp];
+    const double vt = s_v, r = vol2rad(P.benv.frac, vt);
+    const RecD qxd = make_rec_v(P, r, vt, s_m, cls);
+    const RecF qxf = to_f32(qxd);
+    const int C = cell_of(P, r, cls);
+    if (C < 0 || cw.len >= kChainMaxLen) break;  // off the grid (reported by the apply) or long enough
+    if (C != s.C) walk_stretch(P, C, q, pos, &s);
+    int yy, qq;
+    bool first;
+    double ry, vty;
+    int rw = walk_next<KT, T, FLAT>(P, x, s, t_next, qxd, qxf, true, &n_tests, &yy, &pos, &qq, &first, &ry, &vty);
+    if (rw == 0) done = true;  // every later pair of the cell was walked
+    if (rw != 1) break;
+    const PairDesc d = P.pair_desc[qq];
+    const PairState& S = P.pair[qq];
+    unsigned long long k2 = make_key((uint32_t)qq, 1u, (uint32_t)x);
+    Rng gm = make_rng(P, kStreamChain, (uint32_t)(cw.len + 1), (uint32_t)x);
+    const MergeDecision m = merge_decide_v(P, gm, first ? r : ry, first ? vt : vty, first ? ry : r,
+                                           first ? vty : vt, d.c1, d.c2, S.cc);
+    bool rm_x = first ? m.rm1 : m.rm2, rm_y = first ? m.rm2 : m.rm1;
+    // the chain ends before an event that is no absorb, or when the pool
+    // is full; that event is pending for the next round (kPendingTerm)
+    if (!(m.create && rm_x && m.new_group != 0) || !cw.append(pool, yy, qq | (rm_y ? kChainRemoves : 0), pos)) {
+      if (m.new_group == 0) set_status(P.ctr, kErrTimeout);
+      A.it_term[e] = make_int4(yy, qq | (first ? kTermFirst : 0), (int)pack_decision(m, gm.used()),
+                               __float_as_int(pos));
+      break;
+    }
+    claim_slot(P, yy, claim_key(P, k2), rm_y);
+    y = yy;
+    q = qq;
+    cls = S.cc + 1;
+  }
+  // a chain that ended at its first event is that event alone
+  A.it_len[e] = cw.len > 1 ? cw.len : 0;
+  A.it_head[e] = cw.head;
+  A.it_done[e] = done ? 1 : 0;
+  if (n_tests) {
+    add_ll_warp(&P.ctr->tot_samp, (int)n_tests);
+    add_ll_warp(&P.ctr->walk_tests, (int)n_tests);
+  }
+}
+
+// do_chain by a warp, the same events from the same draws: 32 tests at a time
+// (WalkBatch).  What is left in sequence per absorb is the coagulated
+// particle's radius, record and cell and the acceptance of the tests already
+// drawn; its radius and the decision's are one vol2rad call, on two lanes.
+// vs: 2 x kMaxSpec doubles of the warp's shared memory (the walking
+// particle's volumes, and those with the partner's added).
+template <int KT, class T, bool FLAT>
+__device__ __forceinline__ void do_chain_warp(const ItemArgs& A, const ChainPool& pool, long long e, double* vs) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const bool lead = lane == 0;
+  if (!A.it_flag[e] || A.it_len[e] != -1) return;
+  const PopDev& P = A.pops[A.gpair_pop[A.it_gp[e]]];
+  const unsigned long long key = A.it_key[e];
+  const int x = (int)key_idx(key);
+  int q = (int)key_pair(key);
+  const int2 sl = A.it_c[e];
+  int y = sl.x == x ? sl.y : sl.x;
+  uint32_t used;
+  const MergeDecision m1 = unpack_decision(A.it_dec[e], &used);
+  const bool rm_y1 = sl.x == x ? m1.rm2 : m1.rm1;
+  float pos = A.it_pos[e];
+  uint32_t t_next = A.it_gused[e];
+  __syncwarp();  // every lane has read the item
+  if (lead) A.it_len[e] = 0;
+  if (x < 0 || x >= P.cap || y < 0 || y >= P.cap || q >= P.n_pairs) return;
+  ChainWriter cw;
+  // the lead's append, its result for every lane (len counts on all of them)
+  auto append = [&](int yy, int qw, float ps) {
+    bool ok = true;
+    const int len = cw.len;
+    if (lead) ok = cw.append(pool, yy, qw, ps);
+    ok = __shfl_sync(kFull, ok ? 1 : 0, 0) != 0;
+    cw.len = ok ? len + 1 : len;
+    return ok;
+  };
+  if (!append(y, q | (rm_y1 ? kChainRemoves : 0), pos)) return;
+  long long n_tests = 0;
+  bool done = false;
+  const int ns = P.n_spec;
+  const bool flat1 = one_flat_weight(P);
+  double* vcur = vs;
+  double* vnew = vs + kMaxSpec;
+  for (int sp = lane; sp < ns; sp += 32) vcur[sp] = P.vol[vol_at(P, x, sp)] + P.vol[vol_at(P, y, sp)];
+  int cls = P.pair[q].cc + 1;
+  // total volume and mass of v, in species order
+  auto totals = [&](const double* v, double* s_v, double* s_m) {
+    __syncwarp();
+    double a = 0.0, b = 0.0;
+    for (int sp = 0; sp < ns; sp++) {
+      const double z = v[sp];
+      a = a + z;
+      b = b + z * P.density[sp];
+    }
+    *s_v = a;
+    *s_m = b;
+  };
+  double vt, ms;
+  totals(vcur, &vt, &ms);
+  double r = vol2rad(P.benv.frac, vt);
+  Stretch s;
+  s.C = -1;
+  WalkBatch<T> B;
+  int from = 32;  // lane of the batch's next test (32: none left)
+  B.n_in = 32;
+  for (;;) {
+    const RecD qxd = make_rec_v(P, r, vt, ms, cls);
+    const RecF qxf = to_f32(qxd);
+    const int C = cell_of(P, r, cls);
+    if (C < 0 || cw.len >= kChainMaxLen) break;  // off the grid (reported by the apply) or long enough
+    if (C != s.C) {
+      walk_stretch(P, C, q, pos, &s);
+      from = 32;
+      B.n_in = 32;
+    }
+    // the next accepted test
+    int at;
     for (;;) {
-      // absorb y: the coagulated particle's volumes, radius, class, record
-      for (int sp = 0; sp < ns; sp++) vcur[sp] = vcur[sp] + P.vol[vol_at(P, y, sp)];
-      double s_v = 0.0, s_m = 0.0;
-      for (int sp = 0; sp < ns; sp++) s_v = s_v + vcur[sp];
-      for (int sp = 0; sp < ns; sp++) s_m = s_m + vcur[sp] * P.density[sp];
-      const double vt = s_v, r = vol2rad(P.benv.frac, vt);
-      const RecD qxd = make_rec_v(P, r, vt, s_m, cls);
-      const RecF qxf = to_f32(qxd);
-      const int C = cell_of(P, r, cls);
-      if (C < 0 || cw.len >= kChainMaxLen) break;  // off the grid (reported by the apply) or long enough
-      if (C != s.C) walk_stretch(P, C, q, pos, &s);
-      int yy, qq;
-      bool first;
-      double ry, vty;
-      int rw = walk_next<KT, T, FLAT>(P, x, s, t_next, qxd, qxf, true, &n_tests, &yy, &pos, &qq, &first, &ry,
-                                      &vty);
-      if (rw == 0) done = true;  // every later pair of the cell was walked
-      if (rw != 1) break;
-      const PairDesc d = P.pair_desc[qq];
-      const PairState& S = P.pair[qq];
-      unsigned long long k2 = make_key((uint32_t)qq, 1u, (uint32_t)x);
-      Rng gm = make_rng(P, kStreamChain, (uint32_t)(cw.len + 1), (uint32_t)x);
-      MergeDecision m = first ? merge_decide_v(P, gm, r, vt, ry, vty, d.c1, d.c2, S.cc)
-                              : merge_decide_v(P, gm, ry, vty, r, vt, d.c1, d.c2, S.cc);
-      bool rm_x = first ? m.rm1 : m.rm2, rm_y = first ? m.rm2 : m.rm1;
-      // the chain ends before an event that is no absorb, or when the pool
-      // is full; that event is pending for the next round (kPendingTerm)
-      if (!(m.create && rm_x && m.new_group != 0) || !cw.append(pool, yy, qq | (rm_y ? kChainRemoves : 0), pos)) {
-        if (m.new_group == 0) set_status(P.ctr, kErrTimeout);
-        it_term[e] = make_int4(yy, qq | (first ? kTermFirst : 0), (int)pack_decision(m, gm.used()), __float_as_int(pos));
-        break;
+      if (from >= 32) {
+        batch_draw(P, x, s, t_next, true, B);
+        from = 0;
       }
-      claim_slot(P, yy, claim_key(P, k2), rm_y);
-      y = yy;
-      q = qq;
-      cls = S.cc + 1;
+      at = batch_first<KT, T, FLAT>(P, B, from, qxd, qxf, &n_tests);
+      if (at != 32 || B.n_in < 32) break;
+      s.at = B.end;
+      s.j = __shfl_sync(kFull, B.j, 31);
+      t_next = __shfl_sync(kFull, B.t, 31) + 1u;
+      from = 32;
     }
+    if (at == 32) done = s.stop < 0;  // every later pair of the cell was walked
+    if (at < 0 || at == 32) break;
+    t_next = __shfl_sync(kFull, B.t, at) + 1u;
+    s.at = __shfl_sync(kFull, B.at, at);
+    s.j = __shfl_sync(kFull, B.j, at);
+    from = at + 1;
+    const int yy = __shfl_sync(kFull, B.y, at), qq = __shfl_sync(kFull, B.q, at);
+    const int c1 = __shfl_sync(kFull, B.c1, at), c2 = __shfl_sync(kFull, B.c2, at);
+    const int cc = __shfl_sync(kFull, B.cc, at);
+    const bool first = __shfl_sync(kFull, B.first ? 1 : 0, at) != 0;
+    const double ry = __shfl_sync(kFull, B.ry, at), vty = __shfl_sync(kFull, B.vty, at);
+    pos = __shfl_sync(kFull, B.pos, at);
+    for (int sp = lane; sp < ns; sp += 32) vnew[sp] = vcur[sp] + P.vol[vol_at(P, yy, sp)];
+    double vt2, ms2;
+    totals(vnew, &vt2, &ms2);
+    const double r1 = first ? r : ry, r2 = first ? ry : r;
+    const double rr = vol2rad(P.benv.frac, lane == 1 && !flat1 ? merge_vol(P, r1, r2) : vt2);
+    const double rnew = __shfl_sync(kFull, rr, 0), rc = __shfl_sync(kFull, rr, 1);
+    Rng gm = make_rng(P, kStreamChain, (uint32_t)(cw.len + 1), (uint32_t)x);
+    const MergeDecision m = merge_decide_rc(P, gm, r1, first ? vt : vty, r2, first ? vty : vt, c1, c2, cc, rc);
+    const bool rm_x = first ? m.rm1 : m.rm2, rm_y = first ? m.rm2 : m.rm1;
+    // the chain ends before an event that is no absorb, or when the pool
+    // is full; that event is pending for the next round (kPendingTerm)
+    if (!(m.create && rm_x && m.new_group != 0) || !append(yy, qq | (rm_y ? kChainRemoves : 0), pos)) {
+      if (lead) {
+        if (m.new_group == 0) set_status(P.ctr, kErrTimeout);
+        A.it_term[e] = make_int4(yy, qq | (first ? kTermFirst : 0), (int)pack_decision(m, gm.used()),
+                                 __float_as_int(pos));
+      }
+      break;
+    }
+    if (lead) claim_slot(P, yy, claim_key(P, make_key((uint32_t)qq, 1u, (uint32_t)x)), rm_y);
+    __syncwarp();  // the claim is seen by the other lanes
+    if (lane >= from && lane < B.n_in && B.state != -1 && B.y == yy) batch_redraw(P, x, B);
+    q = qq;
+    cls = cc + 1;
+    double* v = vcur;
+    vcur = vnew;
+    vnew = v;
+    vt = vt2;
+    ms = ms2;
+    r = rnew;
+  }
+  if (lead) {
     // a chain that ended at its first event is that event alone
-    it_len[e] = cw.len > 1 ? cw.len : 0;
-    it_head[e] = cw.head;
-    it_done[e] = done ? 1 : 0;
+    A.it_len[e] = cw.len > 1 ? cw.len : 0;
+    A.it_head[e] = cw.head;
+    A.it_done[e] = done ? 1 : 0;
     if (n_tests) {
-      add_ll_warp(&P.ctr->tot_samp, (int)n_tests);
-      add_ll_warp(&P.ctr->walk_tests, (int)n_tests);
+      add_ll(&P.ctr->tot_samp, n_tests);
+      add_ll(&P.ctr->walk_tests, n_tests);
     }
+  }
+}
+
+// Bound by the longest chain: about 5 us an absorb for one thread, its FP64
+// pow, log and exp calls one after another; by a warp 1.5 (37,000 sedimenting
+// drops: 102 us a launch, now 34; 4000 in FP64: 57 and 33).
+constexpr int kChainThreads = 128;
+template <int KT, class T, bool FLAT>
+__global__ void __launch_bounds__(kChainThreads, 4) k_chain(ItemArgs A, ChainPool pool) {
+  __shared__ double sh_v[kChainThreads / 32][2 * kMaxSpec];
+  const long long n = *A.n_start;
+  const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+  if (n <= kWarpShare * (nt >> 5)) {
+    for (long long ci = tid >> 5; ci < n; ci += nt >> 5) {
+      do_chain_warp<KT, T, FLAT>(A, pool, A.start_list[ci], sh_v[threadIdx.x >> 5]);
+      __syncwarp();
+    }
+  } else {
+    // by item, not by the list: the chains then lie spread over the warps,
+    // and few of a warp's threads wait for one another
+    const long long n_it = *A.n_items;
+    for (long long e = tid; e < n_it; e += nt) do_chain<KT, T, FLAT>(A, pool, e);
   }
 }
 
@@ -1119,8 +1567,8 @@ __global__ void __launch_bounds__(32) k_apply_chain(const PopDev* pops, const in
           first_k = C_b == st.cell1;
           const int i = base + lane;
           Rng g = i == 0 ? merge_rng(P, key1) : make_rng(P, kStreamChain, (uint32_t)(i + 1), (uint32_t)x);
-          MergeDecision m = first_k ? merge_decide_v(P, g, r_b, vt_b, st.ry, st.vty, st.c1, st.c2, st.cc)
-                                    : merge_decide_v(P, g, st.ry, st.vty, r_b, vt_b, st.c1, st.c2, st.cc);
+          const MergeDecision m = merge_decide_v(P, g, first_k ? r_b : st.ry, first_k ? vt_b : st.vty,
+                                                 first_k ? st.ry : r_b, first_k ? st.vty : vt_b, st.c1, st.c2, st.cc);
           bool rm_x = first_k ? m.rm1 : m.rm2;
           rm_y_k = first_k ? m.rm2 : m.rm1;
           lost_x_k = first_k ? m.lost1 : m.lost2;

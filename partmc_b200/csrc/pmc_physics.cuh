@@ -265,11 +265,12 @@ struct BrownPart {
   double rad, diffus, speedsq, deltasq;
 };
 
-PMC_HD BrownPart brown_part(const BrownEnv& e, double vol, double den, bool* ok) {
+// rad is vol2rad(e.frac, vol); a sphere's mobility radius is the same number.
+PMC_HD BrownPart brown_part(const BrownEnv& e, double rad, double vol, double den, bool* ok) {
   BrownPart p;
   double temp = e.temp;
-  p.rad = vol2rad(e.frac, vol);
-  double rme = mobility_rad(e.frac, vol, e.fp, ok);
+  p.rad = rad;
+  double rme = e.frac.spherical ? rad : mobility_rad(e.frac, vol, e.fp, ok);
   double knud = e.gasfreepath / rme;
   double cunning = 1.0 + knud * (1.249 + 0.42 * exp(-0.87 / knud));
   p.diffus = (kBoltzmann * temp * cunning) / (6.0 * kPi * rme * e.viscosd);
@@ -296,8 +297,8 @@ PMC_HD T brown_pair(T rad_i, T diffus_i, T speedsq_i, T deltasq_i, T rad_j, T di
 
 // Full FP64 form in the reference's order, for k-bound tables and checks.
 PMC_HD double brown_kernel(const BrownEnv& e, double vi, double di, double vj, double dj, bool* ok) {
-  BrownPart a = brown_part(e, vi, di, ok);
-  BrownPart b = brown_part(e, vj, dj, ok);
+  BrownPart a = brown_part(e, vol2rad(e.frac, vi), vi, di, ok);
+  BrownPart b = brown_part(e, vol2rad(e.frac, vj), vj, dj, ok);
   double rad_sum = a.rad + b.rad;
   double diffus_sum = a.diffus + b.diffus;
   double tmp1 = rad_sum / (rad_sum + sqrt(a.deltasq + b.deltasq));
@@ -317,23 +318,35 @@ PMC_HD double fall_g(double r) {
   double stb = 32.0 * rhoa * (rhow - rhoa) * grav / (3.0 * eta * eta);
   double eta4 = (eta * eta) * (eta * eta);
   double phy = sigma * sigma * sigma * rhoa * rhoa / (eta4 * grav * (rhow - rhoa));
-  double py = pow(phy, 1.0 / 6.0);
   double rr = r * 1e2;
   double w = 0.0;
   if (rr <= 1e-3) {
     w = stok * (rr * rr + cunh * rr);
   } else if (rr > 1e-3 && rr <= 5.35e-2) {
     double x = log(stb * rr * rr * rr);
-    double y = 0.0;
-    for (int i = 1; i <= 7; i++) y = y + b[i - 1] * powi(x, i - 1);
+    // x**i by squaring, as powi forms them
+    double x2 = x * x, x4 = x2 * x2, y = 0.0;
+    y = y + b[0];
+    y = y + b[1] * x;
+    y = y + b[2] * x2;
+    y = y + b[3] * (x * x2);
+    y = y + b[4] * x4;
+    y = y + b[5] * (x * x4);
+    y = y + b[6] * (x2 * x4);
     double xrey = (1.0 + cunh / rr) * exp(y);
     w = xrey * eta / (2.0 * rhoa * rr);
   } else if (rr > 5.35e-2) {
     double bond = grav * (rhow - rhoa) * (rr * rr) / sigma;
     if (rr > 0.35) bond = grav * (rhow - rhoa) * (0.35 * 0.35) / sigma;
+    double py = pow(phy, 1.0 / 6.0);
     double x = log(16.0 * bond * py / 3.0);
-    double y = 0.0;
-    for (int i = 1; i <= 6; i++) y = y + c[i - 1] * powi(x, i - 1);
+    double x2 = x * x, x4 = x2 * x2, y = 0.0;
+    y = y + c[0];
+    y = y + c[1] * x;
+    y = y + c[2] * x2;
+    y = y + c[3] * (x * x2);
+    y = y + c[4] * x4;
+    y = y + c[5] * (x * x4);
     double xrey = py * exp(y);
     w = xrey * eta / (2.0 * rhoa * rr);
     if (rr > 0.35) w = xrey * eta / (2.0 * rhoa * 0.35);
@@ -651,6 +664,17 @@ PMC_HD U4 philox4x32_10(U4 ctr, uint32_t k0, uint32_t k1) {
   return ctr;
 }
 
+// The same as a call: a stream's uniforms are drawn at many places of a kernel,
+// and the block's instructions at each of them would be fetched cold by
+// kernels that run for 10 to 20 us.
+#ifdef __CUDACC__
+__host__ __device__ __noinline__ static U4 philox_call(U4 ctr, uint32_t k0, uint32_t k1) {
+  return philox4x32_10(ctr, k0, k1);
+}
+#else
+static inline U4 philox_call(U4 ctr, uint32_t k0, uint32_t k1) { return philox4x32_10(ctr, k0, k1); }
+#endif
+
 // uniform in (0, 1) with 53 random bits
 PMC_HD double u53(uint32_t a, uint32_t b) {
   uint64_t x = ((uint64_t)a << 21) ^ (uint64_t)(b >> 11);
@@ -670,7 +694,7 @@ struct Rng {
       : k0((uint32_t)seed), k1((uint32_t)(seed >> 32)), c0(a), c1(b), c2(c), n(0), have(0) {}
   PMC_HD double next() {
     if (have == 0) {
-      buf = philox4x32_10(U4{c0, c1, c2, n++}, k0, k1);
+      buf = philox_call(U4{c0, c1, c2, n++}, k0, k1);
       have = 2;
       return u53(buf.x, buf.y);
     }
@@ -682,7 +706,7 @@ struct Rng {
   PMC_HD void seek(uint32_t u) {
     n = (u + 1) / 2;
     if (u & 1u) {
-      buf = philox4x32_10(U4{c0, c1, c2, n - 1}, k0, k1);
+      buf = philox_call(U4{c0, c1, c2, n - 1}, k0, k1);
       have = 2;
     } else {
       have = 0;

@@ -86,7 +86,7 @@ def test_claim_generations_restart_after_a_smaller_upload(gpu_lib):
     slots must not lose to them."""
     import partmc_b200 as pm
     from partmc_b200 import aero_dist
-    pop = aero_dist.brown_20spec(2500, seed=6)
+    pop = aero_dist.brown_bimodal(20000, seed=6)
     st = pm.AeroState(pop.aero_data, pop.awa, seed=5)
     env = pm.EnvState(288.0, 1e5)
     first, rounds = None, 0
@@ -94,7 +94,7 @@ def test_claim_generations_restart_after_a_smaller_upload(gpu_lib):
         st.set_next_id(1)
         st.add_particles(pop.vol, pop.group)
         st.set_seed(9)
-        for _ in range(12):
+        for _ in range(6):
             pm.mc_coag(pm.COAG_KERNEL_TYPE_BROWN, env, pop.aero_data, st, 600.0)
             rounds += st.stats()["rounds"]
         got = st.particles()
