@@ -801,32 +801,4 @@ __global__ void __launch_bounds__(256) k_test(const PopDev* pops, const int* gpa
   }
 }
 
-// Round 0's merge decisions, one thread per accepted sample in sample order
-// (after the compaction): the decision (coagulate_weighting,
-// coagulation.F90:810-922) from the sample's own stream (merge_rng of its
-// key), stored in dec[e], and the claims on its two slots by it: a write
-// claim on a slot the merge removes or rewrites, a read claim on one it
-// keeps.
-__global__ void __launch_bounds__(256) k_decide(const PopDev* pops, const int* gpair_pop,
-                                                const long long* n_events, const unsigned long long* ev_key,
-                                                const int2* ev_c, const int* gp_c, uint32_t* dec) {
-  long long E = *n_events;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < E;
-       e += (long long)gridDim.x * blockDim.x) {
-    const PopDev& P = pops[gpair_pop[gp_c[e]]];
-    const unsigned long long key = ev_key[e];
-    const int p = (int)key_pair(key);
-    const int2 sl = ev_c[e];
-    const PairState& S = P.pair[p];
-    const PairDesc d = P.pair_desc[p];
-    const unsigned long long ck = claim_key(P, key);
-    Rng gm = merge_rng(P, key);
-    MergeDecision m = merge_decide(P, gm, sl.x, sl.y, d.c1, d.c2, S.cc);
-    if (m.new_group == 0) set_status(P.ctr, kErrTimeout);
-    dec[e] = pack_decision(m, gm.used());
-    claim_slot(P, sl.x, ck, m.rm1);
-    claim_slot(P, sl.y, ck, m.rm2);
-  }
-}
-
 }  // namespace pmc

@@ -98,68 +98,6 @@ __device__ __forceinline__ void kill_slot(const PopDev& P, int i) {
   P.cell[i] = -1;
 }
 
-// Resolve the events of a round: winner test, slot/id needs.  Event e has
-// key ev_key[e], slots ev[e], global pair ev_gp[e] and merge decision dec[e]
-// (drawn when the event was formed); the events are ordered by population.
-// A winning chain (ev_len[e] > 0) gets win 2 and the number of its events
-// whose claims hold (ev_app[e]).
-__global__ void k_resolve_set(const PopDev* pops, const int* gpair_pop, const long long* n_events,
-                              const unsigned long long* ev_key, const int2* ev, const int* ev_gp, int* need_slot,
-                              int* need_id, uint8_t* win, const uint32_t* dec, long long* n_losers, const int* ev_len,
-                              const int* ev_head, int* ev_app, ChainPool pool, int* chain_list, long long* n_chain) {
-  long long E = *n_events;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < E;
-       e += (long long)gridDim.x * blockDim.x) {
-    int gp = ev_gp[e];
-    const PopDev& P = pops[gpair_pop[gp]];
-    unsigned long long key = ev_key[e];
-    int p = (int)key_pair(key);
-    int2 sl = ev[e];
-    win[e] = 0;
-    need_slot[e] = 0;
-    need_id[e] = 0;
-    if (sl.x < 0 || sl.x >= P.cap || sl.y < 0 || sl.y >= P.cap || p >= P.n_pairs) {
-      bad_index(P.ctr, kBadEventSlot, sl.x < 0 || sl.x >= P.cap ? sl.x : sl.y);
-      continue;
-    }
-    uint32_t used;
-    MergeDecision m = unpack_decision(dec[e], &used);
-    unsigned long long ck = claim_key(P, key);
-    bool winner = holds_slot(P, sl.x, ck, m.rm1) && holds_slot(P, sl.y, ck, m.rm2);
-    if (!winner) {
-      add_ll_warp(n_losers, 1);
-      continue;
-    }
-    int len = ev_len[e];
-    if (len > 0) {
-      // a chain: its events apply as far as each partner's claim holds (the
-      // walking particle's is the first event's)
-      ChainReader rd(ev_head[e]);
-      uint32_t x = key_idx(key);
-      int app = 0;
-      for (int i = 0; i < len; i++) {
-        long long ix = rd.next(pool);
-        if (ix < 0) break;
-        int y = pool.y[ix], qw = pool.q[ix];
-        int q = qw & kChainPairMask;
-        if (y < 0 || y >= P.cap || q < 0 || q >= P.n_pairs) break;
-        if (!holds_slot(P, y, claim_key(P, make_key((uint32_t)q, 1u, x)), (qw & kChainRemoves) != 0)) break;
-        app++;
-      }
-      ev_app[e] = app;
-      win[e] = 2;
-      chain_list[inc_warp((unsigned long long*)n_chain)] = (int)e;
-      continue;
-    }
-    win[e] = 1;
-    if (m.create) {
-      need_slot[e] = (!m.rm1 && !m.rm2) ? 1 : 0;
-      bool keep1 = m.rm1 && !m.lost1, keep2 = m.rm2 && !m.lost2;
-      need_id[e] = (!keep1 && !keep2) ? 1 : 0;
-    }
-  }
-}
-
 // destination slot of a winning event that creates a particle (-1: none)
 __device__ __forceinline__ int event_dest(const MergeDecision& m, int s1, int s2, int slot_base,
                                           long long slot_rank) {
@@ -169,104 +107,85 @@ __device__ __forceinline__ int event_dest(const MergeDecision& m, int s1, int s2
   return slot_base + (int)slot_rank;
 }
 
-// Apply winning per-set events (coagulate, coagulation.F90:928-985), part 1:
-// the per-particle vectors, one thread per event.  The species of the two
-// sources (particle-major, each source a few cache lines) are added in blocks
-// of kMoveBlock: a block's loads are all issued before its sums are stored,
-// and the destination (which may be a source) is written species by species
-// after that species was read.  The components are gathered into local
-// arrays before any is written, in the order of the random selection
-// (computed from the stream position the test stored).  The summed volume and
-// mass go to the destination's caches for part 2; the water volumes of the
-// sources, which part 2 needs after the destination may have been
-// overwritten, go to ice[e].
 constexpr int kMoveBlock = 8;
 
-__global__ void __launch_bounds__(256) k_apply_move(const PopDev* pops, const int* gpair_pop,
-                                                    const long long* n_events, const unsigned long long* ev_key,
-                                                    const int2* ev, const int* ev_gp, const uint8_t* win,
-                                                    const uint32_t* dec, const long long* slot_rank,
-                                                    const int* slot_base, double2* ice) {
-  long long E = *n_events;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < E;
-       e += (long long)gridDim.x * blockDim.x) {
-    if (win[e] != 1) continue;  // chains apply in k_apply_chain
-    uint32_t used;
-    MergeDecision m = unpack_decision(dec[e], &used);
-    if (!m.create) continue;
-    int gp = ev_gp[e];
-    int pop = gpair_pop[gp];
-    const PopDev& P = pops[pop];
-    int2 sl = ev[e];
-    int s1 = sl.x, s2 = sl.y;
-    int dest = event_dest(m, s1, s2, slot_base[pop], m.rm1 || m.rm2 ? 0 : slot_rank[e]);
-    if (dest < 0 || dest >= P.cap) continue;  // reported by part 2
-    const int ns = P.n_spec;
-    const double* v1 = P.vol + vol_at(P, s1, 0);
-    const double* v2 = P.vol + vol_at(P, s2, 0);
-    double* vd = P.vol + vol_at(P, dest, 0);
-    if (P.i_water > 0) ice[e] = make_double2(v1[P.i_water - 1], v2[P.i_water - 1]);
-    // components: every source entry is read before the first write
-    int na = P.ncomp[s1], nb = P.ncomp[s2];
-    na = na < kMaxComponent ? na : kMaxComponent;
-    nb = nb < kMaxComponent ? nb : kMaxComponent;
-    int ca[kMaxComponent], cb[kMaxComponent];
-    double ta[kMaxComponent], tb[kMaxComponent];
+// The particle of a winning event that creates one, its per-particle vectors:
+// the species of the two sources (particle-major, each source a few cache
+// lines) are added in blocks of kMoveBlock: a block's loads are all issued
+// before its sums are stored, and the destination (which may be a source) is
+// written species by species after that species was read.  The components are
+// gathered into local arrays before any is written, in the order of the
+// random selection (computed from the stream position the test stored).
+// Returns the sources' water volumes, read before the destination may be
+// overwritten.
+__device__ __forceinline__ double2 move_vectors(const PopDev& P, unsigned long long key, int s1, int s2, int dest,
+                                                uint32_t used) {
+  const int ns = P.n_spec;
+  const double* v1 = P.vol + vol_at(P, s1, 0);
+  const double* v2 = P.vol + vol_at(P, s2, 0);
+  double* vd = P.vol + vol_at(P, dest, 0);
+  const double2 ice = P.i_water > 0 ? make_double2(v1[P.i_water - 1], v2[P.i_water - 1]) : make_double2(0.0, 0.0);
+  // components: every source entry is read before the first write
+  int na = P.ncomp[s1], nb = P.ncomp[s2];
+  na = na < kMaxComponent ? na : kMaxComponent;
+  nb = nb < kMaxComponent ? nb : kMaxComponent;
+  int ca[kMaxComponent], cb[kMaxComponent];
+  double ta[kMaxComponent], tb[kMaxComponent];
+  for (int k = 0; k < na; k++) {
+    ca[k] = P.csrc[comp_at(s1, k)];
+    ta[k] = P.ctime[comp_at(s1, k)];
+  }
+  for (int k = 0; k < nb; k++) {
+    cb[k] = P.csrc[comp_at(s2, k)];
+    tb[k] = P.ctime[comp_at(s2, k)];
+  }
+  // totals in the reference's order (species 1..n)
+  double vt = 0.0, ms = 0.0;
+  for (int s0 = 0; s0 < ns; s0 += kMoveBlock) {
+    double x1[kMoveBlock], x2[kMoveBlock];
+#pragma unroll
+    for (int j = 0; j < kMoveBlock; j++) {
+      x1[j] = s0 + j < ns ? v1[s0 + j] : 0.0;
+      x2[j] = s0 + j < ns ? v2[s0 + j] : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < kMoveBlock; j++) {
+      if (s0 + j < ns) {
+        double v = x1[j] + x2[j];
+        vt = vt + v;
+        ms = ms + v * P.density[s0 + j];
+        vd[s0 + j] = v;
+      }
+    }
+  }
+  int n1_new = na, n2_new = nb;
+  if (na + nb > kMaxComponent) {
+    int sa[kMaxComponent], sb[kMaxComponent];
+    Rng g = merge_rng(P, key);
+    g.seek(used);
+    coag_components(g, na, P.nprim[s1], nb, P.nprim[s2], &n1_new, &n2_new, sa, sb);
+    for (int k = 0; k < n1_new; k++) {
+      P.csrc[comp_at(dest, k)] = ca[sa[k] - 1];
+      P.ctime[comp_at(dest, k)] = ta[sa[k] - 1];
+    }
+    for (int k = 0; k < n2_new; k++) {
+      P.csrc[comp_at(dest, n1_new + k)] = cb[sb[k] - 1];
+      P.ctime[comp_at(dest, n1_new + k)] = tb[sb[k] - 1];
+    }
+  } else {
     for (int k = 0; k < na; k++) {
-      ca[k] = P.csrc[comp_at(s1, k)];
-      ta[k] = P.ctime[comp_at(s1, k)];
+      P.csrc[comp_at(dest, k)] = ca[k];
+      P.ctime[comp_at(dest, k)] = ta[k];
     }
     for (int k = 0; k < nb; k++) {
-      cb[k] = P.csrc[comp_at(s2, k)];
-      tb[k] = P.ctime[comp_at(s2, k)];
+      P.csrc[comp_at(dest, na + k)] = cb[k];
+      P.ctime[comp_at(dest, na + k)] = tb[k];
     }
-    // totals in the reference's order (species 1..n)
-    double vt = 0.0, ms = 0.0;
-    for (int s0 = 0; s0 < ns; s0 += kMoveBlock) {
-      double x1[kMoveBlock], x2[kMoveBlock];
-#pragma unroll
-      for (int j = 0; j < kMoveBlock; j++) {
-        x1[j] = s0 + j < ns ? v1[s0 + j] : 0.0;
-        x2[j] = s0 + j < ns ? v2[s0 + j] : 0.0;
-      }
-#pragma unroll
-      for (int j = 0; j < kMoveBlock; j++) {
-        if (s0 + j < ns) {
-          double v = x1[j] + x2[j];
-          vt = vt + v;
-          ms = ms + v * P.density[s0 + j];
-          vd[s0 + j] = v;
-        }
-      }
-    }
-    int n1_new = na, n2_new = nb;
-    if (na + nb > kMaxComponent) {
-      int sa[kMaxComponent], sb[kMaxComponent];
-      Rng g = merge_rng(P, ev_key[e]);
-      g.seek(used);
-      coag_components(g, na, P.nprim[s1], nb, P.nprim[s2], &n1_new, &n2_new, sa, sb);
-      for (int k = 0; k < n1_new; k++) {
-        P.csrc[comp_at(dest, k)] = ca[sa[k] - 1];
-        P.ctime[comp_at(dest, k)] = ta[sa[k] - 1];
-      }
-      for (int k = 0; k < n2_new; k++) {
-        P.csrc[comp_at(dest, n1_new + k)] = cb[sb[k] - 1];
-        P.ctime[comp_at(dest, n1_new + k)] = tb[sb[k] - 1];
-      }
-    } else {
-      for (int k = 0; k < na; k++) {
-        P.csrc[comp_at(dest, k)] = ca[k];
-        P.ctime[comp_at(dest, k)] = ta[k];
-      }
-      for (int k = 0; k < nb; k++) {
-        P.csrc[comp_at(dest, na + k)] = cb[k];
-        P.ctime[comp_at(dest, na + k)] = tb[k];
-      }
-    }
-    P.vtot[dest] = vt;
-    P.mass[dest] = ms;
-    P.ncomp[dest] = n1_new + n2_new;
   }
+  P.vtot[dest] = vt;
+  P.mass[dest] = ms;
+  P.ncomp[dest] = n1_new + n2_new;
+  return ice;
 }
 
 // particle fields that coag_scalars reads (component lists excluded)
@@ -282,26 +201,31 @@ __device__ __forceinline__ void load_scalars(const PopDev& P, int i, PMeta& m) {
   m.frozen = P.frozen[i];
 }
 
-// Part 2, one thread per event: removals, the scalar fields of the
-// coagulated particle, its radius, bin and pair-test record.  Every slot an
-// event removes or rewrites is stamped with the round's claim generation,
-// and dest[e] gets the slot of the particle the event made (-1 if none).
-__global__ void k_apply_set(const PopDev* pops, const int* gpair_pop, const long long* n_events,
-                            const unsigned long long* ev_key, const int2* ev, const int* ev_gp,
-                            const uint8_t* win, const uint32_t* dec, const long long* slot_rank,
-                            const long long* id_rank, const int* slot_base, const long long* id_base,
-                            const double2* ice, const uint8_t* ev_done, int* dest_out, unsigned long long* ev_key_w,
-                            int2* ev_w, int* gp_w, float* pos_w, uint32_t* dec_w, const int4* ev_term,
-                            const long long* pop_pair_base) {
+// Apply winning per-set events (coagulate, coagulation.F90:928-985), one
+// thread per event: the coagulated particle's vectors (move_vectors), the
+// removals, its scalar fields, its radius, bin and pair-test record.  Among
+// the round's winners a slot is written by one event or read by any number, so
+// the events need no order among themselves.  Every slot an event removes or
+// rewrites is stamped with the round's claim generation, and dest_out[e] gets
+// the slot of the particle the event made (-1 if none).  One launch for what
+// were two (vectors, then scalars), with the event's words loaded once.
+__global__ void __launch_bounds__(256) k_apply(const PopDev* pops, const int* gpair_pop, const long long* n_events,
+                                               const uint8_t* win, const long long* slot_rank,
+                                               const long long* id_rank, const int* slot_base,
+                                               const long long* id_base, const uint8_t* ev_done, int* dest_out,
+                                               unsigned long long* ev_key, int2* ev, int* ev_gp, float* ev_pos,
+                                               uint32_t* dec, const int4* ev_term, const long long* pop_pair_base) {
   long long E = *n_events;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < E;
        e += (long long)gridDim.x * blockDim.x) {
+    if (win[e] == 2) continue;  // a chain: k_apply_chain's
     dest_out[e] = -1;
     if (win[e] != 1) continue;
     int gp = ev_gp[e];
     int pop = gpair_pop[gp];
     const PopDev& P = pops[pop];
-    int p = (int)key_pair(ev_key[e]);
+    const unsigned long long key = ev_key[e];
+    int p = (int)key_pair(key);
     int2 sl = ev[e];
     int s1 = sl.x, s2 = sl.y;
     uint32_t gen = *P.gen_p;
@@ -332,7 +256,7 @@ __global__ void k_apply_set(const PopDev* pops, const int* gpair_pop, const long
     PMeta a, b, c;
     load_scalars(P, s1, a);
     load_scalars(P, s2, b);
-    double2 wi = P.i_water > 0 ? ice[e] : make_double2(0.0, 0.0);
+    const double2 wi = move_vectors(P, key, s1, s2, dest, used);
     coag_scalars(a, wi.x, b, wi.y, c);
     P.grp[dest] = m.new_group;
     P.cls[dest] = P.pair[p].cc + 1;
@@ -365,13 +289,13 @@ __global__ void k_apply_set(const PopDev* pops, const int* gpair_pop, const long
       const int4 t = ev_term[e];
       const int tq = t.y & (kTermFirst - 1);
       const bool tfirst = (t.y & kTermFirst) != 0;
-      ev_key_w[e] = make_key((uint32_t)tq, 1u, (uint32_t)dest);
-      ev_w[e] = tfirst ? make_int2(dest, t.x) : make_int2(t.x, dest);
-      gp_w[e] = (int)(pop_pair_base[pop] + tq);
-      pos_w[e] = __int_as_float(t.w);
-      dec_w[e] = (uint32_t)t.z;
+      ev_key[e] = make_key((uint32_t)tq, 1u, (uint32_t)dest);
+      ev[e] = tfirst ? make_int2(dest, t.x) : make_int2(t.x, dest);
+      ev_gp[e] = (int)(pop_pair_base[pop] + tq);
+      ev_pos[e] = __int_as_float(t.w);
+      dec[e] = (uint32_t)t.z;
       dest_out[e] = kPendingTerm;
-    } else if (!(key_kind(ev_key[e]) == 1u && ev_done[e])) {
+    } else if (!(key_kind(key) == 1u && ev_done[e])) {
       dest_out[e] = dest;  // a walk that ran to its end stops
     }
     if (m.rm1 && dest != s1) kill_slot(P, s1);
@@ -1472,6 +1396,7 @@ __global__ void __launch_bounds__(32) k_apply_chain(const PopDev* pops, const in
       unsigned long long key1 = ev_key[e];
       int x = (int)key_idx(key1);
       int app = ev_app[e];
+      if (lane == 0) dest_out[e] = -1;
       if (x < 0 || x >= P.cap) {
         if (lane == 0) bad_index(P.ctr, kBadEventSlot, x);
         continue;
