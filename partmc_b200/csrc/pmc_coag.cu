@@ -187,52 +187,211 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lb(ScanJobs jobs, unsigne
 // small helper kernels
 
 
-// accepted samples of round 0 in sample order: event e gets its key (pair,
-// sample), its two slots, its global pair and its position in the pair's
-// test sequence ((s + 1) / n_samp: the part of the pair done after it)
-__global__ void k_compact_flags(const uint8_t* flag, const long long* off, const long long* n_samples,
-                                const int2* ev, const int* ev_gp, const int* gpair_local, const long long* work_off,
-                                unsigned long long* ev_key, int2* ev_c, int* gp_c, float* ev_pos, int* ev_len,
-                                int4* ev_term) {
-  long long n = *n_samples;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    if (flag[i]) {
-      long long e = off[i];
-      int gp = ev_gp[i];
-      long long s = i - work_off[gp], ns = work_off[gp + 1] - work_off[gp];
-      ev_key[e] = make_key((uint32_t)gpair_local[gp], 0u, (uint32_t)s);
-      ev_c[e] = ev[i];
-      gp_c[e] = gp;
-      ev_pos[e] = (float)((double)(s + 1) / (double)ns);
-      ev_len[e] = 0;
-      ev_term[e] = no_term();
+// The exclusive prefix of a tile's sum (62 bits) over the tiles before it, by
+// the block's first warp (decoupled look-back, 32 predecessors at a time; see
+// k_scan_lb for the status words).  Tiles are numbered in the order blocks
+// start, so a tile only waits on running blocks.
+__device__ unsigned long long tile_prefix(unsigned long long* st, long long tile, unsigned long long agg,
+                                          unsigned long long* err) {
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr unsigned long long kMask = (1ULL << 62) - 1;
+  const int lane = threadIdx.x & 31;
+  if (tile == 0) {
+    if (lane == 0) atomicExch(&st[0], scan_word(2u, (long long)agg));
+    return 0ULL;
+  }
+  if (lane == 0) atomicExch(&st[tile], scan_word(1u, (long long)agg));
+  unsigned long long excl = 0ULL;
+  int spins = 0;
+  for (long long base = tile - 1; base >= 0;) {
+    const long long i = base - lane;
+    const unsigned long long w = i >= 0 ? *(volatile unsigned long long*)&st[i] : (2ULL << 62);
+    const unsigned flag = (unsigned)(w >> 62);
+    const unsigned m2 = __ballot_sync(kFull, flag == 2u), m0 = __ballot_sync(kFull, flag == 0u);
+    const unsigned upto = m2 ? (m2 & (0u - m2)) * 2u - 1u : kFull;  // lanes to the nearest inclusive prefix
+    if (m0 & upto) {
+      if (++spins > kScanSpinLimit) {
+        if (lane == 0) atomicAdd(err, 1ULL);
+        break;
+      }
+      __nanosleep(20);
+      continue;
     }
+    unsigned long long v = ((upto >> lane) & 1u) ? (w & kMask) : 0ULL;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    excl += v;
+    if (m2) break;
+    base -= 32;
+  }
+  if (lane == 0) atomicExch(&st[tile], scan_word(2u, (long long)((excl + agg) & kMask)));
+  return excl;
 }
 
-// the events a later round's items made, in item order
-__global__ void k_compact_items(const uint8_t* it_flag, const long long* off, const long long* n_items,
-                                const unsigned long long* it_key, const int2* it_c, const int* it_gp,
-                                const float* it_pos, const int* it_len, const int* it_head, const uint8_t* it_done,
-                                const uint32_t* it_dec, const int4* it_term, unsigned long long* ev_key, int2* ev_c,
-                                int* gp_c, float* ev_pos, int* ev_len, int* ev_head, uint8_t* ev_done, uint32_t* dec,
-                                int4* ev_term, const long long* grouped) {
-  long long n = *n_items;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    if (it_flag[i]) {
-      long long e = grouped ? grouped[i] : off[i];
-      if (e < 0) continue;
-      ev_key[e] = it_key[i];
-      ev_c[e] = it_c[i];
-      gp_c[e] = it_gp[i];
-      ev_pos[e] = it_pos[i];
-      ev_len[e] = it_len[i];
-      ev_head[e] = it_head[i];
-      ev_done[e] = it_done[i];
-      dec[e] = it_dec[i];
-      ev_term[e] = it_term[i];
+// what a tiled kernel shares between its blocks: status words (zero between
+// launches), tile and finished-block counters, give-ups
+struct TileCtl {
+  unsigned long long* status;
+  unsigned *tile_ctr, *done_ctr;
+  unsigned long long* err;
+};
+
+// the block's tile, in the order blocks start
+__device__ __forceinline__ long long take_tile(const TileCtl& T) {
+  __shared__ unsigned tile_sh;
+  if (threadIdx.x == 0) {
+    const unsigned t = atomicAdd(T.tile_ctr, 1u);
+    if (t == gridDim.x - 1) *T.tile_ctr = 0;  // the last claimant re-arms the counter
+    tile_sh = t;
+  }
+  __syncthreads();
+  return tile_sh;
+}
+
+// true in the last block to come here, which then sees what the others wrote
+// and has cleared the status words for the next launch
+__device__ __forceinline__ bool last_block(const TileCtl& T) {
+  __shared__ bool last_sh;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last_sh = atomicAdd(T.done_ctr, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last_sh) return false;
+  __threadfence();
+  for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) T.status[k] = 0ULL;
+  if (threadIdx.x == 0) *T.done_ctr = 0;
+  return true;
+}
+
+// The events of a round in order, from the flagged samples (round 0) or items:
+// flags are counted, ranked and their events written in one launch.  A tile is
+// small so that a round of a few thousand events still spreads over the chip.
+constexpr int kCompactThreads = 256;
+constexpr int kCompactTile = 4 * kCompactThreads;
+
+struct CompactArgs {
+  const uint8_t* flag;
+  const long long* n;  // flags
+  long long* n_events;
+  TileCtl ctl;
+  // the events
+  unsigned long long* ev_key;
+  int2* ev_c;
+  int* gp_c;
+  float* ev_pos;
+  int* ev_len;
+  int4* ev_term;
+  uint32_t* dec;
+};
+
+// places of the tile's flagged entries: sh_idx[r] is the tile's r-th, and the
+// tile's first event is returned
+__device__ long long compact_tile(const CompactArgs& A, int* sh_idx, int* count) {
+  __shared__ unsigned long long excl_sh;
+  const long long n = *A.n, n_tiles = (n + kCompactTile - 1) / kCompactTile;
+  const long long tile = take_tile(A.ctl);
+  if (tile >= n_tiles) {
+    if (n_tiles == 0 && tile == 0 && threadIdx.x == 0) *A.n_events = 0;
+    *count = 0;
+    return 0;
+  }
+  const long long base = tile * kCompactTile + 4 * threadIdx.x;
+  uchar4 f = make_uchar4(0, 0, 0, 0);
+  if (base + 4 <= n) f = *reinterpret_cast<const uchar4*>(A.flag + base);
+  else {
+    if (base < n) f.x = A.flag[base];
+    if (base + 1 < n) f.y = A.flag[base + 1];
+    if (base + 2 < n) f.z = A.flag[base + 2];
+  }
+  const int c = (f.x != 0) + (f.y != 0) + (f.z != 0) + (f.w != 0);
+  int tot;
+  int r = block_excl_scan(c, &tot);
+  const int i = 4 * (int)threadIdx.x;
+  if (f.x) sh_idx[r++] = i;
+  if (f.y) sh_idx[r++] = i + 1;
+  if (f.z) sh_idx[r++] = i + 2;
+  if (f.w) sh_idx[r++] = i + 3;
+  if (threadIdx.x < 32) {
+    const unsigned long long e = tile_prefix(A.ctl.status, tile, (unsigned long long)tot, A.ctl.err);
+    if (threadIdx.x == 0) {
+      excl_sh = e;
+      if (tile == n_tiles - 1) *A.n_events = (long long)e + tot;
     }
+  }
+  __syncthreads();
+  *count = tot;
+  for (int k = threadIdx.x; k < tot; k += kCompactThreads) sh_idx[k] += (int)(tile * kCompactTile);
+  __syncthreads();
+  return (long long)excl_sh;
+}
+
+// Round 0: accepted samples in sample order.  Event e gets its key (pair,
+// sample), its two slots, its global pair and its position in the pair's test
+// sequence ((s + 1) / n_samp: the part of the pair done after it), its merge
+// decision (coagulate_weighting, coagulation.F90:810-922) from the sample's
+// own stream (merge_rng of its key), and the claims on its two slots by it: a
+// write claim on a slot the merge removes or rewrites, a read claim on one it
+// keeps.  One launch for what were three (scan, compaction, decisions).
+__global__ void __launch_bounds__(kCompactThreads) k_compact_samples(CompactArgs A, const PopDev* pops,
+                                                                     const int* gpair_pop, const int* gpair_local,
+                                                                     const int2* ev, const int* ev_gp,
+                                                                     const long long* work_off) {
+  __shared__ int sh_idx[kCompactTile];
+  int count;
+  const long long e0 = compact_tile(A, sh_idx, &count);
+  for (int r = threadIdx.x; r < count; r += kCompactThreads) {
+    const long long i = sh_idx[r], e = e0 + r;
+    const int gp = ev_gp[i];
+    const int2 sl = ev[i];
+    const long long w0 = work_off[gp];
+    const long long s = i - w0, ns = work_off[gp + 1] - w0;
+    const int p = gpair_local[gp];
+    const PopDev& P = pops[gpair_pop[gp]];
+    const unsigned long long key = make_key((uint32_t)p, 0u, (uint32_t)s);
+    A.ev_key[e] = key;
+    A.ev_c[e] = sl;
+    A.gp_c[e] = gp;
+    A.ev_pos[e] = (float)((double)(s + 1) / (double)ns);
+    A.ev_len[e] = 0;
+    A.ev_term[e] = no_term();
+    const PairState& S = P.pair[p];
+    const PairDesc d = P.pair_desc[p];
+    Rng gm = merge_rng(P, key);
+    const MergeDecision m = merge_decide(P, gm, sl.x, sl.y, d.c1, d.c2, S.cc);
+    if (m.new_group == 0) set_status(P.ctr, kErrTimeout);
+    A.dec[e] = pack_decision(m, gm.used());
+    const unsigned long long ck = claim_key(P, key);
+    claim_slot(P, sl.x, ck, m.rm1);
+    claim_slot(P, sl.y, ck, m.rm2);
+  }
+  last_block(A.ctl);
+}
+
+// Later rounds: the events the items made, in item order (grouped: at the
+// places group_by_pop gave them)
+__global__ void __launch_bounds__(kCompactThreads) k_compact_items(CompactArgs A, const unsigned long long* it_key,
+                                                                   const int2* it_c, const int* it_gp,
+                                                                   const float* it_pos, const int* it_len,
+                                                                   const int* it_head, const uint8_t* it_done,
+                                                                   const uint32_t* it_dec, const int4* it_term,
+                                                                   int* ev_head, uint8_t* ev_done,
+                                                                   const long long* grouped) {
+  __shared__ int sh_idx[kCompactTile];
+  int count;
+  const long long e0 = compact_tile(A, sh_idx, &count);
+  for (int r = threadIdx.x; r < count; r += kCompactThreads) {
+    const long long i = sh_idx[r], e = grouped ? grouped[i] : e0 + r;
+    if (e < 0) continue;
+    A.ev_key[e] = it_key[i];
+    A.ev_c[e] = it_c[i];
+    A.gp_c[e] = it_gp[i];
+    A.ev_pos[e] = it_pos[i];
+    A.ev_len[e] = it_len[i];
+    ev_head[e] = it_head[i];
+    ev_done[e] = it_done[i];
+    A.dec[e] = it_dec[i];
+    A.ev_term[e] = it_term[i];
+  }
+  last_block(A.ctl);
 }
 
 // target operations of round 0, in the reference's backwards target order
@@ -302,13 +461,11 @@ __device__ long long first_event_of(int k, long long E, const int* ev_gp, const 
 // stored in per_pop for the host); per-particle counts were summed into
 // per_pop by k_count_per_pop.  The slot and ID counters of each population
 // advance here by the round's allocations: the apply kernels read only the
-// bases.  One block; populations in tiles of blockDim.x.
-__global__ void k_alloc_bases(const PopDev* pops, int n_pop, const long long* n_events, const int* ev_gp,
-                              const int* gpair_pop, int has_set, const long long* rank_slot_set,
-                              const long long* rank_id_set, int* per_pop, int* set_slot_base,
-                              long long* set_id_base, int* pp_slot_base, long long* pp_id_base) {
+// bases.  By one block; populations in tiles of blockDim.x.
+__device__ void alloc_bases(const PopDev* pops, int n_pop, long long E, const int* ev_gp, const int* gpair_pop,
+                            const long long* rank_slot_set, const long long* rank_id_set, int* per_pop,
+                            int* set_slot_base, long long* set_id_base, int* pp_slot_base, long long* pp_id_base) {
   long long carry[4] = {0, 0, 0, 0};
-  long long E = has_set ? *n_events : 0;
   for (int base = 0; base < n_pop; base += blockDim.x) {
     int k = base + threadIdx.x;
     long long cnt[4] = {0, 0, 0, 0};
@@ -338,6 +495,118 @@ __global__ void k_alloc_bases(const PopDev* pops, int n_pop, const long long* n_
     }
     for (int j = 0; j < 4; j++) carry[j] += tot[j];
   }
+}
+
+// Resolve the events of a round: winner test, slot/id needs.  Event e has
+// key ev_key[e], slots ev[e], global pair ev_gp[e] and merge decision dec[e]
+// (drawn when the event was formed); the events are ordered by population.
+// A winning chain (ev_len[e] > 0) gets win 2 and the number of its events
+// whose claims hold (ev_app[e]).  The same launch ranks the winners' new slots
+// and IDs (31 bits of a status word each) and, in its last block, sets the
+// populations' bases (alloc_bases): three launches in one.
+constexpr int kResolveMin = 64;  // smallest block of k_resolve
+
+struct ResolveArgs {
+  const PopDev* pops;
+  const int* gpair_pop;
+  const long long* n_events;  // null: the round has no events, only bases to set
+  const unsigned long long* ev_key;
+  const int2* ev;
+  const int* ev_gp;
+  uint8_t* win;
+  const uint32_t* dec;
+  long long* n_losers;
+  const int *ev_len, *ev_head;
+  int* ev_app;
+  ChainPool pool;
+  int* chain_list;
+  long long* n_chain;
+  long long *rank_slot, *rank_id;
+  TileCtl ctl;
+  int n_pop;
+  int *per_pop, *set_slot_base, *pp_slot_base;
+  long long *set_id_base, *pp_id_base;
+};
+
+// 1 if event e wins (2: a chain), with its needs
+__device__ __forceinline__ int resolve_event(const ResolveArgs& A, long long e, int* need_slot, int* need_id) {
+  *need_slot = *need_id = 0;
+  const int gp = A.ev_gp[e];
+  const PopDev& P = A.pops[A.gpair_pop[gp]];
+  const unsigned long long key = A.ev_key[e];
+  const int p = (int)key_pair(key);
+  const int2 sl = A.ev[e];
+  const int len = A.ev_len[e];
+  uint32_t used;
+  const MergeDecision m = unpack_decision(A.dec[e], &used);
+  if (sl.x < 0 || sl.x >= P.cap || sl.y < 0 || sl.y >= P.cap || p >= P.n_pairs) {
+    bad_index(P.ctr, kBadEventSlot, sl.x < 0 || sl.x >= P.cap ? sl.x : sl.y);
+    return 0;
+  }
+  const unsigned long long ck = claim_key(P, key);
+  if (!(holds_slot(P, sl.x, ck, m.rm1) && holds_slot(P, sl.y, ck, m.rm2))) {
+    add_ll_warp(A.n_losers, 1);
+    return 0;
+  }
+  if (len > 0) {
+    // a chain: its events apply as far as each partner's claim holds (the
+    // walking particle's is the first event's)
+    ChainReader rd(A.ev_head[e]);
+    const uint32_t x = key_idx(key);
+    int app = 0;
+    for (int i = 0; i < len; i++) {
+      const long long ix = rd.next(A.pool);
+      if (ix < 0) break;
+      const int y = A.pool.y[ix], qw = A.pool.q[ix];
+      const int q = qw & kChainPairMask;
+      if (y < 0 || y >= P.cap || q < 0 || q >= P.n_pairs) break;
+      if (!holds_slot(P, y, claim_key(P, make_key((uint32_t)q, 1u, x)), (qw & kChainRemoves) != 0)) break;
+      app++;
+    }
+    A.ev_app[e] = app;
+    A.chain_list[inc_warp((unsigned long long*)A.n_chain)] = (int)e;
+    return 2;
+  }
+  if (m.create) {
+    *need_slot = (!m.rm1 && !m.rm2) ? 1 : 0;
+    const bool keep1 = m.rm1 && !m.lost1, keep2 = m.rm2 && !m.lost2;
+    *need_id = (!keep1 && !keep2) ? 1 : 0;
+  }
+  return 1;
+}
+
+__global__ void __launch_bounds__(256) k_resolve(ResolveArgs A) {
+  __shared__ unsigned long long excl_sh;
+  const long long E = A.n_events ? *A.n_events : 0;
+  const int tb = blockDim.x;  // events of a tile
+  const long long n_tiles = (E + tb - 1) / tb;
+  const long long tile = take_tile(A.ctl);
+  if (tile < n_tiles) {
+    const long long e = tile * tb + threadIdx.x;
+    int ns = 0, ni = 0;
+    if (e < E) A.win[e] = (uint8_t)resolve_event(A, e, &ns, &ni);
+    // at most 256 of each in a tile: one scan of both
+    int tot;
+    const int pre = block_excl_scan(ns | (ni << 16), &tot);
+    if (threadIdx.x < 32) {
+      const unsigned long long agg = (unsigned long long)(tot & 0xffff) | ((unsigned long long)(tot >> 16) << 31);
+      const unsigned long long x = tile_prefix(A.ctl.status, tile, agg, A.ctl.err);
+      if (threadIdx.x == 0) excl_sh = x;
+    }
+    __syncthreads();
+    const long long s0 = (long long)(excl_sh & 0x7fffffffULL), i0 = (long long)(excl_sh >> 31);
+    if (e < E) {
+      A.rank_slot[e] = s0 + (pre & 0xffff);
+      A.rank_id[e] = i0 + (pre >> 16);
+    }
+    if (tile == n_tiles - 1 && threadIdx.x == 0) {
+      A.rank_slot[E] = s0 + (tot & 0xffff);
+      A.rank_id[E] = i0 + (tot >> 16);
+    }
+  }
+  if (last_block(A.ctl))
+    alloc_bases(A.pops, A.n_pop, E, A.ev_gp, A.gpair_pop, A.rank_slot, A.rank_id, A.per_pop, A.set_slot_base,
+                A.set_id_base, A.pp_slot_base, A.pp_id_base);
 }
 
 // need[q] of target operation q summed per population (op_pop[q])
@@ -872,6 +1141,14 @@ struct Tuner {
   std::vector<cudaEvent_t> spare;
 };
 
+void pool_release(int dev);
+struct PoolRef {  // a context's hold on its device's memory pool
+  int dev = -1;
+  ~PoolRef() {
+    if (dev >= 0) pool_release(dev);
+  }
+};
+
 struct Ctx {
   int n_pop = 1, n_spec = 1, n_group = 1, n_class = 1, i_water = 0;
   std::vector<double> density;
@@ -893,6 +1170,10 @@ struct Ctx {
   bool use_graph = true;
   cudaStream_t cap_stream = nullptr;  // capture stream
   cudaMemPool_t mem = nullptr;        // the populations' arrays (dalloc)
+  PoolRef mem_ref;
+  cudaStream_t side_stream = nullptr;  // a branch of a captured step
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  bool fork = false;                   // capturing: independent launches go to branches
   cudaGraph_t rg_graph = nullptr;
   cudaGraphExec_t rg_exec = nullptr;
   std::vector<long long> rg_key;
@@ -944,9 +1225,7 @@ struct Ctx {
   DevBuf<int> ev_len, ev_head, ev_app;  // chains: events, first chunk, events applied
   DevBuf<uint8_t> ev_done;   // chains: the walk ran to the end
   DevBuf<int> chain_list;    // the round's winning chains (round_dev[4] of them)
-  DevBuf<double2> ice_set;   // water volumes of the sources of each event
   DevBuf<int2> ev;
-  DevBuf<long long> flag_off;
   // a later round's items (one per event of the round before) and what they made
   DevBuf<uint8_t> it_flag, it_done;
   DevBuf<unsigned long long> it_key;
@@ -962,12 +1241,11 @@ struct Ctx {
   long long ppw_cap = 0;
   long long op_cap = 0;   // room in the target-operation arrays this round
   bool pp_step = false;   // the step has target operations (per-particle path)
-  DevBuf<long long> it_off;
   // chain events of a round (ChainPool), in chunks
   DevBuf<int> ch_y, ch_q;
   DevBuf<float> ch_pos;
   long long ch_chunks = 0;
-  DevBuf<int> need_slot_set, need_id_set, need_slot_pp, need_id_pp, lost_pp;
+  DevBuf<int> need_slot_pp, need_id_pp, lost_pp;
   DevBuf<long long> rank_slot_set, rank_id_set, rank_slot_pp, rank_id_pp, lost_off;
   DevBuf<int> op_pop, op_pair, op_slot, op_k, r_pop, r_pair, r_slot, r_k;
   DevBuf<unsigned long long> op_key, r_key;
@@ -1024,15 +1302,55 @@ struct Ctx {
   Fractal frac = fractal_spherical();
 };
 
-// Population arrays come from a memory pool of the context, in the order of
-// its stream: a server's slot is emptied and filled again for every job, and
+// Population arrays come from a memory pool, in the order of the context's
+// stream: a server's slot is emptied and filled again for every job, and
 // the 76 cudaMalloc and cudaFree calls of that (each a device
 // synchronisation) made emptying and uploading take 19.2 ms at 1e6 particles
 // of 20 species, 3.0 ms of it the copy, and 3.2 ms a population in a context
 // of 256; from the pool 3.3 and 0.4 ms.
-// The pool keeps at most kPoolKeep bytes that are not in use past a
-// synchronisation and goes with its context.
+// One pool per device, shared by its contexts (the driver orders memory that
+// moves between their streams; a pool per context took 1 ms to create); it
+// keeps at most kPoolKeep bytes that are not in use past a synchronisation,
+// and the last context to go destroys it.
 constexpr uint64_t kPoolKeep = 4ULL << 30;
+
+struct DevicePools {
+  std::mutex mu;
+  std::vector<std::pair<cudaMemPool_t, int>> by_dev;  // pool, contexts
+};
+DevicePools& device_pools() {
+  static DevicePools* p = new DevicePools();  // lives until the process ends: contexts may be destroyed at exit
+  return *p;
+}
+
+cudaMemPool_t pool_acquire(int dev) {
+  DevicePools& d = device_pools();
+  std::lock_guard<std::mutex> l(d.mu);
+  if ((int)d.by_dev.size() <= dev) d.by_dev.resize(dev + 1, {nullptr, 0});
+  auto& e = d.by_dev[dev];
+  if (!e.first) {
+    cudaMemPoolProps mp = {};
+    mp.allocType = cudaMemAllocationTypePinned;
+    mp.handleTypes = cudaMemHandleTypeNone;
+    mp.location.type = cudaMemLocationTypeDevice;
+    mp.location.id = dev;
+    CK(cudaMemPoolCreate(&e.first, &mp));
+    uint64_t keep = kPoolKeep;
+    CK(cudaMemPoolSetAttribute(e.first, cudaMemPoolAttrReleaseThreshold, &keep));
+  }
+  e.second++;
+  return e.first;
+}
+
+void pool_release(int dev) {
+  DevicePools& d = device_pools();
+  std::lock_guard<std::mutex> l(d.mu);
+  auto& e = d.by_dev[dev];
+  if (--e.second == 0) {
+    cudaMemPoolDestroy(e.first);
+    e.first = nullptr;
+  }
+}
 
 void free_list(Ctx& c, std::vector<void*>& v) {
   for (void* p : v) cudaFreeAsync(p, c.stream);
@@ -1147,6 +1465,17 @@ void scan_multi(Ctx& c, std::initializer_list<ScanArg<T>> args, cudaStream_t st 
   k_scan_lb<T><<<g, kScanThreads, 0, st>>>(jobs, c.scan_status.p, (int)nb, c.scan_ctr.p, c.scan_ctr.p + kScanMaxJobs,
                                            c.scan_err.p);
   note_launch();
+}
+
+// shared words of a tiled launch of at most `tiles` blocks
+TileCtl tile_ctl(Ctx& c, long long tiles, cudaStream_t st) {
+  if (tiles > (1LL << 30)) cap_throw("scan longer than its tile limit");
+  c.scan_status.reserve((size_t)std::max<long long>(tiles, 1));
+  if (c.scan_status.n > c.scan_status_n) {  // fresh memory: clear it once
+    CK(cudaMemsetAsync(c.scan_status.p, 0, sizeof(unsigned long long) * c.scan_status.n, st));
+    c.scan_status_n = c.scan_status.n;
+  }
+  return TileCtl{c.scan_status.p, c.scan_ctr.p, c.scan_ctr.p + kScanMaxJobs, c.scan_err.p};
 }
 
 template <class T>
@@ -2272,23 +2601,11 @@ __global__ void k_step_check(const PopDev* pops, int n_pop, const long long* pop
 }
 
 // Resolve and apply the events of a round (E at round_dev[1], at most W) and,
-// with Q > 0 (host loop only), its Q target operations.
-void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q) {
+// with Q > 0 (host loop only), its Q target operations.  chains: the round may
+// have chains (every round but the first).
+void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q, bool chains) {
   long long* Ed = c.round_dev.p + 1;
   ChainPool pool = chain_pool(c);
-  if (W > 0) {
-    const int tr = c.tune.threads[kTuneResolve];
-    {
-      TuneScope ts(c, kTuneResolve, st);
-      k_resolve_set<<<grid_for(W, tr), tr, 0, st>>>(c.d_pops, c.gpair_pop.p, Ed, c.ev_key.p, c.ev_c.p, c.gp_c.p,
-                                                      c.need_slot_set.p, c.need_id_set.p, c.win_set.p, c.dec_set.p,
-                                                      c.round_dev.p, c.ev_len.p, c.ev_head.p, c.ev_app.p, pool,
-                                                      c.chain_list.p, c.round_dev.p + 4);
-    }
-    note_launch();
-    scan_multi<int>(c, {{c.need_slot_set.p, W, Ed, c.rank_slot_set.p}, {c.need_id_set.p, W, Ed, c.rank_id_set.p}},
-                    st);
-  }
   // Q bounds the round's target operations; their count is n_dev[0] (the
   // redone ones, then those that walks appended)
   if (Q > 0) {
@@ -2304,33 +2621,67 @@ void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q) {
                                                       c.per_pop_i.p + 3 * c.n_pop);
     note_launch();
   }
-  k_alloc_bases<<<1, 256, 0, st>>>(c.d_pops, c.n_pop, Ed, c.gp_c.p, c.gpair_pop.p, W > 0 ? 1 : 0, c.rank_slot_set.p,
-                                   c.rank_id_set.p, c.per_pop_i.p, c.slot_base_set.p, c.id_base_set.p,
-                                   c.slot_base_pp.p, c.id_base_pp.p);
-  note_launch();
+  {
+    TuneScope ts(c, kTuneResolve, st);
+    ResolveArgs A;
+    A.pops = c.d_pops;
+    A.gpair_pop = c.gpair_pop.p;
+    A.n_events = W > 0 ? Ed : nullptr;
+    A.ev_key = c.ev_key.p;
+    A.ev = c.ev_c.p;
+    A.ev_gp = c.gp_c.p;
+    A.win = c.win_set.p;
+    A.dec = c.dec_set.p;
+    A.n_losers = c.round_dev.p;
+    A.ev_len = c.ev_len.p;
+    A.ev_head = c.ev_head.p;
+    A.ev_app = c.ev_app.p;
+    A.pool = pool;
+    A.chain_list = c.chain_list.p;
+    A.n_chain = c.round_dev.p + 4;
+    A.rank_slot = c.rank_slot_set.p;
+    A.rank_id = c.rank_id_set.p;
+    const int tr = c.tune.threads[kTuneResolve];
+    const long long tiles = std::max<long long>(1, (W + tr - 1) / tr);
+    A.ctl = tile_ctl(c, tiles, st);
+    A.n_pop = c.n_pop;
+    A.per_pop = c.per_pop_i.p;
+    A.set_slot_base = c.slot_base_set.p;
+    A.pp_slot_base = c.slot_base_pp.p;
+    A.set_id_base = c.id_base_set.p;
+    A.pp_id_base = c.id_base_pp.p;
+    k_resolve<<<(unsigned)tiles, tr, 0, st>>>(A);
+    note_launch();
+  }
   if (W > 0) {
-    // part 1, one thread per event: species and components
     const int ta = c.tune.threads[kTuneApply];
-    {
-      TuneScope ts(c, kTuneApply, st);
-      k_apply_move<<<grid_for(W, ta), ta, 0, st>>>(c.d_pops, c.gpair_pop.p, Ed, c.ev_key.p, c.ev_c.p, c.gp_c.p,
-                                                          c.win_set.p, c.dec_set.p, c.rank_slot_set.p,
-                                                          c.slot_base_set.p, c.ice_set.p);
-      note_launch();
-      // part 2, one thread per event: removals, scalar fields, caches
-      k_apply_set<<<grid_for(W, ta), ta, 0, st>>>(c.d_pops, c.gpair_pop.p, Ed, c.ev_key.p, c.ev_c.p, c.gp_c.p,
-                                                    c.win_set.p, c.dec_set.p, c.rank_slot_set.p, c.rank_id_set.p,
-                                                    c.slot_base_set.p, c.id_base_set.p, c.ice_set.p, c.ev_done.p,
-                                                    c.ev_dest.p, c.ev_key.p, c.ev_c.p, c.gp_c.p, c.ev_pos.p, c.dec_set.p,
-                                                    c.ev_term.p, c.pop_pair_base.p);
-      note_launch();
+    // chains, one warp each, beside the other events (their claims keep them
+    // on different slots): a branch of its own in a captured step
+    cudaStream_t sc = st;
+    if (chains && c.fork) {
+      CK(cudaEventRecord(c.ev_fork, st));
+      CK(cudaStreamWaitEvent(c.side_stream, c.ev_fork, 0));
+      sc = c.side_stream;
     }
-    // chains, one warp each
-    k_apply_chain<<<grid_for(W, 32), 32, 0, st>>>(c.d_pops, c.gpair_pop.p, c.pop_pair_base.p, c.chain_list.p,
+    if (chains) {
+      k_apply_chain<<<grid_for(W, 32), 32, 0, sc>>>(c.d_pops, c.gpair_pop.p, c.pop_pair_base.p, c.chain_list.p,
                                                     c.round_dev.p + 4, c.ev_key.p, c.ev_len.p, c.ev_app.p,
                                                     c.ev_head.p, c.ev_done.p, pool, c.gp_c.p, c.ev_pos.p,
                                                     c.ev_dest.p, c.ev_key.p, c.ev_c.p, c.dec_set.p, c.ev_term.p);
-    note_launch();
+      note_launch();
+    }
+    {
+      TuneScope ts(c, kTuneApply, st);
+      k_apply<<<grid_for(W, ta), ta, 0, st>>>(c.d_pops, c.gpair_pop.p, Ed, c.win_set.p, c.rank_slot_set.p,
+                                              c.rank_id_set.p, c.slot_base_set.p, c.id_base_set.p, c.ev_done.p,
+                                              c.ev_dest.p, c.ev_key.p, c.ev_c.p, c.gp_c.p, c.ev_pos.p, c.dec_set.p,
+                                              c.ev_term.p, c.pop_pair_base.p);
+      note_launch();
+    }
+    if (chains && c.fork) {
+      CK(cudaEventRecord(c.ev_join, c.side_stream));
+      CK(cudaStreamWaitEvent(st, c.ev_join, 0));
+    }
   }
   if (Q > 0) {
     const size_t nw = (size_t)Q * kMaxCopies;
@@ -2349,6 +2700,32 @@ void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q) {
     note_launch();
     scan_multi<int>(c, {ScanArg<int>{c.lost_pp.p, Q, c.n_dev.p, c.lost_off.p, c.round_dev.p + 8}}, st);
   }
+}
+
+long long compact_tiles(long long n) { return std::max<long long>(1, (n + kCompactTile - 1) / kCompactTile); }
+
+CompactArgs compact_args(Ctx& c, const uint8_t* flag, const long long* n, long long bound, cudaStream_t st) {
+  CompactArgs A;
+  A.flag = flag;
+  A.n = n;
+  A.n_events = c.round_dev.p + 1;
+  A.ctl = tile_ctl(c, compact_tiles(bound), st);
+  A.ev_key = c.ev_key.p;
+  A.ev_c = c.ev_c.p;
+  A.gp_c = c.gp_c.p;
+  A.ev_pos = c.ev_pos.p;
+  A.ev_len = c.ev_len.p;
+  A.ev_term = c.ev_term.p;
+  A.dec = c.dec_set.p;
+  return A;
+}
+
+// round 0's events from the tests' flags (their count *n on the device, at most W)
+void launch_compact_samples(Ctx& c, const long long* n, long long W, cudaStream_t st) {
+  k_compact_samples<<<(unsigned)compact_tiles(W), kCompactThreads, 0, st>>>(
+      compact_args(c, c.flag.p, n, W, st), c.d_pops, c.gpair_pop.p, c.gpair_local.p, c.ev.p, c.ev_gp.p,
+      c.work_off.p);
+  note_launch();
 }
 
 struct RoundBounds {
@@ -2384,8 +2761,6 @@ void enqueue_round_body(Ctx& c, cudaStream_t st, const RoundBounds& b, long long
     launch_pp(c, b.kt, Q, false);
   }
   const long long* Id = c.round_dev.p + 2;
-  long long* Ed = c.round_dev.p + 1;
-  scan_multi<uint8_t>(c, {ScanArg<uint8_t>{c.it_flag.p, W, Id, c.it_off.p, Ed}}, st);
   // a batched step with target operations: the walkers they made join the
   // items after the events, from every population, so the events are
   // grouped by population for the allocation (group_by_pop)
@@ -2399,13 +2774,11 @@ void enqueue_round_body(Ctx& c, cudaStream_t st, const RoundBounds& b, long long
     group_by_pop(c, Id, W, c.item_pop.p, c.grp_dest.p, st);
     grouped = c.grp_dest.p;
   }
-  k_compact_items<<<grid_for(W, 256), 256, 0, st>>>(c.it_flag.p, c.it_off.p, Id, c.it_key.p, c.it_c.p, c.it_gp.p,
-                                                    c.it_pos.p, c.it_len.p, c.it_head.p, c.it_done.p, c.it_dec.p,
-                                                    c.it_term.p, c.ev_key.p, c.ev_c.p, c.gp_c.p, c.ev_pos.p,
-                                                    c.ev_len.p, c.ev_head.p, c.ev_done.p, c.dec_set.p, c.ev_term.p,
-                                                    grouped);
+  k_compact_items<<<(unsigned)compact_tiles(W), kCompactThreads, 0, st>>>(
+      compact_args(c, c.it_flag.p, Id, W, st), c.it_key.p, c.it_c.p, c.it_gp.p, c.it_pos.p, c.it_len.p, c.it_head.p,
+      c.it_done.p, c.it_dec.p, c.it_term.p, c.ev_head.p, c.ev_done.p, grouped);
   note_launch();
-  resolve_apply(c, st, W, Q);
+  resolve_apply(c, st, W, Q, true);
 }
 
 // everything the captured launches depend on: sizes and device addresses
@@ -2419,13 +2792,13 @@ std::vector<long long> round_graph_key(const Ctx& c, const RoundBounds& b) {
           (long long)c.ev_pos.p, (long long)c.ev_dest.p, (long long)c.ev_len.p, (long long)c.ev_head.p,
           (long long)c.ev_app.p, (long long)c.ev_done.p, (long long)c.chain_list.p, (long long)c.it_flag.p, (long long)c.it_key.p,
           (long long)c.it_c.p, (long long)c.it_gp.p, (long long)c.it_pos.p, (long long)c.it_len.p,
-          (long long)c.it_head.p, (long long)c.it_start.p, (long long)c.it_done.p, (long long)c.it_dec.p, (long long)c.it_gused.p, (long long)c.it_off.p,
+          (long long)c.it_head.p, (long long)c.it_start.p, (long long)c.it_done.p, (long long)c.it_dec.p, (long long)c.it_gused.p,
           (long long)c.it_term.p, (long long)c.ev_term.p, (long long)c.ppw_slot.p, (long long)c.ppw_gp.p,
           (long long)c.ch_y.p,
-          (long long)c.ch_q.p, (long long)c.ch_pos.p, (long long)c.need_slot_set.p, (long long)c.need_id_set.p,
+          (long long)c.ch_q.p, (long long)c.ch_pos.p,
           (long long)c.win_set.p, (long long)c.dec_set.p, (long long)c.rank_slot_set.p, (long long)c.rank_id_set.p,
           (long long)c.slot_base_set.p, (long long)c.id_base_set.p, (long long)c.slot_base_pp.p,
-          (long long)c.id_base_pp.p, (long long)c.ice_set.p, (long long)c.scan_status.p, (long long)c.scan_ctr.p,
+          (long long)c.id_base_pp.p, (long long)c.scan_status.p, (long long)c.scan_ctr.p,
           (long long)c.scan_err.p, (long long)c.graph_stats.p};
 }
 
@@ -2457,7 +2830,6 @@ void reserve_events(Ctx& c, long long W) {
   c.ev_len.reserve(w + 1); c.ev_head.reserve(w + 1); c.ev_app.reserve(w + 1); c.ev_done.reserve(w + 1);
   c.ev_term.reserve(w + 1);
   c.chain_list.reserve(w + 1);
-  c.need_slot_set.reserve(w + 1); c.need_id_set.reserve(w + 1); c.ice_set.reserve(w + 1);
   c.rank_slot_set.reserve(w + 2); c.rank_id_set.reserve(w + 2);
   size_t chunks = w + 4096;
   c.ch_y.reserve(chunks * kChainChunk);
@@ -2472,8 +2844,7 @@ bool events_fit(const Ctx& c, long long W) {
          c.ev_dest.n >= w + 1 && c.win_set.n >= w + 1 && c.dec_set.n >= w + 1 && c.ev_len.n >= w + 1 &&
          c.ev_head.n >= w + 1 && c.ev_app.n >= w + 1 && c.ev_done.n >= w + 1 && c.chain_list.n >= w + 1 &&
          c.ev_term.n >= w + 1 &&
-         c.need_slot_set.n >= w + 1 &&
-         c.need_id_set.n >= w + 1 && c.ice_set.n >= w + 1 && c.rank_slot_set.n >= w + 2 &&
+         c.rank_slot_set.n >= w + 2 &&
          c.rank_id_set.n >= w + 2;
 }
 
@@ -2484,7 +2855,6 @@ void reserve_round(Ctx& c, long long W) {
   c.it_flag.reserve(w + 1); c.it_key.reserve(w + 1); c.it_c.reserve(w + 1); c.it_gp.reserve(w + 1);
   c.it_pos.reserve(w + 1); c.it_len.reserve(w + 1); c.it_head.reserve(w + 1); c.it_done.reserve(w + 1); c.it_start.reserve(w + 1);
   c.it_dec.reserve(w + 1); c.it_gused.reserve(w + 1); c.it_term.reserve(w + 1);
-  c.it_off.reserve(w + 2);
 }
 
 struct GraphRun {
@@ -2523,8 +2893,8 @@ GraphRun run_round_graph(Ctx& c, int kt, bool flat, int n_gpairs, long long e0) 
   reserve_round(c, b.W);
   c.graph_stats.reserve(8);
   {
-    long long nb = (b.W + kScanTile - 1) / kScanTile;
-    c.scan_status.reserve((size_t)kScanMaxJobs * nb);
+    const long long nb = (b.W + kScanTile - 1) / kScanTile;
+    c.scan_status.reserve((size_t)std::max(kScanMaxJobs * nb, b.W / kResolveMin + 2));
     if (c.scan_status.n > c.scan_status_n) {
       CK(cudaMemsetAsync(c.scan_status.p, 0, sizeof(unsigned long long) * c.scan_status.n, c.stream));
       c.scan_status_n = c.scan_status.n;
@@ -2658,7 +3028,7 @@ std::vector<long long> step_graph_key(const Ctx& c, const RoundBounds& b, long l
   for (long long v : {w_cap, (long long)max_pairs, (long long)c.prof, (long long)c.tune.threads[kTuneTest],
                       (long long)c.nwork_set.p, (long long)c.nwork_pp.p, (long long)c.work_off.p,
                       (long long)c.pp_off.p, (long long)c.flag.p, (long long)c.ev.p, (long long)c.ev_gp.p,
-                      (long long)c.flag_off.p, (long long)c.d_stat})
+                      (long long)c.d_stat})
     k.push_back(v);
   return k;
 }
@@ -2698,16 +3068,8 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
     launch_test_kt(c, b.kt, b.flat, n_gp, w_cap, st);
     mark(3);
     const long long* Wd = c.work_off.p + n_gp;
-    scan_multi<uint8_t>(c, {ScanArg<uint8_t>{c.flag.p, w_cap, Wd, c.flag_off.p, c.round_dev.p + 1}}, st);
-    k_compact_flags<<<grid_for(w_cap, 256), 256, 0, st>>>(c.flag.p, c.flag_off.p, Wd, c.ev.p, c.ev_gp.p,
-                                                         c.gpair_local.p, c.work_off.p, c.ev_key.p, c.ev_c.p,
-                                                         c.gp_c.p, c.ev_pos.p, c.ev_len.p, c.ev_term.p);
-    note_launch();
-    const int td = c.tune.threads[kTuneResolve];
-    k_decide<<<grid_for(w_cap, td), td, 0, st>>>(c.d_pops, c.gpair_pop.p, c.round_dev.p + 1, c.ev_key.p, c.ev_c.p,
-                                                 c.gp_c.p, c.dec_set.p);
-    note_launch();
-    resolve_apply(c, st, w_cap, 0);
+    launch_compact_samples(c, Wd, w_cap, st);
+    resolve_apply(c, st, w_cap, 0, false);
     k_round_end<<<1, 128, 0, st>>>(c.round_dev.p, c.d_stat, c.d_round, c.max_rounds, c.d_pops, c.d_ctrs, c.n_pop,
                                    sort_slots, b.W, c.scan_err.p, cond);
     note_launch();
@@ -2737,12 +3099,15 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
                                      cudaStreamCaptureModeRelaxed));
     k_round_begin<<<1, 128, 0, st>>>(c.d_round, c.round_dev.p, c.per_pop_i.p, 4 * c.n_pop);
     note_launch();
+    c.fork = true;
     enqueue_round_body(c, st, b, 0);
+    c.fork = false;
     k_round_end<<<1, 128, 0, st>>>(c.round_dev.p, c.d_stat, c.d_round, c.max_rounds, c.d_pops, c.d_ctrs, c.n_pop,
                                    sort_slots, b.W, c.scan_err.p, cond);
     note_launch();
     c.sg_nodes = g_launches - n1;
   } catch (...) {
+    c.fork = false;
     cudaStreamEndCapture(st, &done);
     cudaGetLastError();
     g_launches = n0;
@@ -2808,12 +3173,12 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   c.work_off.reserve(ng);
   c.pp_off.reserve(ng);
   const size_t ws = (size_t)c.sg_w;
-  c.flag.reserve(ws + 1); c.ev.reserve(ws + 1); c.flag_off.reserve(ws + 2); c.ev_gp.reserve(ws + 1);
+  c.flag.reserve(ws + 1); c.ev.reserve(ws + 1); c.ev_gp.reserve(ws + 1);
   reserve_events(c, c.sg_w);
   reserve_round(c, b.W);
   {
     const long long nb = std::max<long long>((c.sg_w + kScanTile - 1) / kScanTile, (b.n_gpairs + kScanTile - 1) / kScanTile);
-    c.scan_status.reserve((size_t)kScanMaxJobs * nb);
+    c.scan_status.reserve((size_t)std::max(kScanMaxJobs * nb, c.sg_w / kResolveMin + 2));
     if (c.scan_status.n > c.scan_status_n) {
       CK(cudaMemsetAsync(c.scan_status.p, 0, sizeof(unsigned long long) * c.scan_status.n, c.stream));
       c.scan_status_n = c.scan_status.n;
@@ -3032,7 +3397,7 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
   }
   {
     size_t w = (size_t)W;
-    c.flag.reserve(w + 1); c.ev.reserve(w + 1); c.flag_off.reserve(w + 2); c.ev_gp.reserve(w + 1);
+    c.flag.reserve(w + 1); c.ev.reserve(w + 1); c.ev_gp.reserve(w + 1);
     // the walkers that target operations make (the target and its copies)
     // join a later round's items and events
     reserve_events(c, W + kMaxCopies * Q);
@@ -3064,18 +3429,9 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
   // and the event count E goes to round_dev[1], both on the device
   if (W > 0) {
     const long long* Wd = c.work_off.p + n_gpairs;
-    scan_multi<uint8_t>(c, {ScanArg<uint8_t>{c.flag.p, W, Wd, c.flag_off.p, c.round_dev.p + 1}});
-    k_compact_flags<<<grid_for(W, 256), 256, 0, c.stream>>>(c.flag.p, c.flag_off.p, Wd, c.ev.p, c.ev_gp.p,
-                                                           c.gpair_local.p, c.work_off.p, c.ev_key.p, c.ev_c.p,
-                                                           c.gp_c.p, c.ev_pos.p, c.ev_len.p, c.ev_term.p);
-    note_launch();
-    const int td = c.tune.threads[kTuneResolve];
-    TuneScope ts(c, kTuneResolve, c.stream);
-    k_decide<<<grid_for(W, td), td, 0, c.stream>>>(c.d_pops, c.gpair_pop.p, c.round_dev.p + 1, c.ev_key.p, c.ev_c.p,
-                                                   c.gp_c.p, c.dec_set.p);
-    note_launch();
+    launch_compact_samples(c, Wd, W, c.stream);
   }
-  resolve_apply(c, c.stream, W, Q);
+  resolve_apply(c, c.stream, W, Q, false);
 
   c.last_w = W;
   step_rounds(c, kt, flat, n_gpairs, Q, 0, 0, false);
@@ -3275,15 +3631,14 @@ static int do_init(int n_pop, int n_spec, const double* density, int i_water, in
     }
   CK(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&c.cap_stream, cudaStreamNonBlocking));
+  CK(cudaStreamCreateWithFlags(&c.side_stream, cudaStreamNonBlocking));
+  CK(cudaEventCreateWithFlags(&c.ev_fork, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&c.ev_join, cudaEventDisableTiming));
   {
-    cudaMemPoolProps mp = {};
-    mp.allocType = cudaMemAllocationTypePinned;
-    mp.handleTypes = cudaMemHandleTypeNone;
-    mp.location.type = cudaMemLocationTypeDevice;
-    CK(cudaGetDevice(&mp.location.id));
-    CK(cudaMemPoolCreate(&c.mem, &mp));
-    uint64_t keep = kPoolKeep;
-    CK(cudaMemPoolSetAttribute(c.mem, cudaMemPoolAttrReleaseThreshold, &keep));
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    c.mem = pool_acquire(dev);
+    c.mem_ref.dev = dev;
   }
   {
     int dev = 0, n_sm = 0, coop = 0;
@@ -3340,15 +3695,15 @@ int pmc_coag_gpu_destroy(pmc_coag_gpu_ctx* x) {
   cudaFree(c.d_pops);
   cudaFree(c.d_stat);
   cudaFree(c.d_round);
-  DevBuf<int>* bi[] = {&c.gpair_pop, &c.gpair_local, &c.need_slot_set, &c.need_id_set, &c.need_slot_pp,
+  DevBuf<int>* bi[] = {&c.gpair_pop, &c.gpair_local, &c.need_slot_pp,
                        &c.need_id_pp, &c.lost_pp, &c.op_pop, &c.op_pair, &c.op_slot, &c.op_k, &c.r_pop,
                        &c.r_pair, &c.r_slot, &c.r_k, &c.per_pop_i, &c.slot_base_set, &c.slot_base_pp,
                        &c.ev_dest, &c.ev_len, &c.ev_head, &c.ev_app, &c.it_gp, &c.it_len, &c.it_head, &c.it_start,
                        &c.ch_y, &c.ch_q};
   for (auto* b : bi) b->release();
-  DevBuf<long long>* bl[] = {&c.pop_pair_base, &c.nwork_set, &c.nwork_pp, &c.work_off, &c.pp_off, &c.flag_off,
+  DevBuf<long long>* bl[] = {&c.pop_pair_base, &c.nwork_set, &c.nwork_pp, &c.work_off, &c.pp_off,
                              &c.rank_slot_set, &c.rank_id_set, &c.rank_slot_pp, &c.rank_id_pp, &c.lost_off,
-                             &c.id_base_set, &c.id_base_pp, &c.n_dev, &c.it_off};
+                             &c.id_base_set, &c.id_base_pp, &c.n_dev};
   for (auto* b : bl) b->release();
   DevBuf<unsigned long long>* bk[] = {&c.ev_key, &c.it_key, &c.op_key, &c.r_key};
   for (auto* b : bk) b->release();
@@ -3371,7 +3726,6 @@ int pmc_coag_gpu_destroy(pmc_coag_gpu_ctx* x) {
   c.ev_gp.release();
   c.gp_c.release();
   c.ev_c.release();
-  c.ice_set.release();
   c.scan_status.release();
   c.scan_ctr.release();
   c.scan_err.release();
@@ -3415,8 +3769,10 @@ int pmc_coag_gpu_destroy(pmc_coag_gpu_ctx* x) {
   }
   for (auto e : c.tuner.spare) cudaEventDestroy(e);
   cudaStreamSynchronize(c.stream);  // the arrays are back in the pool
-  if (c.mem) cudaMemPoolDestroy(c.mem);
   cudaStreamDestroy(c.cap_stream);
+  cudaStreamDestroy(c.side_stream);
+  cudaEventDestroy(c.ev_fork);
+  cudaEventDestroy(c.ev_join);
   cudaStreamDestroy(c.stream);
   delete x;
   return PMC_OK;
