@@ -295,15 +295,18 @@ PMC_HD T brown_pair(T rad_i, T diffus_i, T speedsq_i, T deltasq_i, T rad_j, T di
   return T(4.0 * kPi) * rad_sum * diffus_sum / (tmp1 + tmp2);
 }
 
-// Full FP64 form in the reference's order, for k-bound tables and checks.
-PMC_HD double brown_kernel(const BrownEnv& e, double vi, double di, double vj, double dj, bool* ok) {
-  BrownPart a = brown_part(e, vol2rad(e.frac, vi), vi, di, ok);
-  BrownPart b = brown_part(e, vol2rad(e.frac, vj), vj, dj, ok);
+// the FP64 pair half for two particles' parts
+PMC_HD double brown_of_parts(const BrownPart& a, const BrownPart& b) {
   double rad_sum = a.rad + b.rad;
   double diffus_sum = a.diffus + b.diffus;
   double tmp1 = rad_sum / (rad_sum + sqrt(a.deltasq + b.deltasq));
   double tmp2 = 4.0 * diffus_sum / (rad_sum * sqrt(a.speedsq + b.speedsq));
   return 4.0 * kPi * rad_sum * diffus_sum / (tmp1 + tmp2);
+}
+
+// Full FP64 form in the reference's order, for k-bound tables and checks.
+PMC_HD double brown_kernel(const BrownEnv& e, double vi, double di, double vj, double dj, bool* ok) {
+  return brown_of_parts(brown_part(e, vol2rad(e.frac, vi), vi, di, ok), brown_part(e, vol2rad(e.frac, vj), vj, dj, ok));
 }
 
 // fall_g, coag_kernel_sedi.F90:110-172 (terminal velocity, m/s; r in m)
