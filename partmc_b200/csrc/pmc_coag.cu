@@ -1952,7 +1952,7 @@ void prepare_chunks(Ctx& c, long long extra = 0) {
 // blocks, for chunk and cell counts up to max_chunks and max_cells
 // co-resident blocks of the sort for max_cells cells (its shared memory)
 size_t size_sort(Ctx& c, int max_cells) {
-  size_t smem = sizeof(int) * (kSortWarps + 1) * (size_t)max_cells;
+  size_t smem = sizeof(int) * ((kSortWarps + 1) * (size_t)max_cells + (c.n_pop <= kSortMapPops ? c.n_pop + 1 : 0));
   if (smem != c.sort_smem) {
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sort_all, kSortThreads, smem));

@@ -231,17 +231,28 @@ __global__ void k_refresh_all(const PopDev* pops, const uint8_t* on) {
 // one cooperative launch.  The grid is persistent (co-resident blocks looping
 // over work items); two grid-wide barriers separate three phases:
 //   1. per chunk of kChunk slots: the cell keys go to registers (thread
-//      (w, lane) holds slots w * kWarpSlots + j * 32 + lane, j < kKeysPerThread)
-//      and a warp-aggregated histogram to chunk_hist, cell-major
-//      (chunk_hist[cell * n_chunks + chunk]); the occupied bin range is reset
+//      (w, lane) holds slots w * kWarpSlots + j * 32 + lane, j < kKeysPerThread),
+//      each with its rank among the warp's earlier slots of the same cell
+//      (__match_any_sync over a tile of 32), and the chunk's counts to
+//      chunk_hist, cell-major (chunk_hist[cell * n_chunks + chunk]); the
+//      occupied bin range is reset
 //   2. per cell (one warp): exclusive scan of its chunk column in place and
 //      the cell total; the occupied bin range
 //   3. per chunk: the cell starts (a block scan of the totals; the chunk-0
-//      block of each population stores them), then the scatter, ranking the
-//      slots of one cell inside a 32-slot tile with __match_any_sync.  A block
-//      reuses the keys it loaded in phase 1 for the same chunk.
+//      block of each population stores them), then the scatter by cell start,
+//      chunk, warp and rank.  A block that had one chunk in phase 1 still has
+//      its keys, ranks and warp counts; otherwise it takes them again.
+// The work items are the populations' chunks that hold slots (chunk_base, the
+// running count of them, in shared memory): with 256 populations of 3e3 to
+// 1e5 particles, items up to the largest population's chunk count in every
+// population were six times as many, and the sort took 120 us, now 80.
+// At 1e6 particles it takes 21 to 23 (26 with the ranks taken again by two more
+// rounds of matches in phase 3), at 1e4 10.5 (13), bound by the two barriers and the phases'
+// dependent loads; the keys and lists (8 MB) stay in L2.
 constexpr int kKeysPerThread = kWarpSlots / 32;
+constexpr int kSortMapPops = 2048;  // populations whose chunk counts are kept in shared memory
 
+// keys of a thread's slots, -1 for a slot without a cell
 __device__ __forceinline__ void sort_load_keys(const PopDev& P, int chunk, int n, int nc, int w, int lane,
                                                int* keys) {
 #pragma unroll
@@ -252,38 +263,92 @@ __device__ __forceinline__ void sort_load_keys(const PopDev& P, int chunk, int n
   }
 }
 
-__global__ void __launch_bounds__(kSortThreads) k_sort_all(const PopDev* pops, int n_pop, int max_chunks,
+// adds to each key (below 2^16: at most kMaxBin x kMaxClass cells) its rank
+// among the warp's earlier slots of the same cell (below kWarpSlots) in bits
+// 16 and up, and leaves the warp's counts in cnt[0..nc) (zero before)
+__device__ __forceinline__ void sort_rank_keys(int* keys, int lane, int* cnt) {
+  const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+  for (int j = 0; j < kKeysPerThread; j++) {
+    const int key = keys[j];
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    const int before = key >= 0 ? cnt[key] : 0;
+    if (key >= 0) keys[j] = key | ((before + __popc(peers & lt)) << 16);
+    __syncwarp();
+    if (key >= 0 && lane == __ffs(peers) - 1) cnt[key] = before + __popc(peers);
+    __syncwarp();
+  }
+}
+
+__global__ void __launch_bounds__(kSortThreads, 6) k_sort_all(const PopDev* pops, int n_pop, int max_chunks,
                                                            int max_cells) {
   namespace cg = cooperative_groups;
   cg::grid_group grid = cg::this_grid();
-  extern __shared__ int sm[];  // [kSortWarps][max_cells] counters, then [max_cells] cell starts
+  extern __shared__ int sm[];  // [kSortWarps][max_cells] counters, [max_cells] cell starts, [n_pop + 1] chunk_base
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const long long n_chunk_items = (long long)n_pop * max_chunks;
+  int* starts = sm + kSortWarps * max_cells;
+  int* chunk_base = starts + max_cells;
+  const bool mapped = n_pop > 1 && n_pop <= kSortMapPops;
+  long long n_items = n_pop == 1 ? n_chunks_of(pops[0]) : (long long)n_pop * max_chunks;
+  if (mapped) {
+    int carry = 0;
+    for (int base = 0; base < n_pop; base += kSortThreads) {
+      const int k = base + threadIdx.x;
+      const int v = k < n_pop ? n_chunks_of(pops[k]) : 0;
+      int tot;
+      const int pre = block_excl_scan(v, &tot);
+      if (k < n_pop) chunk_base[k] = carry + pre;
+      carry += tot;
+    }
+    if (threadIdx.x == 0) chunk_base[n_pop] = carry;
+    __syncthreads();
+    n_items = carry;
+  }
+  // population and chunk of an item
+  auto locate = [&](long long item, int* chunk) -> const PopDev& {
+    if (n_pop == 1) {
+      *chunk = (int)item;
+      return pops[0];
+    }
+    if (!mapped) {
+      *chunk = (int)(item % max_chunks);
+      return pops[item / max_chunks];
+    }
+    int lo = 0, hi = n_pop;  // largest k with chunk_base[k] <= item
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (chunk_base[mid] <= (int)item) lo = mid;
+      else hi = mid;
+    }
+    *chunk = (int)item - chunk_base[lo];
+    return pops[lo];
+  };
   int keys[kKeysPerThread];
-  long long kept = -1;  // chunk item whose keys are in registers
+  long long kept = -1;  // chunk item whose keys, ranks and warp counts are at hand
   // phase 1
   if (blockIdx.x == 0)
     for (int k = threadIdx.x; k < n_pop; k += blockDim.x) {
       pops[k].ctr->bmin = 1 << 30;
       pops[k].ctr->bmax = -1;
     }
-  for (long long item = blockIdx.x; item < n_chunk_items; item += gridDim.x) {
-    const PopDev& P = pops[item / max_chunks];
-    int chunk = (int)(item % max_chunks);
-    int n_chunks = n_chunks_of(P);
+  for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
+    int chunk;
+    const PopDev& P = locate(item, &chunk);
+    const int n_chunks = n_chunks_of(P);
     if (chunk >= n_chunks || !chunk_hist_fits(P, n_chunks)) continue;  // the same for the whole block
-    int nc = P.n_cells;
+    const int nc = P.n_cells;
     sort_load_keys(P, chunk, P.ctr->n_slots, nc, w, lane, keys);
     kept = item;
-    for (int c = threadIdx.x; c < nc; c += blockDim.x) sm[c] = 0;
+    for (int c = threadIdx.x; c < kSortWarps * nc; c += blockDim.x) sm[c] = 0;
     __syncthreads();
+    sort_rank_keys(keys, lane, sm + w * nc);
+    __syncthreads();
+    for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+      int x = 0;
 #pragma unroll
-    for (int j = 0; j < kKeysPerThread; j++) {
-      unsigned peers = __match_any_sync(0xffffffffu, keys[j]);
-      if (keys[j] >= 0 && lane == __ffs(peers) - 1) atomicAdd(&sm[keys[j]], __popc(peers));
+      for (int q = 0; q < kSortWarps; q++) x += sm[q * nc + c];
+      P.chunk_hist[(size_t)c * n_chunks + chunk] = x;
     }
-    __syncthreads();
-    for (int c = threadIdx.x; c < nc; c += blockDim.x) P.chunk_hist[(size_t)c * n_chunks + chunk] = sm[c];
     __syncthreads();
   }
   grid.sync();
@@ -307,6 +372,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_all(const PopDev* pops, i
         }
 #pragma unroll
         for (int u = 0; u < 4; u++) {
+          if (base + u * 32 >= n_chunks) break;
           int x = h[u];
           for (int o = 1; o < 32; o <<= 1) {
             int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -329,21 +395,25 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_all(const PopDev* pops, i
   }
   grid.sync();
   // phase 3
-  int* starts = sm + kSortWarps * max_cells;
-  for (long long item = blockIdx.x; item < n_chunk_items; item += gridDim.x) {
-    const PopDev& P = pops[item / max_chunks];
-    int chunk = (int)(item % max_chunks);
-    int n_chunks = n_chunks_of(P);
-    int nc = P.n_cells;
-    if (chunk == 0 && n_chunks == 0) {  // an empty population still gets its (zero) cell starts
-      for (int c = threadIdx.x; c <= nc; c += blockDim.x) P.cell_start[c] = 0;
-      continue;
-    }
+  // an empty population still gets its (zero) cell starts
+  for (int k = blockIdx.x; k < n_pop; k += gridDim.x) {
+    const PopDev& P = pops[k];
+    if (n_chunks_of(P) == 0)
+      for (int c = threadIdx.x; c <= P.n_cells; c += blockDim.x) P.cell_start[c] = 0;
+  }
+  for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
+    int chunk;
+    const PopDev& P = locate(item, &chunk);
+    const int n_chunks = n_chunks_of(P);
+    const int nc = P.n_cells;
     if (chunk >= n_chunks || !chunk_hist_fits(P, n_chunks)) continue;
-    int n = P.ctr->n_slots;
+    const int n = P.ctr->n_slots;
     if (item != kept) {
       sort_load_keys(P, chunk, n, nc, w, lane, keys);
-      kept = item;
+      for (int c = threadIdx.x; c < kSortWarps * nc; c += blockDim.x) sm[c] = 0;
+      __syncthreads();
+      sort_rank_keys(keys, lane, sm + w * nc);
+      kept = -1;  // the counts become positions below
     }
     // cell starts
     int carry = 0;
@@ -359,16 +429,10 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_all(const PopDev* pops, i
       for (int c = threadIdx.x; c < nc; c += blockDim.x) P.cell_start[c] = starts[c];
       if (threadIdx.x == 0) P.cell_start[nc] = carry;
     }
-    for (int k = threadIdx.x; k < kSortWarps * nc; k += blockDim.x) sm[k] = 0;
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kKeysPerThread; j++) {
-      unsigned peers = __match_any_sync(0xffffffffu, keys[j]);
-      if (keys[j] >= 0 && lane == __ffs(peers) - 1) sm[w * nc + keys[j]] += __popc(peers);
-    }
     __syncthreads();
     for (int c = threadIdx.x; c < nc; c += blockDim.x) {
       int run = starts[c] + P.chunk_hist[(size_t)c * n_chunks + chunk];
+#pragma unroll
       for (int q = 0; q < kSortWarps; q++) {
         int x = sm[q * nc + c];
         sm[q * nc + c] = run;
@@ -376,22 +440,12 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_all(const PopDev* pops, i
       }
     }
     __syncthreads();
-    unsigned lt = (1u << lane) - 1u;
 #pragma unroll
     for (int j = 0; j < kKeysPerThread; j++) {
-      int key = keys[j];
-      int i = chunk * kChunk + w * kWarpSlots + j * 32 + lane;
-      unsigned peers = __match_any_sync(0xffffffffu, key);
-      int leader = __ffs(peers) - 1;
-      int pos = 0;
-      if (key >= 0) pos = sm[w * nc + key] + __popc(peers & lt);
-      __syncwarp();
-      if (key >= 0 && lane == leader) sm[w * nc + key] += __popc(peers);
-      __syncwarp();
-      if (key >= 0) {
-        if (pos >= 0 && pos < P.cap) P.list[pos] = i;
-        else bad_index(P.ctr, kBadScatterPos, pos);
-      }
+      if (keys[j] < 0) continue;
+      const int pos = sm[w * nc + (keys[j] & 0xffff)] + (keys[j] >> 16);
+      if (pos >= 0 && pos < P.cap) P.list[pos] = chunk * kChunk + w * kWarpSlots + j * 32 + lane;
+      else bad_index(P.ctr, kBadScatterPos, pos);
     }
     __syncthreads();
   }
