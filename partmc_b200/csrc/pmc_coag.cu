@@ -1281,12 +1281,15 @@ struct Ctx {
   cudaGraph_t sg_graph = nullptr;
   cudaGraphExec_t sg_exec = nullptr;
   std::vector<long long> sg_key, sg_seen;
-  long long sg_w = 0, sg_e = 0;      // samples and events it holds room for
+  long long sg_w = 0, sg_e = 0;      // samples and items it holds room for
+  long long sg_q = 0, sg_qb = 0;     // target operations of round 0 and of a later round
   long long sg_nodes0 = 0, sg_nodes = 0;  // launches of its round 0 and of one later round
   cudaEvent_t sg_ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // when profiling: sort, tests, later rounds
   bool sg_prof = false;              // the captured graph records them
   long long* d_stat = nullptr;       // kStatWords words before the counter blocks, read back with them
-  long long last_w = -1, last_e0 = 0;  // samples and round-0 events of the last step
+  // the last step's samples, largest items and target operations of a later
+  // round, target operations of round 0 and largest removal bound
+  long long last_w = -1, last_e0 = 0, last_qb = 0, last_q = 0, last_rm = 0;
   bool ctrs_fresh = false;           // h_ctrs and n_slots_host are the device's counters
   Tune tune;
   Tuner tuner;
@@ -1294,13 +1297,12 @@ struct Ctx {
   DevBuf<int> pp_rm_n, pp_rm_pool;
   DevBuf<uint8_t> pop_on;  // the populations a refresh covers
   // a batched round's lists grouped by population (group_by_pop)
-  DevBuf<int> grp_hist, item_pop, g_pop, g_pair, g_slot, g_k;
+  DevBuf<int> grp_hist, item_pop;
   DevBuf<long long> grp_off, grp_dest;
   // walkers of the round's operations, one place per operation and copy
   DevBuf<int> wk_slot, wk_gp;
   DevBuf<uint8_t> wk_flag;
   DevBuf<long long> wk_off;
-  DevBuf<unsigned long long> g_key;
   DevBuf<long long> pp_rm_off, pp_rm_tot;
   // initial-condition sampler: staging of the modes, copy counts, radix select
   DevBuf<double> sample_buf;
@@ -1333,9 +1335,7 @@ struct Ctx {
   DevBuf<int4> it_term, ev_term;  // pending tests where chains stopped (kPendingTerm)
   // walkers made by target operations (slot, global pair), read by the next
   // round's k_items; their count is round_dev[5]
-  DevBuf<int> ppw_slot, ppw_gp;      // written by this round's k_pp_apply
-  DevBuf<int> ppw_slot_in, ppw_gp_in;  // read by this round's k_items (the round before's)
-  long long ppw_cap = 0;
+  DevBuf<int> ppw_slot, ppw_gp;  // read by a round's k_items, then written by its k_compact_walkers
   long long op_cap = 0;   // room in the target-operation arrays this round
   bool pp_step = false;   // the step has target operations (per-particle path)
   // chain events of a round (ChainPool), in chunks
@@ -1634,8 +1634,8 @@ void push_pops(Ctx& c) {
 }
 
 // words of the step graph's report, in front of the counter blocks:
-// [0..3] as k_round_end's stats, [4] why round 0 was not run (kNoGo*, 0: it
-// was), [5] samples, [6] scan look-backs that gave up, [7] round-0 events
+// [0..3] and [6..11] as k_round_end's stats, [4] why round 0 was not run
+// (kNoGo*, 0: it was), [5] samples, [12] target operations of round 0
 constexpr int kStatWords = 16;
 
 // counters of every population in one copy
@@ -2220,13 +2220,13 @@ void launch_items_kt(Ctx& c, int kt, bool flat, int n_gpairs, long long W, cudaS
   A.n_gpairs = n_gpairs;
   A.n_items = c.round_dev.p + 2;
   A.n_items_ev = c.round_dev.p + 6;
-  A.ppw_slot = c.ppw_slot_in.p;
-  A.ppw_gp = c.ppw_gp_in.p;
-  A.op_pop = c.op_pop.p;
-  A.op_pair = c.op_pair.p;
-  A.op_slot = c.op_slot.p;
-  A.op_k = c.op_k.p;
-  A.op_key = c.op_key.p;
+  A.ppw_slot = c.ppw_slot.p;
+  A.ppw_gp = c.ppw_gp.p;
+  A.op_pop = c.r_pop.p;
+  A.op_pair = c.r_pair.p;
+  A.op_slot = c.r_slot.p;
+  A.op_k = c.r_k.p;
+  A.op_key = c.r_key.p;
   A.n_ops = c.n_dev.p;
   A.op_cap = c.op_cap;
   A.win = c.win_set.p;
@@ -2267,9 +2267,8 @@ void launch_items_kt(Ctx& c, int kt, bool flat, int n_gpairs, long long W, cudaS
   note_launch();
 }
 
-__global__ void k_ops_span(long long* n_ops, long long n_redo, const long long* n_items) {
-  n_ops[0] = n_redo + *n_items;
-}
+// the round's staged target operations: the redone ones, then one place per item
+__global__ void k_ops_span(long long* n_ops, const long long* n_items) { n_ops[0] += *n_items; }
 
 // Stable grouping by population of a batched context's per-round lists.
 // Slot and ID ranks come from one scan over a list, and the per-population
@@ -2356,7 +2355,8 @@ __global__ void k_item_pops(const long long* n_items, const uint8_t* it_flag, co
 
 // dest for the entries of a list of at most bound entries (count *n on the
 // device), grouped by population (k_grp_hist, k_grp_rank)
-void group_by_pop(Ctx& c, const long long* n, long long bound, const int* pop_of, long long* dest, cudaStream_t st) {
+void group_by_pop(Ctx& c, const long long* n, long long bound, const int* pop_of, long long* dest, cudaStream_t st,
+                  long long* kept = nullptr) {
   const int n_tiles = (int)std::max<long long>(1, (bound + kGrpTile - 1) / kGrpTile);
   const long long nh = (long long)n_tiles * c.n_pop;
   c.grp_hist.reserve((size_t)nh);
@@ -2364,70 +2364,86 @@ void group_by_pop(Ctx& c, const long long* n, long long bound, const int* pop_of
   CK(cudaMemsetAsync(c.grp_hist.p, 0, sizeof(int) * (size_t)nh, st));
   k_grp_hist<<<n_tiles, kGrpTile, 0, st>>>(n, pop_of, c.n_pop, n_tiles, c.grp_hist.p, c.d_ctrs);
   note_launch();
-  scan_multi<int>(c, {ScanArg<int>{c.grp_hist.p, nh, nullptr, c.grp_off.p}}, st);
+  scan_multi<int>(c, {ScanArg<int>{c.grp_hist.p, nh, nullptr, c.grp_off.p, kept}}, st);
   k_grp_rank<<<n_tiles, kGrpTile, 0, st>>>(n, pop_of, n_tiles, c.grp_off.p, dest);
   note_launch();
 }
 
-// The round's target operations (at most Q, counted on the device): the
-// bound on each one's removals, scanned into its place in the removal pool,
-// then the operations themselves.  An operation whose place runs past the
-// pool loses, as one that lost a claim does, and is redone in the next
-// round; the host reads the round's total with its other counts and grows
-// the pool before that round.
-void launch_pp(Ctx& c, int kt, long long Q, bool grouped) {
-  int blocks = grid_for(Q, 128);
-  if (!grouped) {
-    // a later round's list: the redone operations, then one place per item
-    // (population -1 where the item made none); grouping also drops those
-    c.grp_dest.reserve((size_t)Q + 1);
-    c.g_pop.reserve(Q); c.g_pair.reserve(Q); c.g_slot.reserve(Q); c.g_k.reserve(Q); c.g_key.reserve(Q);
-    group_by_pop(c, c.n_dev.p + 0, Q, c.op_pop.p, c.grp_dest.p, c.stream);
-    k_scatter_ops<<<grid_for(Q, 256), 256, 0, c.stream>>>(c.n_dev.p + 0, c.grp_dest.p, c.op_pop.p, c.op_pair.p,
-                                                          c.op_slot.p, c.op_k.p, c.op_key.p, c.g_pop.p, c.g_pair.p,
-                                                          c.g_slot.p, c.g_k.p, c.g_key.p);
-    note_launch();
-    // the operations kept: the scan's total
-    const long long nh = (long long)std::max<long long>(1, (Q + kGrpTile - 1) / kGrpTile) * c.n_pop;
-    CK(cudaMemcpyAsync(c.n_dev.p, c.grp_off.p + nh, sizeof(long long), cudaMemcpyDeviceToDevice, c.stream));
-    std::swap(c.op_pop, c.g_pop); std::swap(c.op_pair, c.g_pair); std::swap(c.op_slot, c.g_slot);
-    std::swap(c.op_k, c.g_k); std::swap(c.op_key, c.g_key);
-  }
-  c.pp_rm_n.reserve((size_t)Q + 1);
-  c.pp_rm_off.reserve((size_t)Q + 2);
+// Buffers of a round's at most Q target operations that carry nothing from
+// the round before
+void reserve_ops(Ctx& c, long long Q) {
+  const size_t q = (size_t)Q;
+  c.op_pop.reserve(q); c.op_pair.reserve(q); c.op_slot.reserve(q); c.op_k.reserve(q); c.op_key.reserve(q);
+  c.pp_res.reserve(q);
+  c.pp_vol.reserve(q * c.n_spec);
+  c.pp_rm_n.reserve(q + 1);
+  c.pp_rm_off.reserve(q + 2);
   c.pp_rm_tot.reserve(1);
-  k_pp_count<<<blocks, 128, 0, c.stream>>>(c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p,
-                                           c.n_dev.p + 0, c.pp_rm_n.p);
-  note_launch();
-  scan_multi<int>(c, {ScanArg<int>{c.pp_rm_n.p, Q, c.n_dev.p + 0, c.pp_rm_off.p, c.pp_rm_tot.p}});
-  // every operation's removals fit the pool: one that did not would lose
-  // and draw anew a round later, so the pool's size (in a batch, the other
-  // populations' removals) would decide the particles.  One read-back; the
-  // steps that have target operations run their rounds from the host.
-  {
-    long long rm_tot = 0;
-    unsigned long long scan_err = 0;
-    CK(cudaMemcpyAsync(&rm_tot, c.pp_rm_tot.p, sizeof(rm_tot), cudaMemcpyDeviceToHost, c.stream));
-    CK(cudaMemcpyAsync(&scan_err, c.scan_err.p, sizeof(scan_err), cudaMemcpyDeviceToHost, c.stream));
-    CK(cudaStreamSynchronize(c.stream));
-    if (scan_err) {
-      CK(cudaMemsetAsync(c.scan_err.p, 0, sizeof(scan_err), c.stream));
-      throw Fail(PMC_ERR_TIMEOUT);
-    }
-    if (rm_tot < 0 || rm_tot >= (1LL << 31)) cap_throw("more than 2^31 removals in one round");
-    if (rm_tot + 1 > (long long)c.pp_rm_pool.n) c.pp_rm_pool.reserve((size_t)(rm_tot + rm_tot / 2 + 1024));
-  }
-  with_kt(c, kt, [&](auto ktc, auto) {
-    constexpr int KT = decltype(ktc)::value;
-    k_pp_ops<KT><<<grid_for(32 * Q, 32 * kPPWarps), 32 * kPPWarps, 0, c.stream>>>(c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p,
-                                               c.op_key.p, c.n_dev.p + 0, c.pp_res.p, c.pp_vol.p, c.pp_rm_off.p,
-                                               c.pp_rm_pool.p, (long long)c.pp_rm_pool.n);
-  });
+  c.need_slot_pp.reserve(q + 1); c.need_id_pp.reserve(q + 1); c.win_pp.reserve(q + 1); c.lost_pp.reserve(q + 1);
+  c.lost_off.reserve(q + 2); c.rank_slot_pp.reserve(q + 2); c.rank_id_pp.reserve(q + 2);
+  c.grp_dest.reserve(q + 1);
+  const size_t nw = q * kMaxCopies;
+  c.wk_slot.reserve(nw); c.wk_gp.reserve(nw); c.wk_flag.reserve(nw); c.wk_off.reserve(nw + 1);
+  const size_t nh = std::max<size_t>(1, (q + kGrpTile - 1) / kGrpTile) * c.n_pop;
+  c.grp_hist.reserve(nh);
+  c.grp_off.reserve(nh + 1);
+}
+
+// staging list of a later round's target operations (redone and added ones)
+void reserve_redo(Ctx& c, long long Q) {
+  const size_t q = (size_t)Q;
+  c.r_pop.reserve(q); c.r_pair.reserve(q); c.r_slot.reserve(q); c.r_k.reserve(q); c.r_key.reserve(q);
+}
+
+// A later round's target operations (at most Q staged in r_*, n_dev[0] of
+// them): the redone ones, then one place per item (population -1 where the
+// item made none).  Grouped by population into op_*, which also drops the
+// empty places; n_dev[1] counts the operations kept.
+void launch_pp_group(Ctx& c, long long Q, cudaStream_t st) {
+  group_by_pop(c, c.n_dev.p, Q, c.r_pop.p, c.grp_dest.p, st, c.n_dev.p + 1);
+  k_scatter_ops<<<grid_for(Q, 256), 256, 0, st>>>(c.n_dev.p, c.grp_dest.p, c.r_pop.p, c.r_pair.p, c.r_slot.p,
+                                                  c.r_k.p, c.r_key.p, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p,
+                                                  c.op_key.p);
   note_launch();
 }
 
-void set_n_dev(Ctx& c, long long v) {
-  CK(cudaMemcpyAsync(c.n_dev.p, &v, sizeof(long long), cudaMemcpyHostToDevice, c.stream));
+// the bound on each target operation's removals, scanned into its place in
+// the removal pool (their total in pp_rm_tot); n_ops: their count
+void launch_pp_count(Ctx& c, long long Q, const long long* n_ops, cudaStream_t st) {
+  k_pp_count<<<grid_for(Q, 128), 128, 0, st>>>(c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p, n_ops,
+                                               c.pp_rm_n.p);
+  note_launch();
+  scan_multi<int>(c, {ScanArg<int>{c.pp_rm_n.p, Q, n_ops, c.pp_rm_off.p, c.pp_rm_tot.p}}, st);
+}
+
+// Every operation's removals fit the pool: one that did not would lose
+// and draw anew a round later, so the pool's size (in a batch, the other
+// populations' removals) would decide the particles.  One read-back; in a
+// step graph the device checks it (k_step_check, k_pp_fits).
+void fit_rm_pool(Ctx& c) {
+  long long rm_tot = 0;
+  unsigned long long scan_err = 0;
+  CK(cudaMemcpyAsync(&rm_tot, c.pp_rm_tot.p, sizeof(rm_tot), cudaMemcpyDeviceToHost, c.stream));
+  CK(cudaMemcpyAsync(&scan_err, c.scan_err.p, sizeof(scan_err), cudaMemcpyDeviceToHost, c.stream));
+  CK(cudaStreamSynchronize(c.stream));
+  if (scan_err) {
+    CK(cudaMemsetAsync(c.scan_err.p, 0, sizeof(scan_err), c.stream));
+    throw Fail(PMC_ERR_TIMEOUT);
+  }
+  if (rm_tot < 0 || rm_tot >= (1LL << 31)) cap_throw("more than 2^31 removals in one round");
+  if (rm_tot + 1 > (long long)c.pp_rm_pool.n) c.pp_rm_pool.reserve((size_t)(rm_tot + rm_tot / 2 + 1024));
+  c.last_rm = std::max(c.last_rm, rm_tot);
+}
+
+// the round's target operations (n_dev[1], at most Q)
+void launch_pp_ops(Ctx& c, int kt, long long Q, cudaStream_t st) {
+  with_kt(c, kt, [&](auto ktc, auto) {
+    constexpr int KT = decltype(ktc)::value;
+    k_pp_ops<KT><<<grid_for(32 * Q, 32 * kPPWarps), 32 * kPPWarps, 0, st>>>(
+        c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p, c.op_key.p, c.n_dev.p + 1, c.pp_res.p, c.pp_vol.p,
+        c.pp_rm_off.p, c.pp_rm_pool.p, (long long)c.pp_rm_pool.n);
+  });
+  note_launch();
 }
 
 // One mc_coag call in replay mode: the grid decision of
@@ -2604,7 +2620,7 @@ __global__ void k_pop_work(const long long* pop_pair_base, int n_pop, const long
 // graph stops and the host loop, which can grow both, carries on.  Rounds
 // with per-particle redo operations run from the host loop.
 
-__global__ void k_round_begin(uint32_t* d_round, long long* round_dev, int* per_pop, int n_per_pop) {
+__global__ void k_round_begin(uint32_t* d_round, long long* round_dev, int* per_pop, int n_per_pop, long long* n_dev) {
   if (blockIdx.x != 0) return;
   if (threadIdx.x == 0) {
     d_round[0] += 1u;
@@ -2614,6 +2630,7 @@ __global__ void k_round_begin(uint32_t* d_round, long long* round_dev, int* per_
     round_dev[6] = round_dev[1];
     round_dev[7] = round_dev[5];
     round_dev[2] = round_dev[1] + round_dev[5];
+    n_dev[0] = round_dev[8];  // the target operations redone in this round
     round_dev[0] = 0;
     round_dev[1] = 0;
     round_dev[3] = 0;
@@ -2626,42 +2643,69 @@ __global__ void k_round_begin(uint32_t* d_round, long long* round_dev, int* per_
 }
 
 // stats: [0] events that lost a claim, [1] events, [2] rounds, [3] 1 if the
-// graph stopped for lack of room (slots, sort chunks, or more events than the
-// max_events its later launches are bounded by) with events left, [6] scans
-// that gave up, [7] the events of round 0
+// graph stopped for lack of room (slots, sort chunks, or more items or target
+// operations than its later launches are bounded by) with work left (2: in the
+// middle of a round, k_pp_fits), [6] scans that gave up, [7] the largest number
+// of items of a later round, [8] of its target operations, at most, [9] target
+// operations, [10] those that lost a claim, [11] the largest removal bound
 __global__ void k_round_end(const long long* round_dev, long long* stats, const uint32_t* d_round, int max_rounds,
-                            const PopDev* pops, PopCtr* ctrs, int n_pop, long long sort_slots, long long max_events,
-                            const unsigned long long* scan_err, cudaGraphConditionalHandle cond) {
-  const long long E = round_dev[1];
-  bool fits = E <= max_events;
+                            const PopDev* pops, PopCtr* ctrs, int n_pop, long long sort_slots, long long max_items,
+                            long long max_ops, const long long* n_dev, const unsigned long long* scan_err,
+                            cudaGraphConditionalHandle cond) {
+  const long long E = round_dev[1], lost = round_dev[8], items = E + round_dev[5];
+  // a step with target operations: at most one more per item
+  const long long ops = max_ops > 0 ? lost + items : 0;
+  bool fits = items <= max_items && ops <= max_ops;
   for (int k = threadIdx.x; k < n_pop; k += blockDim.x) {
-    long long need = (long long)ctrs[k].n_slots + E;
+    const long long need = (long long)ctrs[k].n_slots + items + (kMaxCopies - 1) * ops;
     if (need > (long long)pops[k].cap || need > sort_slots) fits = false;
   }
   const bool room = __syncthreads_and(fits);
-  const bool more = E > 0 && room && (int)d_round[0] + 1 < max_rounds;
-  if (E > 0 && room && !more)
+  const bool left = items > 0 || lost > 0;
+  const bool more = left && room && (int)d_round[0] + 1 < max_rounds;
+  if (left && room && !more)
     for (int k = threadIdx.x; k < n_pop; k += blockDim.x)
       if (ctrs[k].status == 0) ctrs[k].status = kErrTimeout;
   if (threadIdx.x != 0) return;
-  if (stats[2] == 0) stats[7] = E;
   stats[0] += round_dev[0];
   stats[1] += E;
   stats[2] += 1;
   stats[6] = (long long)*scan_err;
-  if (E > 0 && !room) stats[3] = 1;
+  if (items > stats[7]) stats[7] = items;
+  if (ops > stats[8]) stats[8] = ops;
+  if (max_ops > 0) {
+    stats[9] += n_dev[1];
+    stats[10] += lost;
+  }
+  if (left && !room) stats[3] = 1;
   cudaGraphSetConditional(cond, more ? 1u : 0u);
+}
+
+// The removals of a later round's target operations fit their pool: the
+// round's tail runs.  Otherwise the graph stops here and the host, which can
+// grow the pool, runs the tail.
+__global__ void k_pp_fits(const long long* rm_tot, long long pool, long long* stats, cudaGraphConditionalHandle tail,
+                          cudaGraphConditionalHandle loop) {
+  const bool fits = *rm_tot + 1 <= pool;
+  if (*rm_tot > stats[11]) stats[11] = *rm_tot;
+  if (!fits) {
+    stats[3] = 2;
+    cudaGraphSetConditional(loop, 0u);
+  }
+  cudaGraphSetConditional(tail, fits ? 1u : 0u);
 }
 
 // ---------------------------------------------------------------------------
 // A whole step as one graph: round 0 in stream order, then the later rounds'
 // WHILE node.  What round 0 needed the host for is checked on the device
-// (k_step_check): the grid is kept (aero_sorted_remake_if_needed's rule on
-// the occupied bins), no pair takes the per-particle path, the samples fit
-// the buffers, and every population has room for a particle per sample.  If
-// not, the sample total is set to zero, so the rest of the graph does nothing
-// and the host runs the step the long way.
-enum : long long { kNoGoGrid = 1, kNoGoOps = 2, kNoGoSamples = 4, kNoGoSlots = 8 };
+// (k_step_check): the grid is kept (aero_sorted_remake_if_needed's rule on the
+// occupied bins), the samples and target operations (none in a graph without
+// them) and their removals fit the buffers, every population's walks stop at
+// per-particle pairs exactly if it has target operations, and it has room for
+// a particle per sample and the copies.  If not, the totals are set to zero,
+// so the rest of the graph does nothing and the host runs the step the long
+// way.
+enum : long long { kNoGoGrid = 1, kNoGoOps = 2, kNoGoSamples = 4, kNoGoSlots = 8, kNoGoStops = 16, kNoGoPool = 32 };
 
 __global__ void k_step_begin(PopDev* pops, PopCtr* ctrs, int n_pop, uint32_t* d_round, long long* round_dev,
                              int* per_pop, long long* stat, const long long* pop_pair_base, int n_gp,
@@ -2688,12 +2732,13 @@ __global__ void k_step_begin(PopDev* pops, PopCtr* ctrs, int n_pop, uint32_t* d_
 }
 
 __global__ void k_step_check(const PopDev* pops, int n_pop, const long long* pop_pair_base, long long* work_off,
-                             const long long* pp_off, int n_gp, long long w_cap, long long sort_slots,
-                             long long* stat) {
-  const long long W = work_off[n_gp];
+                             long long* pp_off, int n_gp, long long w_cap, long long q_cap, const long long* rm_tot,
+                             long long pool, long long sort_slots, long long* n_dev, long long* stat) {
+  const long long W = work_off[n_gp], Q = pp_off[n_gp];
   long long why = 0;
-  if (pp_off[n_gp] > 0) why |= kNoGoOps;
+  if (Q > q_cap) why |= kNoGoOps;
   if (W > w_cap) why |= kNoGoSamples;
+  if (Q > 0 && q_cap > 0 && *rm_tot + 1 > pool) why |= kNoGoPool;
   for (int k = threadIdx.x; k < n_pop; k += blockDim.x) {
     const PopDev& P = pops[k];
     const GridDev& G = *P.grid;
@@ -2705,14 +2750,20 @@ __global__ void k_step_check(const PopDev* pops, int n_pop, const long long* pop
     } else if (r.bmax >= 0 || r.n_live > 0) {
       why |= kNoGoGrid;
     }
-    const long long need = (long long)r.n_slots + work_off[pop_pair_base[k + 1]] - work_off[pop_pair_base[k]];
+    const long long a = pop_pair_base[k], b = pop_pair_base[k + 1];
+    const long long Wk = work_off[b] - work_off[a], Qk = pp_off[b] - pp_off[a];
+    if ((Qk > 0) != (P.walk_stops != 0)) why |= kNoGoStops;
+    const long long need = (long long)r.n_slots + Wk + (kMaxCopies - 1) * Qk;
     if (need > (long long)P.cap || (long long)r.n_slots > sort_slots) why |= kNoGoSlots;
   }
   const int all = __syncthreads_or((int)why);
   if (threadIdx.x != 0) return;
   stat[4] = all;
   stat[5] = W;
-  if (all) work_off[n_gp] = 0;
+  stat[12] = Q;
+  if (q_cap > 0) stat[11] = *rm_tot;
+  n_dev[1] = all ? 0 : Q;
+  if (all) work_off[n_gp] = pp_off[n_gp] = 0;
 }
 
 // Resolve and apply the events of a round (E at round_dev[1], at most W) and,
@@ -2721,18 +2772,18 @@ __global__ void k_step_check(const PopDev* pops, int n_pop, const long long* pop
 void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q, bool chains) {
   long long* Ed = c.round_dev.p + 1;
   ChainPool pool = chain_pool(c);
-  // Q bounds the round's target operations; their count is n_dev[0] (the
+  // Q bounds the round's target operations; their count is n_dev[1] (the
   // redone ones, then those that walks appended)
   if (Q > 0) {
-    k_pp_resolve<<<grid_for(Q, 256), 256, 0, st>>>(c.d_pops, c.op_pop.p, c.op_key.p, c.n_dev.p, c.pp_res.p,
+    k_pp_resolve<<<grid_for(Q, 256), 256, 0, st>>>(c.d_pops, c.op_pop.p, c.op_key.p, c.n_dev.p + 1, c.pp_res.p,
                                                    c.pp_rm_pool.p, c.win_pp.p, c.need_slot_pp.p, c.need_id_pp.p, c.lost_pp.p);
     note_launch();
-    scan_multi<int>(c, {{c.need_slot_pp.p, Q, c.n_dev.p, c.rank_slot_pp.p}, {c.need_id_pp.p, Q, c.n_dev.p, c.rank_id_pp.p}},
+    scan_multi<int>(c, {{c.need_slot_pp.p, Q, c.n_dev.p + 1, c.rank_slot_pp.p}, {c.need_id_pp.p, Q, c.n_dev.p + 1, c.rank_id_pp.p}},
                     st);
-    k_count_per_pop<<<grid_for(Q, 256), 256, 0, st>>>(c.need_slot_pp.p, c.n_dev.p, c.op_pop.p,
+    k_count_per_pop<<<grid_for(Q, 256), 256, 0, st>>>(c.need_slot_pp.p, c.n_dev.p + 1, c.op_pop.p,
                                                       c.per_pop_i.p + 2 * c.n_pop);
     note_launch();
-    k_count_per_pop<<<grid_for(Q, 256), 256, 0, st>>>(c.need_id_pp.p, c.n_dev.p, c.op_pop.p,
+    k_count_per_pop<<<grid_for(Q, 256), 256, 0, st>>>(c.need_id_pp.p, c.n_dev.p + 1, c.op_pop.p,
                                                       c.per_pop_i.p + 3 * c.n_pop);
     note_launch();
   }
@@ -2800,20 +2851,19 @@ void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q, bool chain
   }
   if (Q > 0) {
     const size_t nw = (size_t)Q * kMaxCopies;
-    c.wk_slot.reserve(nw); c.wk_gp.reserve(nw); c.wk_flag.reserve(nw); c.wk_off.reserve(nw + 1);
-    k_pp_apply<<<grid_for(Q, 256), 256, 0, st>>>(c.d_pops, c.op_pop.p, c.n_dev.p, c.pp_res.p, c.pp_vol.p,
+    k_pp_apply<<<grid_for(Q, 256), 256, 0, st>>>(c.d_pops, c.op_pop.p, c.n_dev.p + 1, c.pp_res.p, c.pp_vol.p,
                                                  c.pp_rm_pool.p, c.win_pp.p, c.rank_slot_pp.p, c.rank_id_pp.p,
                                                  c.slot_base_pp.p, c.id_base_pp.p, c.pop_pair_base.p, c.op_k.p,
                                                  c.wk_slot.p, c.wk_gp.p, c.wk_flag.p);
     note_launch();
-    k_walkers_span<<<1, 1, 0, st>>>(c.n_dev.p, c.round_dev.p + 9);
+    k_walkers_span<<<1, 1, 0, st>>>(c.n_dev.p + 1, c.round_dev.p + 9);
     note_launch();
     scan_multi<uint8_t>(c, {ScanArg<uint8_t>{c.wk_flag.p, (long long)nw, c.round_dev.p + 9, c.wk_off.p,
                                              c.round_dev.p + 5}}, st);
     k_compact_walkers<<<grid_for((long long)nw, 256), 256, 0, st>>>(c.round_dev.p + 9, c.wk_flag.p, c.wk_off.p,
                                                                     c.wk_slot.p, c.wk_gp.p, c.ppw_slot.p, c.ppw_gp.p);
     note_launch();
-    scan_multi<int>(c, {ScanArg<int>{c.lost_pp.p, Q, c.n_dev.p, c.lost_off.p, c.round_dev.p + 8}}, st);
+    scan_multi<int>(c, {ScanArg<int>{c.lost_pp.p, Q, c.n_dev.p + 1, c.lost_off.p, c.round_dev.p + 8}}, st);
   }
 }
 
@@ -2843,6 +2893,25 @@ void launch_compact_samples(Ctx& c, const long long* n, long long W, cudaStream_
   note_launch();
 }
 
+// a buffer's growth that keeps what it holds
+template <class T>
+void grow_keeping(Ctx& c, DevBuf<T>& b, size_t m) {
+  if (m <= b.n) return;
+  DevBuf<T> nb;
+  nb.reserve(std::max(m, b.n + b.n / 2));
+  if (b.n) CK(cudaMemcpyAsync(nb.p, b.p, b.n * sizeof(T), cudaMemcpyDeviceToDevice, c.stream));
+  CK(cudaStreamSynchronize(c.stream));
+  std::swap(nb, b);
+  nb.release();
+}
+
+// round 0's target operations
+void launch_build_ops(Ctx& c, int n_gpairs, cudaStream_t st) {
+  k_build_ops<<<n_gpairs, 128, 0, st>>>(c.d_pops, c.gpair_pop.p, c.gpair_local.p, c.pp_off.p, n_gpairs, c.op_pop.p,
+                                        c.op_pair.p, c.op_slot.p, c.op_k.p, c.op_key.p);
+  note_launch();
+}
+
 struct RoundBounds {
   int kt;
   bool flat;
@@ -2852,35 +2921,38 @@ struct RoundBounds {
   int max_cells;
 };
 
-// The kernels of one later round on stream st, after k_round_begin: the
-// sort, items, their events in item order, then resolve and apply.  With
-// Q > 0 (host loop only) the round's per-particle redo operations claim
-// alongside.
-// Qn: the round's redone target operations (host loop only); with
-// per-particle pairs in the step, walks append more (at most one per item),
-// so the operations are bounded by Qb = Qn + W and counted on the device.
-void enqueue_round_body(Ctx& c, cudaStream_t st, const RoundBounds& b, long long Qn) {
-  long long W = b.W;
-  const long long Q = c.pp_step ? Qn + W : Qn;
+// The kernels of one later round on stream st, after k_round_begin, in two
+// parts.  The head: the sort, the items and their chains and, with Q > 0 (a
+// step with target operations), the round's at most Q target operations: the
+// redone ones (k_build_redo staged them, before k_round_begin) and those that
+// walks add (at most one per item), with the bound of their removals.  The
+// tail, once the removals fit their pool: the operations, which claim
+// alongside, the items' events in item order, then resolve and apply.
+void enqueue_round_head(Ctx& c, cudaStream_t st, const RoundBounds& b, long long Q) {
   launch_sort(c, st, b.max_chunks, b.max_cells);
   {
     dim3 g(b.max_cells, c.n_pop);
     k_walk_rates<<<g, 128, 0, st>>>(c.d_pops);
     note_launch();
   }
-  if (Q > 0) set_n_dev(c, Qn);
-  launch_items_kt(c, b.kt, b.flat, b.n_gpairs, W, st);
+  launch_items_kt(c, b.kt, b.flat, b.n_gpairs, b.W, st);
   if (Q > 0) {
-    k_ops_span<<<1, 1, 0, st>>>(c.n_dev.p, Qn, c.round_dev.p + 2);  // redone ones + one place per item
+    k_ops_span<<<1, 1, 0, st>>>(c.n_dev.p, c.round_dev.p + 2);
     note_launch();
-    launch_pp(c, b.kt, Q, false);
+    launch_pp_group(c, Q, st);
+    launch_pp_count(c, Q, c.n_dev.p + 1, st);
   }
+}
+
+void enqueue_round_tail(Ctx& c, cudaStream_t st, const RoundBounds& b, long long Q) {
+  const long long W = b.W;
+  if (Q > 0) launch_pp_ops(c, b.kt, Q, st);
   const long long* Id = c.round_dev.p + 2;
   // a batched step with target operations: the walkers they made join the
   // items after the events, from every population, so the events are
   // grouped by population for the allocation (group_by_pop)
   const long long* grouped = nullptr;
-  if (c.pp_step && c.n_pop > 1) {
+  if (Q > 0 && c.n_pop > 1) {
     c.item_pop.reserve((size_t)W + 1);
     c.grp_dest.reserve((size_t)W + 1);
     k_item_pops<<<grid_for(W, 256), 256, 0, st>>>(Id, c.it_flag.p, c.it_gp.p, c.gpair_pop.p, b.n_gpairs,
@@ -2894,6 +2966,13 @@ void enqueue_round_body(Ctx& c, cudaStream_t st, const RoundBounds& b, long long
       c.it_done.p, c.it_dec.p, c.it_term.p, c.ev_head.p, c.ev_done.p, grouped);
   note_launch();
   resolve_apply(c, st, W, Q, true);
+}
+
+void launch_build_redo(Ctx& c, long long Q, cudaStream_t st) {
+  k_build_redo<<<grid_for(Q, 256), 256, 0, st>>>(c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p, c.op_key.p,
+                                                 c.lost_pp.p, c.lost_off.p, c.n_dev.p + 1, c.r_pop.p, c.r_pair.p,
+                                                 c.r_slot.p, c.r_k.p, c.r_key.p);
+  note_launch();
 }
 
 // everything the captured launches depend on: sizes and device addresses
@@ -3006,7 +3085,7 @@ GraphRun run_round_graph(Ctx& c, int kt, bool flat, int n_gpairs, long long e0) 
   size_sort(c, b.max_cells);
   // every other buffer at its final size before the addresses are taken
   reserve_round(c, b.W);
-  c.graph_stats.reserve(8);
+  c.graph_stats.reserve(kStatWords);
   {
     const long long nb = (b.W + kScanTile - 1) / kScanTile;
     c.scan_status.reserve((size_t)std::max(kScanMaxJobs * nb, b.W / kResolveMin + 2));
@@ -3041,11 +3120,12 @@ GraphRun run_round_graph(Ctx& c, int kt, bool flat, int n_gpairs, long long e0) 
     long long n0 = g_launches;
     CK(cudaStreamBeginCaptureToGraph(c.cap_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     try {
-      k_round_begin<<<1, 128, 0, c.cap_stream>>>(c.d_round, c.round_dev.p, c.per_pop_i.p, 4 * c.n_pop);
+      k_round_begin<<<1, 128, 0, c.cap_stream>>>(c.d_round, c.round_dev.p, c.per_pop_i.p, 4 * c.n_pop, c.n_dev.p);
       note_launch();
-      enqueue_round_body(c, c.cap_stream, b, 0);
+      enqueue_round_head(c, c.cap_stream, b, 0);
+      enqueue_round_tail(c, c.cap_stream, b, 0);
       k_round_end<<<1, 128, 0, c.cap_stream>>>(c.round_dev.p, c.graph_stats.p, c.d_round, c.max_rounds, c.d_pops,
-                                               c.d_ctrs, c.n_pop, (long long)b.max_chunks * kChunk, b.W,
+                                               c.d_ctrs, c.n_pop, (long long)b.max_chunks * kChunk, b.W, 0, c.n_dev.p,
                                                c.scan_err.p, cond);
       note_launch();
     } catch (...) {
@@ -3064,7 +3144,7 @@ GraphRun run_round_graph(Ctx& c, int kt, bool flat, int n_gpairs, long long e0) 
     c.rg_key = key;
     c.rg_builds++;
   }
-  CK(cudaMemsetAsync(c.graph_stats.p, 0, sizeof(long long) * 8, c.stream));
+  CK(cudaMemsetAsync(c.graph_stats.p, 0, sizeof(long long) * kStatWords, c.stream));
   {
     ProfScope ps(c, 2, 1);
     CK(cudaGraphLaunch(c.rg_exec, c.stream));
@@ -3138,9 +3218,21 @@ void free_step_graph(Ctx& c) {
 }
 
 // what the step graph's captured launches depend on, beyond round_graph_key
-std::vector<long long> step_graph_key(const Ctx& c, const RoundBounds& b, long long w_cap, int max_pairs) {
+std::vector<long long> step_graph_key(const Ctx& c, const RoundBounds& b, long long w_cap, int max_pairs,
+                                      long long q_cap, long long qb_cap) {
   std::vector<long long> k = round_graph_key(c, b);
-  for (long long v : {w_cap, (long long)max_pairs, (long long)c.prof, (long long)c.tune.threads[kTuneTest],
+  if (q_cap > 0)
+    for (long long v :
+         {q_cap, qb_cap, (long long)c.op_pop.p, (long long)c.op_pair.p, (long long)c.op_slot.p, (long long)c.op_k.p,
+          (long long)c.op_key.p, (long long)c.r_pop.p, (long long)c.r_pair.p, (long long)c.r_slot.p,
+          (long long)c.r_k.p, (long long)c.r_key.p, (long long)c.pp_res.p, (long long)c.pp_vol.p,
+          (long long)c.pp_rm_n.p, (long long)c.pp_rm_off.p, (long long)c.pp_rm_tot.p, (long long)c.pp_rm_pool.p,
+          (long long)c.pp_rm_pool.n, (long long)c.need_slot_pp.p, (long long)c.need_id_pp.p, (long long)c.win_pp.p,
+          (long long)c.lost_pp.p, (long long)c.lost_off.p, (long long)c.rank_slot_pp.p, (long long)c.rank_id_pp.p,
+          (long long)c.grp_dest.p, (long long)c.grp_hist.p, (long long)c.grp_off.p, (long long)c.item_pop.p,
+          (long long)c.wk_slot.p, (long long)c.wk_gp.p, (long long)c.wk_flag.p, (long long)c.wk_off.p})
+      k.push_back(v);
+  for (long long v : {(long long)c.n_dev.p, w_cap, (long long)max_pairs, (long long)c.prof, (long long)c.tune.threads[kTuneTest],
                       (long long)c.nwork_set.p, (long long)c.nwork_pp.p, (long long)c.work_off.p,
                       (long long)c.pp_off.p, (long long)c.flag.p, (long long)c.ev.p, (long long)c.ev_gp.p,
                       (long long)c.d_stat})
@@ -3150,7 +3242,7 @@ std::vector<long long> step_graph_key(const Ctx& c, const RoundBounds& b, long l
 
 // The step graph's nodes, captured on c.cap_stream: round 0, then the WHILE
 // node over the later rounds.
-void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_pairs) {
+void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_pairs, long long q_cap, long long qb_cap) {
   CK(cudaGraphCreate(&c.sg_graph, 0));
   cudaGraphConditionalHandle cond;
   CK(cudaGraphConditionalHandleCreate(&cond, c.sg_graph, 0, cudaGraphCondAssignDefault));
@@ -3176,49 +3268,69 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
     note_launch();
     scan_multi<long long>(c, {{c.nwork_set.p, n_gp, nullptr, c.work_off.p}, {c.nwork_pp.p, n_gp, nullptr, c.pp_off.p}},
                           st);
-    k_step_check<<<1, 256, 0, st>>>(c.d_pops, c.n_pop, c.pop_pair_base.p, c.work_off.p, c.pp_off.p, n_gp, w_cap,
-                                    sort_slots, c.d_stat);
+    if (q_cap > 0) {
+      launch_build_ops(c, n_gp, st);
+      launch_pp_count(c, q_cap, c.pp_off.p + n_gp, st);
+    }
+    k_step_check<<<1, 256, 0, st>>>(c.d_pops, c.n_pop, c.pop_pair_base.p, c.work_off.p, c.pp_off.p, n_gp, w_cap, q_cap,
+                                    c.pp_rm_tot.p, (long long)c.pp_rm_pool.n, sort_slots, c.n_dev.p, c.d_stat);
     note_launch();
+    if (q_cap > 0) launch_pp_ops(c, b.kt, q_cap, st);
     mark(2);
     launch_test_kt(c, b.kt, b.flat, n_gp, w_cap, st);
     mark(3);
     const long long* Wd = c.work_off.p + n_gp;
     launch_compact_samples(c, Wd, w_cap, st);
-    resolve_apply(c, st, w_cap, 0, false);
+    resolve_apply(c, st, w_cap, q_cap, false);
     k_round_end<<<1, 128, 0, st>>>(c.round_dev.p, c.d_stat, c.d_round, c.max_rounds, c.d_pops, c.d_ctrs, c.n_pop,
-                                   sort_slots, b.W, c.scan_err.p, cond);
+                                   sort_slots, b.W, qb_cap, c.n_dev.p, c.scan_err.p, cond);
     note_launch();
     mark(4);
     c.sg_nodes0 = g_launches - n0;
-    // the WHILE node follows the launches captured so far, and what the
+    // a conditional node follows the launches captured so far, and what the
     // stream captures next follows it
-    cudaStreamCaptureStatus cs;
-    unsigned long long id = 0;
-    cudaGraph_t g = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t n_deps = 0;
-    CK(cudaStreamGetCaptureInfo_v2(st, &cs, &id, &g, &deps, &n_deps));
-    std::vector<cudaGraphNode_t> dv(deps, deps + n_deps);
-    cudaGraphNodeParams np = {};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = cond;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t node;
-    CK(cudaGraphAddNode(&node, c.sg_graph, dv.data(), dv.size(), &np));
-    CK(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
+    auto add_conditional = [&](cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type) {
+      cudaStreamCaptureStatus cs;
+      unsigned long long id = 0;
+      cudaGraph_t g = nullptr;
+      const cudaGraphNode_t* deps = nullptr;
+      size_t n_deps = 0;
+      CK(cudaStreamGetCaptureInfo_v2(st, &cs, &id, &g, &deps, &n_deps));
+      std::vector<cudaGraphNode_t> dv(deps, deps + n_deps);
+      cudaGraphNodeParams np = {};
+      np.type = cudaGraphNodeTypeConditional;
+      np.conditional.handle = h;
+      np.conditional.type = type;
+      np.conditional.size = 1;
+      cudaGraphNode_t node;
+      CK(cudaGraphAddNode(&node, g, dv.data(), dv.size(), &np));
+      CK(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
+      return np.conditional.phGraph_out[0];
+    };
+    cudaGraph_t body = add_conditional(cond, cudaGraphCondTypeWhile);
     mark(5);
     CK(cudaStreamEndCapture(st, &done));
     const long long n1 = g_launches;
-    CK(cudaStreamBeginCaptureToGraph(st, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                     cudaStreamCaptureModeRelaxed));
-    k_round_begin<<<1, 128, 0, st>>>(c.d_round, c.round_dev.p, c.per_pop_i.p, 4 * c.n_pop);
+    CK(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+    if (qb_cap > 0) launch_build_redo(c, qb_cap, st);
+    k_round_begin<<<1, 128, 0, st>>>(c.d_round, c.round_dev.p, c.per_pop_i.p, 4 * c.n_pop, c.n_dev.p);
     note_launch();
     c.fork = true;
-    enqueue_round_body(c, st, b, 0);
+    enqueue_round_head(c, st, b, qb_cap);
+    if (qb_cap > 0) {
+      // the tail runs if the round's removals fit their pool
+      cudaGraphConditionalHandle fits;
+      CK(cudaGraphConditionalHandleCreate(&fits, body, 0, cudaGraphCondAssignDefault));
+      k_pp_fits<<<1, 1, 0, st>>>(c.pp_rm_tot.p, (long long)c.pp_rm_pool.n, c.d_stat, fits, cond);
+      note_launch();
+      cudaGraph_t tail = add_conditional(fits, cudaGraphCondTypeIf);
+      CK(cudaStreamEndCapture(st, &done));
+      CK(cudaStreamBeginCaptureToGraph(st, tail, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+    }
+    enqueue_round_tail(c, st, b, qb_cap);
     c.fork = false;
     k_round_end<<<1, 128, 0, st>>>(c.round_dev.p, c.d_stat, c.d_round, c.max_rounds, c.d_pops, c.d_ctrs, c.n_pop,
-                                   sort_slots, b.W, c.scan_err.p, cond);
+                                   sort_slots, b.W, qb_cap, c.n_dev.p, c.scan_err.p, cond);
     note_launch();
     c.sg_nodes = g_launches - n1;
   } catch (...) {
@@ -3236,8 +3348,12 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
 
 struct StepRun {
   bool ran = false;   // round 0 ran on the device
-  bool stopped = false;  // events are left: the host loop carries on after `rounds` rounds
-  long long rounds = 0, losers = 0, events = 0;
+  // 1: work is left, the host loop carries on after `rounds` rounds; 2: also
+  // the last round's tail (the removals of its target operations did not fit)
+  int stopped = 0;
+  long long rounds = 0, losers = 0, events = 0, ops = 0, ops_lost = 0;
+  RoundBounds b;
+  long long Q = 0;    // bound of a later round's target operations
 };
 
 // Run this step as the graph, if what it relies on holds: a valid sort and
@@ -3250,7 +3366,7 @@ struct StepRun {
 // 0.689 for 1e6 particles of 20 species.
 StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   StepRun out;
-  if (!c.use_graph || c.tuner.on || !c.ctrs_fresh || c.last_w < 0 || c.pp_step) return out;
+  if (!c.use_graph || c.tuner.on || !c.ctrs_fresh || c.last_w < 0) return out;
   if (c.claim_gen + 1 + (uint32_t)c.max_rounds + 2u >= kGenLimit) return out;  // the generations restart
   if (c.base_cached.size() != (size_t)c.n_pop + 1) return out;
   RoundBounds b;
@@ -3260,7 +3376,7 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   long long slots = 0, min_slots = -1;
   for (int k = 0; k < c.n_pop; k++) {
     const PopHost& ph = c.pops[k];
-    if (!ph.valid_sort || !caches_current(c, ph) || !ph.h.kmax_valid || !ph.h.pair_setup_valid || ph.h.walk_stops ||
+    if (!ph.valid_sort || !caches_current(c, ph) || !ph.h.kmax_valid || !ph.h.pair_setup_valid || (ph.h.walk_stops && !c.pp_step) ||
         c.base_cached[k + 1] - c.base_cached[k] != ph.h.n_pairs)
       return out;
     b.flat = b.flat && ph.h.flat;
@@ -3273,11 +3389,19 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   const long long w = graph_bound(c.last_w + c.last_w / 4), e = graph_bound(c.last_e0 + c.last_e0 / 4);
   if (w > c.sg_w || 16 * w <= c.sg_w) c.sg_w = w;
   if (e > c.sg_e || 16 * e <= c.sg_e) c.sg_e = e;
-  b.W = std::min(c.sg_e, c.sg_w);
+  long long q_cap = 0, qb_cap = 0;
+  if (c.pp_step) {
+    const long long q = graph_bound(c.last_q + c.last_q / 4), qb = graph_bound(c.last_qb + c.last_qb / 4);
+    if (q > c.sg_q || 16 * q <= c.sg_q) c.sg_q = q;
+    if (qb > c.sg_qb || 16 * qb <= c.sg_qb) c.sg_qb = qb;
+    q_cap = c.sg_q;
+    qb_cap = c.sg_qb;
+  }
+  b.W = c.pp_step ? c.sg_e : std::min(c.sg_e, c.sg_w);
   b.n_gpairs = padded_pairs(c.base_cached[c.n_pop]);
   max_pairs = (max_pairs + 511) / 512 * 512;
   b.max_cells = (max_cells_of(c) + 15) / 16 * 16;
-  b.max_chunks = (int)((slots + 4 * b.W + kChunk - 1) / kChunk);
+  b.max_chunks = (int)((slots + 4 * b.W + kMaxCopies * qb_cap + kChunk - 1) / kChunk);
   b.max_chunks = (b.max_chunks + 15) / 16 * 16;
   prepare_chunks(c, (long long)b.max_chunks * kChunk - min_slots);
   size_sort(c, b.max_cells);
@@ -3289,28 +3413,47 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   c.pp_off.reserve(ng);
   const size_t ws = (size_t)c.sg_w;
   c.flag.reserve(ws + 1); c.ev.reserve(ws + 1); c.ev_gp.reserve(ws + 1);
-  reserve_events(c, c.sg_w);
+  reserve_events(c, std::max(c.sg_w + kMaxCopies * q_cap, b.W));
   reserve_round(c, b.W);
+  c.pp_rm_tot.reserve(1);
+  if (q_cap > 0) {
+    const long long q = std::max(q_cap, qb_cap);
+    reserve_ops(c, q);
+    reserve_redo(c, q);
+    c.ppw_slot.reserve((size_t)(kMaxCopies * (q + 1)));
+    c.ppw_gp.reserve((size_t)(kMaxCopies * (q + 1)));
+    if (c.n_pop > 1) {
+      c.item_pop.reserve((size_t)b.W + 1);
+      c.grp_dest.reserve((size_t)b.W + 1);
+      const size_t nh = (size_t)((b.W + kGrpTile - 1) / kGrpTile) * c.n_pop;
+      c.grp_hist.reserve(nh);
+      c.grp_off.reserve(nh + 1);
+    }
+    // twice the largest bound seen, so that it seldom grows
+    if (2 * c.last_rm + 1024 > (long long)c.pp_rm_pool.n) c.pp_rm_pool.reserve((size_t)(4 * c.last_rm + 65536));
+  }
   {
-    const long long nb = std::max<long long>((c.sg_w + kScanTile - 1) / kScanTile, (b.n_gpairs + kScanTile - 1) / kScanTile);
-    c.scan_status.reserve((size_t)std::max(kScanMaxJobs * nb, c.sg_w / kResolveMin + 2));
+    const long long qs = std::max(q_cap, qb_cap), hist = (std::max(qs, q_cap > 0 ? b.W : 0) / kGrpTile + 2) * c.n_pop;
+    const long long lists = std::max(std::max(kMaxCopies * qs, hist), (long long)b.n_gpairs);
+    const long long nb = std::max((c.sg_w + kScanTile - 1) / kScanTile, (lists + kScanTile - 1) / kScanTile);
+    c.scan_status.reserve((size_t)std::max(kScanMaxJobs * nb, std::max(c.sg_w, b.W) / kResolveMin + 2));
     if (c.scan_status.n > c.scan_status_n) {
       CK(cudaMemsetAsync(c.scan_status.p, 0, sizeof(unsigned long long) * c.scan_status.n, c.stream));
       c.scan_status_n = c.scan_status.n;
     }
   }
-  c.op_cap = 0;
+  c.op_cap = qb_cap;
   if (c.prof)
     for (auto& ev : c.sg_ev)
       if (!ev) CK(cudaEventCreate(&ev));
-  const std::vector<long long> key = step_graph_key(c, b, c.sg_w, max_pairs);
+  const std::vector<long long> key = step_graph_key(c, b, c.sg_w, max_pairs, q_cap, qb_cap);
   if (key != c.sg_key) {
     if (key != c.sg_seen) {  // captured when the bounds and addresses hold for two steps
       c.sg_seen = key;
       return out;
     }
     free_step_graph(c);
-    capture_step_graph(c, b, c.sg_w, max_pairs);
+    capture_step_graph(c, b, c.sg_w, max_pairs, q_cap, qb_cap);
     c.sg_key = key;
   }
   if (c.dirty || !params_same) {
@@ -3326,6 +3469,8 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   long long stat[kStatWords];
   memcpy(stat, c.stat_buf.data(), sizeof(stat));
   c.last_w = stat[5];
+  c.last_q = stat[12];
+  c.last_rm = std::max(c.last_rm, stat[11]);
   if (stat[4]) {
     c.ctrs_fresh = false;
     return out;  // nothing was tested; the long way starts the step over
@@ -3348,17 +3493,23 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
     }
   }
   g_launches += c.sg_nodes0 + c.sg_nodes * (stat[2] - 1);
-  c.claim_gen += (uint32_t)stat[2];
+  c.claim_gen += (uint32_t)(stat[2] + (stat[3] == 2 ? 1 : 0));  // a round left in the middle has begun
   c.last_e0 = stat[7];
+  c.last_qb = stat[8];
   out.ran = true;
   out.rounds = stat[2];
   out.losers = stat[0];
   out.events = stat[1];
-  out.stopped = stat[3] != 0;
+  out.ops = stat[9];
+  out.ops_lost = stat[10];
+  out.stopped = (int)stat[3];
+  out.b = b;
+  out.Q = qb_cap;
   return out;
 }
 
-void step_rounds(Ctx& c, int kt, bool flat, int n_gpairs, long long Q, int round, long long redraws, bool graph_tried);
+void step_rounds(Ctx& c, int kt, bool flat, int n_gpairs, long long Q, int round, bool counted, long long redraws,
+                 bool graph_tried);
 
 // params_same: the populations' parameters are those of the last step
 void step_parallel(Ctx& c, int kt, bool params_same) {
@@ -3366,15 +3517,19 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
     const StepRun g = run_step_graph(c, kt, params_same);
     if (g.ran) {
       c.last_set_losers = g.losers;
-      c.last_pp_lost = c.last_ops = 0;
+      c.last_pp_lost = g.ops_lost;
+      c.last_ops = g.ops;
       c.last_events = g.events;
-      c.last_redraws = g.losers;
+      c.last_redraws = g.losers + g.ops_lost;
       c.last_rounds = g.rounds;
       if (!g.stopped) return;
       c.ctrs_fresh = false;
-      bool flat = true;
-      for (int k = 0; k < c.n_pop; k++) flat = flat && c.pops[k].h.flat;
-      step_rounds(c, kt, flat, (int)c.base_cached[c.n_pop], 0, (int)g.rounds, g.losers, true);
+      if (g.stopped == 2) {
+        fit_rm_pool(c);
+        enqueue_round_tail(c, c.stream, g.b, g.Q);
+      }
+      step_rounds(c, kt, g.b.flat, (int)c.base_cached[c.n_pop], g.Q, (int)g.rounds, g.stopped != 2, g.losers + g.ops_lost,
+                  true);
       return;
     }
   }
@@ -3514,12 +3669,9 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
     // the walkers that target operations make (the target and its copies)
     // join a later round's items and events
     reserve_events(c, W + kMaxCopies * Q);
-    c.ppw_cap = kMaxCopies * (Q + 1);
-    c.ppw_slot.reserve((size_t)c.ppw_cap);
-    c.ppw_gp.reserve((size_t)c.ppw_cap);
+    c.ppw_slot.reserve((size_t)(kMaxCopies * (Q + 1)));
+    c.ppw_gp.reserve((size_t)(kMaxCopies * (Q + 1)));
     c.op_cap = Q;
-    c.need_slot_pp.reserve(Q + 1); c.need_id_pp.reserve(Q + 1); c.win_pp.reserve(Q + 1); c.lost_pp.reserve(Q + 1);
-    c.lost_off.reserve(Q + 2); c.rank_slot_pp.reserve(Q + 2); c.rank_id_pp.reserve(Q + 2);
   }
   if (c.dirty) push_pops(c);
   CK(cudaMemsetAsync(c.round_dev.p, 0, sizeof(long long) * 12, c.stream));
@@ -3529,14 +3681,12 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
     launch_test_kt(c, kt, flat, n_gpairs, W, c.stream);
   }
   if (Q > 0) {
-    c.op_pop.reserve(Q); c.op_pair.reserve(Q); c.op_slot.reserve(Q); c.op_k.reserve(Q); c.op_key.reserve(Q);
-    k_build_ops<<<n_gpairs, 128, 0, c.stream>>>(c.d_pops, c.gpair_pop.p, c.gpair_local.p, c.pp_off.p, n_gpairs,
-                                                c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p, c.op_key.p);
-    note_launch();
-    c.pp_res.reserve(Q);
-    c.pp_vol.reserve((size_t)Q * c.n_spec);
-    set_n_dev(c, Q);
-    launch_pp(c, kt, Q, true);  // built in population order
+    reserve_ops(c, Q);
+    launch_build_ops(c, n_gpairs, c.stream);
+    CK(cudaMemcpyAsync(c.n_dev.p + 1, &Q, sizeof(long long), cudaMemcpyHostToDevice, c.stream));
+    launch_pp_count(c, Q, c.n_dev.p + 1, c.stream);  // built in population order
+    fit_rm_pool(c);
+    launch_pp_ops(c, kt, Q, c.stream);
   }
   // accepted samples in sample order; the sample count is work_off[n_gpairs]
   // and the event count E goes to round_dev[1], both on the device
@@ -3547,19 +3697,20 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
   resolve_apply(c, c.stream, W, Q, false);
 
   c.last_w = W;
-  step_rounds(c, kt, flat, n_gpairs, Q, 0, 0, false);
+  c.last_q = Q;
+  c.last_e0 = c.last_qb = 0;
+  step_rounds(c, kt, flat, n_gpairs, Q, 0, false, 0, false);
 }
 
 // The later rounds: retries, walks and per-particle redo operations, from the
 // end of round 0 (round = 0, its Q target operations), or from a round at
-// which a graph stopped for lack of room (round > 0: that many rounds are
-// counted already).
-void step_rounds(Ctx& c, int kt, bool flat, int n_gpairs, long long Q, int round, long long redraws,
+// which a graph stopped for lack of room, after `round` rounds (counted: the
+// last one's counts are in the statistics already).
+void step_rounds(Ctx& c, int kt, bool flat, int n_gpairs, long long Q, int round, bool counted, long long redraws,
                  bool graph_tried) {
   std::vector<int> per_pop(4 * (size_t)c.n_pop);
   long long E = 0, pp_lost = 0;
   long long last_qb = Q;  // bound of the last round's target operations (0: it had none)
-  bool counted = round > 0;
   for (;;) {
     // one read-back at the end of each host round
     long long losers = 0, ppw = 0;
@@ -3570,7 +3721,7 @@ void step_rounds(Ctx& c, int kt, bool flat, int n_gpairs, long long Q, int round
     pp_lost = 0;
     if (last_qb > 0) {
       CK(cudaMemcpyAsync(&pp_lost, c.round_dev.p + 8, sizeof(long long), cudaMemcpyDeviceToHost, c.stream));
-      CK(cudaMemcpyAsync(&Qr, c.n_dev.p, sizeof(long long), cudaMemcpyDeviceToHost, c.stream));
+      CK(cudaMemcpyAsync(&Qr, c.n_dev.p + 1, sizeof(long long), cudaMemcpyDeviceToHost, c.stream));
     }
     CK(cudaMemcpyAsync(per_pop.data(), c.per_pop_i.p, sizeof(int) * 4 * c.n_pop, cudaMemcpyDeviceToHost, c.stream));
     unsigned long long scan_err = 0;
@@ -3587,7 +3738,6 @@ void step_rounds(Ctx& c, int kt, bool flat, int n_gpairs, long long Q, int round
       c.last_pp_lost += pp_lost;
       c.last_events += E;
       c.last_ops += Qr;
-      if (round == 0) c.last_e0 = E;
       round++;
     }
     counted = false;
@@ -3602,6 +3752,8 @@ void step_rounds(Ctx& c, int kt, bool flat, int n_gpairs, long long Q, int round
     // this round's target operations: the redone ones, and with per-particle
     // pairs in the step at most one more per item (a walk that stops there)
     const long long Qb = pp_lost + (c.pp_step ? E + ppw : 0);
+    c.last_e0 = std::max(c.last_e0, E + ppw);
+    c.last_qb = std::max(c.last_qb, Qb);
     // room for this round's new slots: at most one per item, and
     // kMaxCopies - 1 per target operation
     ensure_room(c, E + ppw + (kMaxCopies - 1) * Qb);
@@ -3633,44 +3785,27 @@ void step_rounds(Ctx& c, int kt, bool flat, int n_gpairs, long long Q, int round
     }
     // one host-driven round
     reserve_round(c, E + ppw);
-    long long Qn = pp_lost;
-    if (Qn > 0) {
-      c.r_pop.reserve(Qb); c.r_pair.reserve(Qb); c.r_slot.reserve(Qb); c.r_k.reserve(Qb); c.r_key.reserve(Qb);
-      k_build_redo<<<grid_for(last_qb, 256), 256, 0, c.stream>>>(c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p,
-                                                                 c.op_k.p, c.op_key.p, c.lost_pp.p, c.lost_off.p,
-                                                                 c.n_dev.p, c.r_pop.p, c.r_pair.p, c.r_slot.p,
-                                                                 c.r_k.p, c.r_key.p);
-      note_launch();
-      std::swap(c.op_pop, c.r_pop); std::swap(c.op_pair, c.r_pair); std::swap(c.op_slot, c.r_slot);
-      std::swap(c.op_k, c.r_k); std::swap(c.op_key, c.r_key);
-    } else if (Qb > 0) {
-      c.op_pop.reserve(Qb); c.op_pair.reserve(Qb); c.op_slot.reserve(Qb); c.op_k.reserve(Qb); c.op_key.reserve(Qb);
-    }
-    if (Qb > 0) {
-      c.pp_res.reserve(Qb);
-      c.pp_vol.reserve((size_t)Qb * c.n_spec);
-      c.need_slot_pp.reserve(Qb + 1); c.need_id_pp.reserve(Qb + 1); c.win_pp.reserve(Qb + 1);
-      c.lost_pp.reserve(Qb + 1); c.lost_off.reserve(Qb + 2); c.rank_slot_pp.reserve(Qb + 2);
-      c.rank_id_pp.reserve(Qb + 2);
-    }
+    // the operations that lost are staged for this round before their
+    // buffers, which they are read from, may grow
+    if (Qb > 0) reserve_redo(c, Qb);
+    if (pp_lost > 0) launch_build_redo(c, last_qb, c.stream);
+    if (Qb > 0) reserve_ops(c, Qb);
     c.op_cap = Qb;
-    // the walkers the last round's operations made are this round's to read;
-    // this round's operations write theirs into the other pair of arrays
-    std::swap(c.ppw_slot, c.ppw_slot_in);
-    std::swap(c.ppw_gp, c.ppw_gp_in);
-    c.ppw_cap = kMaxCopies * (Qb + 1);
-    c.ppw_slot.reserve((size_t)c.ppw_cap);
-    c.ppw_gp.reserve((size_t)c.ppw_cap);
+    // the walkers the last round's operations made are this round's to read
+    grow_keeping(c, c.ppw_slot, (size_t)(kMaxCopies * (Qb + 1)));
+    grow_keeping(c, c.ppw_gp, (size_t)(kMaxCopies * (Qb + 1)));
     // the round's sort covers the current slots exactly
     prepare_chunks(c);
     int mc = 1;
     for (int k = 0; k < c.n_pop; k++) mc = std::max(mc, c.pops[k].h.n_chunks);
     if (c.dirty) push_pops(c);
     RoundBounds b{kt, flat, n_gpairs, E + ppw, mc, max_cells_of(c)};
-    k_round_begin<<<1, 128, 0, c.stream>>>(c.d_round, c.round_dev.p, c.per_pop_i.p, 4 * c.n_pop);
+    k_round_begin<<<1, 128, 0, c.stream>>>(c.d_round, c.round_dev.p, c.per_pop_i.p, 4 * c.n_pop, c.n_dev.p);
     note_launch();
     c.claim_gen++;  // as k_round_begin on the device
-    enqueue_round_body(c, c.stream, b, Qn);
+    enqueue_round_head(c, c.stream, b, Qb);
+    if (Qb > 0) fit_rm_pool(c);
+    enqueue_round_tail(c, c.stream, b, Qb);
     last_qb = Qb;
   }
   c.last_redraws = redraws;
@@ -3863,14 +3998,13 @@ int pmc_coag_gpu_destroy(pmc_coag_gpu_ctx* x) {
   c.graph_stats.release();
   c.sample_buf.release();
   c.pp_rm_n.release();
-  for (auto* b : {&c.grp_hist, &c.item_pop, &c.g_pop, &c.g_pair, &c.g_slot, &c.g_k}) b->release();
+  for (auto* b : {&c.grp_hist, &c.item_pop, &c.ppw_slot, &c.ppw_gp}) b->release();
   c.grp_off.release();
   c.grp_dest.release();
   c.wk_slot.release();
   c.wk_gp.release();
   c.wk_flag.release();
   c.wk_off.release();
-  c.g_key.release();
   c.pp_rm_pool.release();
   c.pp_rm_off.release();
   c.pp_rm_tot.release();
