@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -99,6 +100,7 @@ template <class T>
 __global__ void __launch_bounds__(kScanThreads) k_scan_lb(ScanJobs jobs, unsigned long long* status,
                                                           int status_stride, unsigned* tile_ctr,
                                                           unsigned* done_ctr, unsigned long long* err) {
+  chain_wait();
   const ScanJob J = jobs.j[blockIdx.y];
   __shared__ unsigned tile_sh;
   __shared__ long long carry_sh;
@@ -335,6 +337,7 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact_samples(CompactArgs
                                                                      const int* gpair_pop, const int* gpair_local,
                                                                      const int2* ev, const int* ev_gp,
                                                                      const long long* work_off) {
+  chain_wait();
   __shared__ int sh_idx[kCompactTile];
   int count;
   const long long e0 = compact_tile(A, sh_idx, &count);
@@ -375,6 +378,7 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact_items(CompactArgs A
                                                                    const uint32_t* it_dec, const int4* it_term,
                                                                    int* ev_head, uint8_t* ev_done,
                                                                    const long long* grouped) {
+  chain_wait();
   __shared__ int sh_idx[kCompactTile];
   int count;
   const long long e0 = compact_tile(A, sh_idx, &count);
@@ -394,11 +398,11 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact_items(CompactArgs A
   last_block(A.ctl);
 }
 
-// target operations of round 0, in the reference's backwards target order
-// (coagulation.F90:220-237)
+// target operations of round 0 (the first cap of them), in the reference's
+// backwards target order (coagulation.F90:220-237)
 __global__ void k_build_ops(const PopDev* pops, const int* gpair_pop, const int* gpair_local,
-                            const long long* pp_off, int n_gpairs, int* op_pop, int* op_pair, int* op_slot,
-                            int* op_k, unsigned long long* op_key) {
+                            const long long* pp_off, int n_gpairs, long long cap, int* op_pop, int* op_pair,
+                            int* op_slot, int* op_k, unsigned long long* op_key) {
   int gp = blockIdx.x;
   if (gp >= n_gpairs) return;
   long long n = pp_off[gp + 1] - pp_off[gp];
@@ -411,6 +415,7 @@ __global__ void k_build_ops(const PopDev* pops, const int* gpair_pop, const int*
   int start = P.cell_start[tcell];
   for (long long k = threadIdx.x; k < n; k += blockDim.x) {
     long long q = pp_off[gp] + k;
+    if (q >= cap) break;  // more than a step graph has room for: k_step_check stops it
     op_pop[q] = pop;
     op_pair[q] = p;
     op_slot[q] = P.list[start + (int)(n - 1 - k)];
@@ -576,6 +581,7 @@ __device__ __forceinline__ int resolve_event(const ResolveArgs& A, long long e, 
 }
 
 __global__ void __launch_bounds__(256) k_resolve(ResolveArgs A) {
+  chain_wait();
   __shared__ unsigned long long excl_sh;
   const long long E = A.n_events ? *A.n_events : 0;
   const int tb = blockDim.x;  // events of a tile
@@ -612,6 +618,7 @@ __global__ void __launch_bounds__(256) k_resolve(ResolveArgs A) {
 // need[q] of target operation q summed per population (op_pop[q])
 __global__ void k_count_per_pop(const int* need, const long long* n_items, const int* item_pop_of,
                                 int* per_pop) {
+  chain_wait();
   long long n = *n_items;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
        e += (long long)gridDim.x * blockDim.x) {
@@ -1089,7 +1096,7 @@ struct MappedBuf {
   void reserve(size_t b) {
     if (b <= bytes) return;
     release();
-    size_t want = std::max<size_t>(b + b / 4, 1 << 20);
+    size_t want = b + b / 4;
     if (cudaHostAlloc(&p, want, cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(&dev, p, 0) != cudaSuccess) {
       cudaGetLastError();
@@ -1259,7 +1266,9 @@ struct Ctx {
   uint32_t claim_gen = 0;
   bool dirty = true;            // host PopDev copies changed since the last push
   std::vector<PopCtr> h_ctrs;
-  std::vector<unsigned char> stat_buf;  // the step graph's report and counters
+  MappedBuf report;                // the step graph's report and counters, then its sequence number
+  DevBuf<unsigned> report_seq;
+  unsigned report_count = 0;
   cudaStream_t stream = nullptr;
   int max_rounds = 200;  // below 256: the round is 8 bits of the random streams' counters
   int n_sm = 148;        // multiprocessors of the device
@@ -1271,6 +1280,7 @@ struct Ctx {
   cudaStream_t side_stream = nullptr;  // a branch of a captured step
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   bool fork = false;                   // capturing: independent launches go to branches
+  bool chained = false;                // capturing a step: launch_chained
   cudaGraph_t rg_graph = nullptr;
   cudaGraphExec_t rg_exec = nullptr;
   std::vector<long long> rg_key;
@@ -1470,6 +1480,27 @@ T* dalloc(Ctx& c, std::vector<void*>& owner, size_t n) {
   return (T*)p;
 }
 
+// Launch k on st.  In a captured step (c.chained) it starts while the kernel
+// before it in the stream ends (programmatic dependent launch): every kernel
+// launched this way begins with chain_wait(), which waits for that kernel and
+// its writes, so only the launch itself overlaps, 1 to 1.5 us of a step's 20
+// to 25 kernels that mostly run 3 to 10 us.
+template <class... KA, class... A>
+void launch_chained(Ctx& c, void (*k)(KA...), dim3 g, dim3 b, size_t smem, cudaStream_t st, A... a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = g;
+  cfg.blockDim = b;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = c.chained ? 1 : 0;
+  CK(cudaLaunchKernelEx(&cfg, k, KA(a)...));
+  note_launch();
+}
+
 int grid_for(long long n, int threads) {
   long long b = (n + threads - 1) / threads;
   if (b < 1) b = 1;
@@ -1579,9 +1610,8 @@ void scan_multi(Ctx& c, std::initializer_list<ScanArg<T>> args, cudaStream_t st 
     c.scan_status_n = c.scan_status.n;
   }
   dim3 g((unsigned)nb, (unsigned)k);
-  k_scan_lb<T><<<g, kScanThreads, 0, st>>>(jobs, c.scan_status.p, (int)nb, c.scan_ctr.p, c.scan_ctr.p + kScanMaxJobs,
-                                           c.scan_err.p);
-  note_launch();
+  launch_chained(c, k_scan_lb<T>, g, dim3(kScanThreads), 0, st, jobs, c.scan_status.p, (int)nb, c.scan_ctr.p,
+                 c.scan_ctr.p + kScanMaxJobs, c.scan_err.p);
 }
 
 // shared words of a tiled launch of at most `tiles` blocks
@@ -2181,13 +2211,12 @@ void launch_test_kt(Ctx& c, int kt, bool flat, int n_gpairs, long long W, cudaSt
     constexpr int KT = decltype(ktc)::value;
     using T = decltype(tt);
     if (flat)
-      k_test<KT, T, true><<<blocks, tb, 0, st>>>(c.d_pops, c.gpair_pop.p, c.gpair_local.p, c.work_off.p, n_gpairs,
+      launch_chained(c, k_test<KT, T, true>, dim3(blocks), dim3(tb), 0, st, c.d_pops, c.gpair_pop.p, c.gpair_local.p, c.work_off.p, n_gpairs,
                                                  c.work_off.p + n_gpairs, c.flag.p, c.ev.p, c.ev_gp.p);
     else
-      k_test<KT, T, false><<<blocks, tb, 0, st>>>(c.d_pops, c.gpair_pop.p, c.gpair_local.p, c.work_off.p, n_gpairs,
+      launch_chained(c, k_test<KT, T, false>, dim3(blocks), dim3(tb), 0, st, c.d_pops, c.gpair_pop.p, c.gpair_local.p, c.work_off.p, n_gpairs,
                                                   c.work_off.p + n_gpairs, c.flag.p, c.ev.p, c.ev_gp.p);
   });
-  note_launch();
 }
 
 ChainPool chain_pool(Ctx& c) {
@@ -2255,20 +2284,20 @@ void launch_items_kt(Ctx& c, int kt, bool flat, int n_gpairs, long long W, cudaS
     auto k = flat ? k_items<KT, T, true> : k_items<KT, T, false>;
     {
       TuneScope ts_items(c, kTuneItems, st);
-      k<<<grid_warps(c, W, ti), ti, 0, st>>>(A);
+      launch_chained(c, k, dim3(grid_warps(c, W, ti)), dim3(ti), 0, st, A);
     }
     auto kc = flat ? k_chain<KT, T, true> : k_chain<KT, T, false>;
     {
       TuneScope ts_chain(c, kTuneChain, st);
-      kc<<<grid_warps(c, W, tc), tc, 0, st>>>(A, pool);
+      launch_chained(c, kc, dim3(grid_warps(c, W, tc)), dim3(tc), 0, st, A, pool);
     }
   });
-  note_launch();
-  note_launch();
 }
 
 // the round's staged target operations: the redone ones, then one place per item
-__global__ void k_ops_span(long long* n_ops, const long long* n_items) { n_ops[0] += *n_items; }
+__global__ void k_ops_span(long long* n_ops, const long long* n_items) {
+  chain_wait();
+  n_ops[0] += *n_items; }
 
 // Stable grouping by population of a batched context's per-round lists.
 // Slot and ID ranks come from one scan over a list, and the per-population
@@ -2299,6 +2328,7 @@ __global__ void __launch_bounds__(kGrpTile) k_grp_hist(const long long* n, const
 
 __global__ void __launch_bounds__(kGrpTile) k_grp_rank(const long long* n, const int* pop_of, int n_tiles,
                                                        const long long* off, long long* dest) {
+  chain_wait();
   __shared__ int wpop[kGrpTile / 32][32], wcnt[kGrpTile / 32][32];
   const long long N = *n;
   const long long i = blockIdx.x * (long long)kGrpTile + threadIdx.x;
@@ -2330,6 +2360,7 @@ __global__ void __launch_bounds__(kGrpTile) k_grp_rank(const long long* n, const
 __global__ void k_scatter_ops(const long long* n_ops, const long long* dest, const int* pop, const int* pair,
                               const int* slot, const int* k, const unsigned long long* key, int* pop_o, int* pair_o,
                               int* slot_o, int* k_o, unsigned long long* key_o) {
+  chain_wait();
   const long long Q = *n_ops;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < Q; q += (long long)gridDim.x * blockDim.x) {
     const long long d = dest[q];
@@ -2346,6 +2377,7 @@ __global__ void k_scatter_ops(const long long* n_ops, const long long* dest, con
 // made no event)
 __global__ void k_item_pops(const long long* n_items, const uint8_t* it_flag, const int* it_gp, const int* gpair_pop,
                             int n_gpairs, int* pop_of) {
+  chain_wait();
   const long long n = *n_items;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int gp = it_gp[i];
@@ -2365,8 +2397,7 @@ void group_by_pop(Ctx& c, const long long* n, long long bound, const int* pop_of
   k_grp_hist<<<n_tiles, kGrpTile, 0, st>>>(n, pop_of, c.n_pop, n_tiles, c.grp_hist.p, c.d_ctrs);
   note_launch();
   scan_multi<int>(c, {ScanArg<int>{c.grp_hist.p, nh, nullptr, c.grp_off.p, kept}}, st);
-  k_grp_rank<<<n_tiles, kGrpTile, 0, st>>>(n, pop_of, n_tiles, c.grp_off.p, dest);
-  note_launch();
+  launch_chained(c, k_grp_rank, dim3(n_tiles), dim3(kGrpTile), 0, st, n, pop_of, n_tiles, c.grp_off.p, dest);
 }
 
 // Buffers of a round's at most Q target operations that carry nothing from
@@ -2401,18 +2432,16 @@ void reserve_redo(Ctx& c, long long Q) {
 // empty places; n_dev[1] counts the operations kept.
 void launch_pp_group(Ctx& c, long long Q, cudaStream_t st) {
   group_by_pop(c, c.n_dev.p, Q, c.r_pop.p, c.grp_dest.p, st, c.n_dev.p + 1);
-  k_scatter_ops<<<grid_for(Q, 256), 256, 0, st>>>(c.n_dev.p, c.grp_dest.p, c.r_pop.p, c.r_pair.p, c.r_slot.p,
+  launch_chained(c, k_scatter_ops, dim3(grid_for(Q, 256)), dim3(256), 0, st, c.n_dev.p, c.grp_dest.p, c.r_pop.p, c.r_pair.p, c.r_slot.p,
                                                   c.r_k.p, c.r_key.p, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p,
                                                   c.op_key.p);
-  note_launch();
 }
 
 // the bound on each target operation's removals, scanned into its place in
 // the removal pool (their total in pp_rm_tot); n_ops: their count
 void launch_pp_count(Ctx& c, long long Q, const long long* n_ops, cudaStream_t st) {
-  k_pp_count<<<grid_for(Q, 128), 128, 0, st>>>(c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p, n_ops,
-                                               c.pp_rm_n.p);
-  note_launch();
+  launch_chained(c, k_pp_count, dim3(grid_for(Q, 128)), dim3(128), 0, st, c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p,
+                 c.op_k.p, n_ops, Q, c.pp_rm_n.p);
   scan_multi<int>(c, {ScanArg<int>{c.pp_rm_n.p, Q, n_ops, c.pp_rm_off.p, c.pp_rm_tot.p}}, st);
 }
 
@@ -2439,11 +2468,9 @@ void fit_rm_pool(Ctx& c) {
 void launch_pp_ops(Ctx& c, int kt, long long Q, cudaStream_t st) {
   with_kt(c, kt, [&](auto ktc, auto) {
     constexpr int KT = decltype(ktc)::value;
-    k_pp_ops<KT><<<grid_for(32 * Q, 32 * kPPWarps), 32 * kPPWarps, 0, st>>>(
-        c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p, c.op_key.p, c.n_dev.p + 1, c.pp_res.p, c.pp_vol.p,
+    launch_chained(c, k_pp_ops<KT>, dim3(grid_for(32 * Q, 32 * kPPWarps)), dim3(32 * kPPWarps), 0, st, c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p, c.op_key.p, c.n_dev.p + 1, c.pp_res.p, c.pp_vol.p,
         c.pp_rm_off.p, c.pp_rm_pool.p, (long long)c.pp_rm_pool.n);
   });
-  note_launch();
 }
 
 // One mc_coag call in replay mode: the grid decision of
@@ -2734,6 +2761,7 @@ __global__ void k_step_begin(PopDev* pops, PopCtr* ctrs, int n_pop, uint32_t* d_
 __global__ void k_step_check(const PopDev* pops, int n_pop, const long long* pop_pair_base, long long* work_off,
                              long long* pp_off, int n_gp, long long w_cap, long long q_cap, const long long* rm_tot,
                              long long pool, long long sort_slots, long long* n_dev, long long* stat) {
+  chain_wait();
   const long long W = work_off[n_gp], Q = pp_off[n_gp];
   long long why = 0;
   if (Q > q_cap) why |= kNoGoOps;
@@ -2766,6 +2794,18 @@ __global__ void k_step_check(const PopDev* pops, int n_pop, const long long* pop
   if (all) work_off[n_gp] = pp_off[n_gp] = 0;
 }
 
+// The step graph's last launch: its report and the counter blocks (n16 words of
+// 16 bytes from stat on) into page-locked host memory, then the step's sequence
+// number, which the host waits for.  A copy and a stream synchronisation in its
+// place took 12 us of a step longer (0.131 to 0.119 ms at 1e4 particles).
+__global__ void __launch_bounds__(1024) k_step_report(const uint4* stat, int n16, uint4* out, volatile unsigned* flag,
+                                                      unsigned* seq) {
+  for (int k = threadIdx.x; k < n16; k += blockDim.x) out[k] = stat[k];
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) *flag = ++*seq;
+}
+
 // Resolve and apply the events of a round (E at round_dev[1], at most W) and,
 // with Q > 0 (host loop only), its Q target operations.  chains: the round may
 // have chains (every round but the first).
@@ -2775,17 +2815,14 @@ void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q, bool chain
   // Q bounds the round's target operations; their count is n_dev[1] (the
   // redone ones, then those that walks appended)
   if (Q > 0) {
-    k_pp_resolve<<<grid_for(Q, 256), 256, 0, st>>>(c.d_pops, c.op_pop.p, c.op_key.p, c.n_dev.p + 1, c.pp_res.p,
+    launch_chained(c, k_pp_resolve, dim3(grid_for(Q, 256)), dim3(256), 0, st, c.d_pops, c.op_pop.p, c.op_key.p, c.n_dev.p + 1, c.pp_res.p,
                                                    c.pp_rm_pool.p, c.win_pp.p, c.need_slot_pp.p, c.need_id_pp.p, c.lost_pp.p);
-    note_launch();
     scan_multi<int>(c, {{c.need_slot_pp.p, Q, c.n_dev.p + 1, c.rank_slot_pp.p}, {c.need_id_pp.p, Q, c.n_dev.p + 1, c.rank_id_pp.p}},
                     st);
-    k_count_per_pop<<<grid_for(Q, 256), 256, 0, st>>>(c.need_slot_pp.p, c.n_dev.p + 1, c.op_pop.p,
+    launch_chained(c, k_count_per_pop, dim3(grid_for(Q, 256)), dim3(256), 0, st, c.need_slot_pp.p, c.n_dev.p + 1, c.op_pop.p,
                                                       c.per_pop_i.p + 2 * c.n_pop);
-    note_launch();
-    k_count_per_pop<<<grid_for(Q, 256), 256, 0, st>>>(c.need_id_pp.p, c.n_dev.p + 1, c.op_pop.p,
+    launch_chained(c, k_count_per_pop, dim3(grid_for(Q, 256)), dim3(256), 0, st, c.need_id_pp.p, c.n_dev.p + 1, c.op_pop.p,
                                                       c.per_pop_i.p + 3 * c.n_pop);
-    note_launch();
   }
   {
     TuneScope ts(c, kTuneResolve, st);
@@ -2816,8 +2853,7 @@ void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q, bool chain
     A.pp_slot_base = c.slot_base_pp.p;
     A.set_id_base = c.id_base_set.p;
     A.pp_id_base = c.id_base_pp.p;
-    k_resolve<<<(unsigned)tiles, tr, 0, st>>>(A);
-    note_launch();
+    launch_chained(c, k_resolve, dim3((unsigned)tiles), dim3(tr), 0, st, A);
   }
   if (W > 0) {
     const int ta = c.tune.threads[kTuneApply];
@@ -2838,11 +2874,10 @@ void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q, bool chain
     }
     {
       TuneScope ts(c, kTuneApply, st);
-      k_apply<<<grid_for(W, ta), ta, 0, st>>>(c.d_pops, c.gpair_pop.p, Ed, c.win_set.p, c.rank_slot_set.p,
+      launch_chained(c, k_apply, dim3(grid_for(W, ta)), dim3(ta), 0, st, c.d_pops, c.gpair_pop.p, Ed, c.win_set.p, c.rank_slot_set.p,
                                               c.rank_id_set.p, c.slot_base_set.p, c.id_base_set.p, c.ev_done.p,
                                               c.ev_dest.p, c.ev_key.p, c.ev_c.p, c.gp_c.p, c.ev_pos.p, c.dec_set.p,
                                               c.ev_term.p, c.pop_pair_base.p);
-      note_launch();
     }
     if (chains && c.fork) {
       CK(cudaEventRecord(c.ev_join, c.side_stream));
@@ -2851,18 +2886,15 @@ void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q, bool chain
   }
   if (Q > 0) {
     const size_t nw = (size_t)Q * kMaxCopies;
-    k_pp_apply<<<grid_for(Q, 256), 256, 0, st>>>(c.d_pops, c.op_pop.p, c.n_dev.p + 1, c.pp_res.p, c.pp_vol.p,
+    launch_chained(c, k_pp_apply, dim3(grid_for(Q, 256)), dim3(256), 0, st, c.d_pops, c.op_pop.p, c.n_dev.p + 1, c.pp_res.p, c.pp_vol.p,
                                                  c.pp_rm_pool.p, c.win_pp.p, c.rank_slot_pp.p, c.rank_id_pp.p,
                                                  c.slot_base_pp.p, c.id_base_pp.p, c.pop_pair_base.p, c.op_k.p,
                                                  c.wk_slot.p, c.wk_gp.p, c.wk_flag.p);
-    note_launch();
-    k_walkers_span<<<1, 1, 0, st>>>(c.n_dev.p + 1, c.round_dev.p + 9);
-    note_launch();
+    launch_chained(c, k_walkers_span, dim3(1), dim3(1), 0, st, c.n_dev.p + 1, c.round_dev.p + 9);
     scan_multi<uint8_t>(c, {ScanArg<uint8_t>{c.wk_flag.p, (long long)nw, c.round_dev.p + 9, c.wk_off.p,
                                              c.round_dev.p + 5}}, st);
-    k_compact_walkers<<<grid_for((long long)nw, 256), 256, 0, st>>>(c.round_dev.p + 9, c.wk_flag.p, c.wk_off.p,
+    launch_chained(c, k_compact_walkers, dim3(grid_for((long long)nw, 256)), dim3(256), 0, st, c.round_dev.p + 9, c.wk_flag.p, c.wk_off.p,
                                                                     c.wk_slot.p, c.wk_gp.p, c.ppw_slot.p, c.ppw_gp.p);
-    note_launch();
     scan_multi<int>(c, {ScanArg<int>{c.lost_pp.p, Q, c.n_dev.p + 1, c.lost_off.p, c.round_dev.p + 8}}, st);
   }
 }
@@ -2887,10 +2919,9 @@ CompactArgs compact_args(Ctx& c, const uint8_t* flag, const long long* n, long l
 
 // round 0's events from the tests' flags (their count *n on the device, at most W)
 void launch_compact_samples(Ctx& c, const long long* n, long long W, cudaStream_t st) {
-  k_compact_samples<<<(unsigned)compact_tiles(W), kCompactThreads, 0, st>>>(
+  launch_chained(c, k_compact_samples, dim3((unsigned)compact_tiles(W)), dim3(kCompactThreads), 0, st, 
       compact_args(c, c.flag.p, n, W, st), c.d_pops, c.gpair_pop.p, c.gpair_local.p, c.ev.p, c.ev_gp.p,
       c.work_off.p);
-  note_launch();
 }
 
 // a buffer's growth that keeps what it holds
@@ -2905,10 +2936,10 @@ void grow_keeping(Ctx& c, DevBuf<T>& b, size_t m) {
   nb.release();
 }
 
-// round 0's target operations
-void launch_build_ops(Ctx& c, int n_gpairs, cudaStream_t st) {
-  k_build_ops<<<n_gpairs, 128, 0, st>>>(c.d_pops, c.gpair_pop.p, c.gpair_local.p, c.pp_off.p, n_gpairs, c.op_pop.p,
-                                        c.op_pair.p, c.op_slot.p, c.op_k.p, c.op_key.p);
+// round 0's target operations, at most cap
+void launch_build_ops(Ctx& c, int n_gpairs, long long cap, cudaStream_t st) {
+  k_build_ops<<<n_gpairs, 128, 0, st>>>(c.d_pops, c.gpair_pop.p, c.gpair_local.p, c.pp_off.p, n_gpairs, cap,
+                                        c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p, c.op_key.p);
   note_launch();
 }
 
@@ -2932,13 +2963,11 @@ void enqueue_round_head(Ctx& c, cudaStream_t st, const RoundBounds& b, long long
   launch_sort(c, st, b.max_chunks, b.max_cells);
   {
     dim3 g(b.max_cells, c.n_pop);
-    k_walk_rates<<<g, 128, 0, st>>>(c.d_pops);
-    note_launch();
+    launch_chained(c, k_walk_rates, dim3(g), dim3(128), 0, st, c.d_pops);
   }
   launch_items_kt(c, b.kt, b.flat, b.n_gpairs, b.W, st);
   if (Q > 0) {
-    k_ops_span<<<1, 1, 0, st>>>(c.n_dev.p, c.round_dev.p + 2);
-    note_launch();
+    launch_chained(c, k_ops_span, dim3(1), dim3(1), 0, st, c.n_dev.p, c.round_dev.p + 2);
     launch_pp_group(c, Q, st);
     launch_pp_count(c, Q, c.n_dev.p + 1, st);
   }
@@ -2955,16 +2984,14 @@ void enqueue_round_tail(Ctx& c, cudaStream_t st, const RoundBounds& b, long long
   if (Q > 0 && c.n_pop > 1) {
     c.item_pop.reserve((size_t)W + 1);
     c.grp_dest.reserve((size_t)W + 1);
-    k_item_pops<<<grid_for(W, 256), 256, 0, st>>>(Id, c.it_flag.p, c.it_gp.p, c.gpair_pop.p, b.n_gpairs,
+    launch_chained(c, k_item_pops, dim3(grid_for(W, 256)), dim3(256), 0, st, Id, c.it_flag.p, c.it_gp.p, c.gpair_pop.p, b.n_gpairs,
                                                   c.item_pop.p);
-    note_launch();
     group_by_pop(c, Id, W, c.item_pop.p, c.grp_dest.p, st);
     grouped = c.grp_dest.p;
   }
-  k_compact_items<<<(unsigned)compact_tiles(W), kCompactThreads, 0, st>>>(
+  launch_chained(c, k_compact_items, dim3((unsigned)compact_tiles(W)), dim3(kCompactThreads), 0, st, 
       compact_args(c, c.it_flag.p, Id, W, st), c.it_key.p, c.it_c.p, c.it_gp.p, c.it_pos.p, c.it_len.p, c.it_head.p,
       c.it_done.p, c.it_dec.p, c.it_term.p, c.ev_head.p, c.ev_done.p, grouped);
-  note_launch();
   resolve_apply(c, st, W, Q, true);
 }
 
@@ -3218,6 +3245,11 @@ void free_step_graph(Ctx& c) {
 }
 
 // what the step graph's captured launches depend on, beyond round_graph_key
+// 16-byte words of the step graph's report
+int report_words(const Ctx& c) {
+  return (int)((sizeof(long long) * kStatWords + sizeof(PopCtr) * c.n_pop + 15) / 16);
+}
+
 std::vector<long long> step_graph_key(const Ctx& c, const RoundBounds& b, long long w_cap, int max_pairs,
                                       long long q_cap, long long qb_cap) {
   std::vector<long long> k = round_graph_key(c, b);
@@ -3232,7 +3264,7 @@ std::vector<long long> step_graph_key(const Ctx& c, const RoundBounds& b, long l
           (long long)c.grp_dest.p, (long long)c.grp_hist.p, (long long)c.grp_off.p, (long long)c.item_pop.p,
           (long long)c.wk_slot.p, (long long)c.wk_gp.p, (long long)c.wk_flag.p, (long long)c.wk_off.p})
       k.push_back(v);
-  for (long long v : {(long long)c.n_dev.p, w_cap, (long long)max_pairs, (long long)c.prof, (long long)c.tune.threads[kTuneTest],
+  for (long long v : {(long long)c.report.dev, (long long)c.report_seq.p, (long long)c.n_dev.p, w_cap, (long long)max_pairs, (long long)c.prof, (long long)c.tune.threads[kTuneTest],
                       (long long)c.nwork_set.p, (long long)c.nwork_pp.p, (long long)c.work_off.p,
                       (long long)c.pp_off.p, (long long)c.flag.p, (long long)c.ev.p, (long long)c.ev_gp.p,
                       (long long)c.d_stat})
@@ -3253,6 +3285,7 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
     if (c.prof) CK(cudaEventRecordWithFlags(c.sg_ev[k], st, cudaEventRecordExternal));
   };
   const long long n0 = g_launches;
+  c.chained = true;
   CK(cudaStreamBeginCaptureToGraph(st, c.sg_graph, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
   cudaGraph_t done = nullptr;
   try {
@@ -3263,18 +3296,16 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
     mark(0);
     launch_sort(c, st, b.max_chunks, b.max_cells);
     mark(1);
-    k_pairs<<<dim3((max_pairs + 127) / 128, c.n_pop), 128, 0, st>>>(c.d_pops, c.pop_pair_base.p, c.nwork_set.p,
+    launch_chained(c, k_pairs, dim3(dim3((max_pairs + 127) / 128, c.n_pop)), dim3(128), 0, st, c.d_pops, c.pop_pair_base.p, c.nwork_set.p,
                                                                    c.nwork_pp.p, 1);
-    note_launch();
     scan_multi<long long>(c, {{c.nwork_set.p, n_gp, nullptr, c.work_off.p}, {c.nwork_pp.p, n_gp, nullptr, c.pp_off.p}},
                           st);
     if (q_cap > 0) {
-      launch_build_ops(c, n_gp, st);
+      launch_build_ops(c, n_gp, q_cap, st);
       launch_pp_count(c, q_cap, c.pp_off.p + n_gp, st);
     }
-    k_step_check<<<1, 256, 0, st>>>(c.d_pops, c.n_pop, c.pop_pair_base.p, c.work_off.p, c.pp_off.p, n_gp, w_cap, q_cap,
+    launch_chained(c, k_step_check, dim3(1), dim3(256), 0, st, c.d_pops, c.n_pop, c.pop_pair_base.p, c.work_off.p, c.pp_off.p, n_gp, w_cap, q_cap,
                                     c.pp_rm_tot.p, (long long)c.pp_rm_pool.n, sort_slots, c.n_dev.p, c.d_stat);
-    note_launch();
     if (q_cap > 0) launch_pp_ops(c, b.kt, q_cap, st);
     mark(2);
     launch_test_kt(c, b.kt, b.flat, n_gp, w_cap, st);
@@ -3309,6 +3340,9 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
     };
     cudaGraph_t body = add_conditional(cond, cudaGraphCondTypeWhile);
     mark(5);
+    k_step_report<<<1, 1024, 0, st>>>((const uint4*)c.d_stat, report_words(c), (uint4*)c.report.dev,
+                                      (unsigned*)((char*)c.report.dev + 16 * (size_t)report_words(c)), c.report_seq.p);
+    note_launch();
     CK(cudaStreamEndCapture(st, &done));
     const long long n1 = g_launches;
     CK(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
@@ -3334,13 +3368,14 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
     note_launch();
     c.sg_nodes = g_launches - n1;
   } catch (...) {
-    c.fork = false;
+    c.fork = c.chained = false;
     cudaStreamEndCapture(st, &done);
     cudaGetLastError();
     g_launches = n0;
     free_step_graph(c);
     throw;
   }
+  c.chained = false;
   CK(cudaStreamEndCapture(st, &done));
   g_launches = n0;  // counted when they run
   CK(cudaGraphInstantiate(&c.sg_exec, c.sg_graph, 0));
@@ -3391,9 +3426,10 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   if (e > c.sg_e || 16 * e <= c.sg_e) c.sg_e = e;
   long long q_cap = 0, qb_cap = 0;
   if (c.pp_step) {
+    // room for twice as many when they outgrow it
     const long long q = graph_bound(c.last_q + c.last_q / 4), qb = graph_bound(c.last_qb + c.last_qb / 4);
-    if (q > c.sg_q || 16 * q <= c.sg_q) c.sg_q = q;
-    if (qb > c.sg_qb || 16 * qb <= c.sg_qb) c.sg_qb = qb;
+    if (q > c.sg_q || 16 * q <= c.sg_q) c.sg_q = 2 * q;
+    if (qb > c.sg_qb || 16 * qb <= c.sg_qb) c.sg_qb = 2 * qb;
     q_cap = c.sg_q;
     qb_cap = c.sg_qb;
   }
@@ -3416,6 +3452,12 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   reserve_events(c, std::max(c.sg_w + kMaxCopies * q_cap, b.W));
   reserve_round(c, b.W);
   c.pp_rm_tot.reserve(1);
+  if (!c.report.p) {
+    c.report.reserve(16 * (size_t)report_words(c) + 64);
+    memset(c.report.p, 0, c.report.bytes);
+    c.report_seq.reserve(1);
+    CK(cudaMemsetAsync(c.report_seq.p, 0, sizeof(unsigned) * c.report_seq.n, c.stream));
+  }
   if (q_cap > 0) {
     const long long q = std::max(q_cap, qb_cap);
     reserve_ops(c, q);
@@ -3448,7 +3490,9 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
       if (!ev) CK(cudaEventCreate(&ev));
   const std::vector<long long> key = step_graph_key(c, b, c.sg_w, max_pairs, q_cap, qb_cap);
   if (key != c.sg_key) {
-    if (key != c.sg_seen) {  // captured when the bounds and addresses hold for two steps
+    // captured when the bounds and addresses hold for two steps; at once where
+    // a step the long way costs several captures (about 1 ms each)
+    if (key != c.sg_seen && !c.pp_step) {
       c.sg_seen = key;
       return out;
     }
@@ -3463,11 +3507,23 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
     for (auto& ph : c.pops) ph.h.step += 1u;
   }
   CK(cudaGraphLaunch(c.sg_exec, c.stream));
-  c.stat_buf.resize(sizeof(long long) * kStatWords + sizeof(PopCtr) * c.n_pop);
-  CK(cudaMemcpyAsync(c.stat_buf.data(), c.d_stat, c.stat_buf.size(), cudaMemcpyDeviceToHost, c.stream));
-  CK(cudaStreamSynchronize(c.stream));
+  c.report_count++;
+  {
+    // the report's sequence number; a look at the stream now and then, for an
+    // error or a graph that ended without it
+    const volatile unsigned* flag = (const volatile unsigned*)((const char*)c.report.p + 16 * (size_t)report_words(c));
+    for (long long spins = 1; *flag != c.report_count; spins++) {
+      if (spins % 4096 != 0) continue;
+      const cudaError_t e = cudaStreamQuery(c.stream);
+      if (e == cudaErrorNotReady) continue;
+      CK(e);
+      if (*flag != c.report_count) throw Fail(PMC_ERR_CUDA);
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+  }
+  const unsigned char* report = (const unsigned char*)c.report.p;
   long long stat[kStatWords];
-  memcpy(stat, c.stat_buf.data(), sizeof(stat));
+  memcpy(stat, report, sizeof(stat));
   c.last_w = stat[5];
   c.last_q = stat[12];
   c.last_rm = std::max(c.last_rm, stat[11]);
@@ -3479,7 +3535,7 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
     CK(cudaMemsetAsync(c.scan_err.p, 0, sizeof(unsigned long long), c.stream));
     throw Fail(PMC_ERR_TIMEOUT);
   }
-  memcpy(c.h_ctrs.data(), c.stat_buf.data() + sizeof(stat), sizeof(PopCtr) * c.n_pop);
+  memcpy(c.h_ctrs.data(), report + sizeof(stat), sizeof(PopCtr) * c.n_pop);
   for (int k = 0; k < c.n_pop; k++) c.n_slots_host[k] = c.h_ctrs[k].n_slots;
   if (c.prof) {
     const long long units[3] = {slots * c.n_pop, stat[5], 1};
@@ -3602,8 +3658,7 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
   }
   {
     dim3 gp((max_pairs + 127) / 128, c.n_pop);
-    k_pairs<<<gp, 128, 0, c.stream>>>(c.d_pops, c.pop_pair_base.p, c.nwork_set.p, c.nwork_pp.p, 1);
-    note_launch();
+    launch_chained(c, k_pairs, dim3(gp), dim3(128), 0, c.stream, c.d_pops, c.pop_pair_base.p, c.nwork_set.p, c.nwork_pp.p, 1);
   }
   // the device copies learn this with the next push
   for (int k = 0; k < c.n_pop; k++) {
@@ -3682,7 +3737,7 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
   }
   if (Q > 0) {
     reserve_ops(c, Q);
-    launch_build_ops(c, n_gpairs, c.stream);
+    launch_build_ops(c, n_gpairs, Q, c.stream);
     CK(cudaMemcpyAsync(c.n_dev.p + 1, &Q, sizeof(long long), cudaMemcpyHostToDevice, c.stream));
     launch_pp_count(c, Q, c.n_dev.p + 1, c.stream);  // built in population order
     fit_rm_pool(c);
@@ -3898,7 +3953,7 @@ static int do_init(int n_pop, int n_spec, const double* density, int i_water, in
   }
   c.pops.resize(n_pop);
   CK(cudaMalloc(&c.d_pops, sizeof(PopDev) * n_pop));
-  CK(cudaMalloc(&c.d_stat, sizeof(long long) * kStatWords + sizeof(PopCtr) * n_pop));
+  CK(cudaMalloc(&c.d_stat, sizeof(long long) * kStatWords + sizeof(PopCtr) * n_pop + 16));  // read in 16-byte words
   c.d_ctrs = (PopCtr*)(c.d_stat + kStatWords);
   CK(cudaMalloc(&c.d_round, 2 * sizeof(uint32_t)));  // round of the step, claim generation
   CK(cudaMemset(c.d_round, 0, 2 * sizeof(uint32_t)));
@@ -3970,6 +4025,8 @@ int pmc_coag_gpu_destroy(pmc_coag_gpu_ctx* x) {
   c.flag.release();
   c.win_set.release();
   c.pop_on.release();
+  c.report.release();
+  c.report_seq.release();
   c.dec_set.release();
   c.ev_gp.release();
   c.gp_c.release();

@@ -147,6 +147,14 @@ __device__ int block_excl_scan(int v, int* total) {
   return pre;
 }
 
+// First thing in a kernel that launch_chained launches: waits until the kernel
+// before it in the stream has ended and its writes are visible, then lets the
+// one after it be launched.  Does nothing in an ordinary launch.
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // pair-test record of a particle of radius r (vol2rad(v)), total volume v,
 // mass m and class cls (1-based) (see RecD).  A sphere's mobility radius is r:
 // taking it saves two of the record's three FP64 pow calls, each about half a
@@ -582,6 +590,7 @@ __global__ void k_pair_setup(const PopDev* pops) {
 // walks test particles that arrive in a pair's cells during the step.
 __global__ void k_pairs(const PopDev* pops, const long long* pop_pair_base, long long* nwork_set,
                         long long* nwork_pp, int use_particle_path) {
+  chain_wait();
   const PopDev& P = pops[blockIdx.y];
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= P.n_pairs) return;
@@ -840,6 +849,7 @@ __global__ void __launch_bounds__(256) k_test(const PopDev* pops, const int* gpa
                                               const int* gpair_local, const long long* work_off,
                                               int n_gpairs, const long long* total, uint8_t* flag,
                                               int2* ev, int* ev_gp) {
+  chain_wait();
   long long W = *total;
   for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < W;
        w += (long long)gridDim.x * blockDim.x) {

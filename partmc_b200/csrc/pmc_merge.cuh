@@ -215,6 +215,7 @@ __global__ void __launch_bounds__(256) k_apply(const PopDev* pops, const int* gp
                                                const long long* id_base, const uint8_t* ev_done, int* dest_out,
                                                unsigned long long* ev_key, int2* ev, int* ev_gp, float* ev_pos,
                                                uint32_t* dec, const int4* ev_term, const long long* pop_pair_base) {
+  chain_wait();
   long long E = *n_events;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < E;
        e += (long long)gridDim.x * blockDim.x) {
@@ -1084,6 +1085,7 @@ __device__ __forceinline__ void do_item(const ItemArgs& A, long long e, long lon
 // dependent loads and the kernel's cold instructions.
 template <int KT, class T, bool FLAT>
 __global__ void __launch_bounds__(256) k_items(ItemArgs A) {
+  chain_wait();
   const long long n = *A.n_items, n_ev = *A.n_items_ev;
   const long long op_base = A.op_cap > 0 ? *A.n_ops : 0;  // the redone operations come first
   const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
@@ -1330,6 +1332,7 @@ __device__ __forceinline__ void do_chain_warp(const ItemArgs& A, const ChainPool
 constexpr int kChainThreads = 128;
 template <int KT, class T, bool FLAT>
 __global__ void __launch_bounds__(kChainThreads, 4) k_chain(ItemArgs A, ChainPool pool) {
+  chain_wait();
   __shared__ double sh_v[kChainThreads / 32][2 * kMaxSpec];
   const long long n = *A.n_start;
   const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
@@ -1687,6 +1690,7 @@ __global__ void __launch_bounds__(32) k_apply_chain(const PopDev* pops, const in
 // all empty at the step's start) are walked at the per-set rate like any
 // pair.
 __global__ void __launch_bounds__(128) k_walk_rates(const PopDev* pops) {
+  chain_wait();
   const PopDev& P = pops[blockIdx.y];
   int c = blockIdx.x;
   if (c >= P.n_cells || P.n_pairs == 0) return;
@@ -1811,8 +1815,10 @@ __device__ __forceinline__ int pp_remove_bound(const PopDev& P, int p, int t, in
 }
 
 __global__ void k_pp_count(const PopDev* pops, const int* op_pop, const int* op_pair, const int* op_slot,
-                           const int* op_k, const long long* n_ops, int* rm_n) {
+                           const int* op_k, const long long* n_ops, long long cap, int* rm_n) {
+  chain_wait();
   long long Q = *n_ops;
+  if (Q > cap) Q = cap;  // a step graph's bound; the step does not run beyond it
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < Q;
        q += (long long)gridDim.x * blockDim.x) {
     const PopDev& P = pops[op_pop[q]];
@@ -1851,6 +1857,7 @@ __global__ void __launch_bounds__(32 * kPPWarps) k_pp_ops(const PopDev* pops, co
                          const int* op_slot, const int* op_k, const unsigned long long* op_key,
                          const long long* n_ops, PPResult* res, double* res_vol, const long long* rm_off,
                          int* rm_pool, long long rm_cap) {
+  chain_wait();
   constexpr unsigned kFull = 0xffffffffu;
   __shared__ PMeta sh_src[kPPWarps];
   __shared__ double sh_u[kPPWarps][64];
@@ -2188,6 +2195,7 @@ __global__ void __launch_bounds__(32 * kPPWarps) k_pp_ops(const PopDev* pops, co
 __global__ void k_pp_resolve(const PopDev* pops, const int* op_pop, const unsigned long long* op_key,
                              const long long* n_ops, const PPResult* res, const int* rm_pool, uint8_t* win,
                              int* need_slot, int* need_id, int* lost) {
+  chain_wait();
   long long Q = *n_ops;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < Q;
        q += (long long)gridDim.x * blockDim.x) {
@@ -2207,10 +2215,13 @@ __global__ void k_pp_resolve(const PopDev* pops, const int* op_pop, const unsign
 
 // phase 2b: apply the winning target operations
 // walker places of the round's operations, compacted in order
-__global__ void k_walkers_span(const long long* n_ops, long long* n_places) { *n_places = *n_ops * kMaxCopies; }
+__global__ void k_walkers_span(const long long* n_ops, long long* n_places) {
+  chain_wait();
+  *n_places = *n_ops * kMaxCopies; }
 
 __global__ void k_compact_walkers(const long long* n_places, const uint8_t* flag, const long long* off,
                                   const int* wk_slot, const int* wk_gp, int* ppw_slot, int* ppw_gp) {
+  chain_wait();
   const long long n = *n_places;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     if (flag[i]) {
@@ -2224,6 +2235,7 @@ __global__ void k_pp_apply(const PopDev* pops, const int* op_pop, const long lon
                            const long long* slot_rank, const long long* id_rank,
                            const int* slot_base, const long long* id_base, const long long* pop_pair_base,
                            const int* op_k, int* wk_slot, int* wk_gp, uint8_t* wk_flag) {
+  chain_wait();
   // the walkers an operation makes (its target, then its copies) go to the
   // operation's own kMaxCopies places, compacted afterwards in operation
   // order, so that the next round's items do not depend on scheduling

@@ -59,6 +59,32 @@ def test_step_graph_matches_host_rounds(gpu_lib, case):
         assert len(ga) > 1  # the grid was made anew on the way
 
 
+@pytest.mark.parametrize("n_part", [4000, 60000])
+def test_step_graph_with_target_operations(gpu_lib, n_part):
+    """Coarse particles scavenging fine ones, at step lengths that take the
+    target operations from few to many more than the step before (and past
+    the bounds a graph was captured for) and back."""
+    import partmc_b200 as pm
+    from partmc_b200 import aero_dist
+    modes = [(1e11, 0.5e-8, np.log10(1.3)), (1e8, 0.25e-6, np.log10(1.3))]
+    pop = aero_dist.brown_bimodal(n_part, seed=11, modes=modes)
+    env = pm.EnvState(288.0, 1e5)
+    res = []
+    for graphs in (True, False):
+        st = pm.AeroState(pop.aero_data, pop.awa, seed=7)
+        st.set_graphs(graphs)
+        st.add_particles(pop.vol, pop.group)
+        counts = []
+        for del_t in (20.0, 20.0, 20.0, 20.0, 150.0, 20.0, 150.0, 150.0, 150.0, 5.0, 5.0, 600.0, 5.0):
+            counts.append(pm.mc_coag(pm.COAG_KERNEL_TYPE_BROWN, env, pop.aero_data, st, del_t))
+            counts.append((st.stats()["rounds"], st.conflicts()["target_ops"], st.conflicts()["target_op_losers"]))
+        res.append((st.particles(components=True), counts))
+    assert res[0][1] == res[1][1]
+    ops = [c[1] for c in res[0][1][1::2]]
+    assert max(ops) > 4 * min(ops)
+    same(res[0][0], res[1][0])
+
+
 def test_batched_step_graph(gpu_lib):
     """Populations of uneven sizes, one of them empty, in one context."""
     import partmc_b200 as pm
