@@ -285,44 +285,52 @@ struct CompactArgs {
   uint32_t* dec;
 };
 
-// places of the tile's flagged entries: sh_idx[r] is the tile's r-th, and the
-// tile's first event is returned
-__device__ long long compact_tile(const CompactArgs& A, int* sh_idx, int* count) {
+// flags i..i+3 of n, as the bits 0..3
+__device__ __forceinline__ unsigned flags_of(const uint8_t* flag, long long i, long long n) {
+  if (i + 4 <= n) {
+    const uchar4 f = *reinterpret_cast<const uchar4*>(flag + i);
+    return (f.x ? 1u : 0u) | (f.y ? 2u : 0u) | (f.z ? 4u : 0u) | (f.w ? 8u : 0u);
+  }
+  unsigned m = 0u;
+  for (int k = 0; k < 4; k++)
+    if (i + k < n && flag[i + k]) m |= 1u << k;
+  return m;
+}
+// the same of entries that hold a population (-1: none)
+__device__ __forceinline__ unsigned flags_of(const int* pop, long long i, long long n) {
+  unsigned m = 0u;
+  for (int k = 0; k < 4; k++)
+    if (i + k < n && pop[i + k] >= 0) m |= 1u << k;
+  return m;
+}
+
+// places of the tile's flagged entries of n: sh_idx[r] is the tile's r-th, and
+// the place of the tile's first among all is returned; *n_out gets their count
+template <class T>
+__device__ long long compact_tile(const T* flag, long long n, long long* n_out, const TileCtl& ctl, int* sh_idx,
+                                  int* count) {
   __shared__ unsigned long long excl_sh;
-  const long long n = *A.n, n_tiles = (n + kCompactTile - 1) / kCompactTile;
-  const long long tile = take_tile(A.ctl);
+  const long long n_tiles = (n + kCompactTile - 1) / kCompactTile;
+  const long long tile = take_tile(ctl);
   if (tile >= n_tiles) {
-    if (n_tiles == 0 && tile == 0 && threadIdx.x == 0) *A.n_events = 0;
+    if (n_tiles == 0 && tile == 0 && threadIdx.x == 0) *n_out = 0;
     *count = 0;
     return 0;
   }
-  const long long base = tile * kCompactTile + 4 * threadIdx.x;
-  uchar4 f = make_uchar4(0, 0, 0, 0);
-  if (base + 4 <= n) f = *reinterpret_cast<const uchar4*>(A.flag + base);
-  else {
-    if (base < n) f.x = A.flag[base];
-    if (base + 1 < n) f.y = A.flag[base + 1];
-    if (base + 2 < n) f.z = A.flag[base + 2];
-  }
-  const int c = (f.x != 0) + (f.y != 0) + (f.z != 0) + (f.w != 0);
+  const unsigned f = flags_of(flag, tile * kCompactTile + 4 * threadIdx.x, n);
   int tot;
-  int r = block_excl_scan(c, &tot);
-  const int i = 4 * (int)threadIdx.x;
-  if (f.x) sh_idx[r++] = i;
-  if (f.y) sh_idx[r++] = i + 1;
-  if (f.z) sh_idx[r++] = i + 2;
-  if (f.w) sh_idx[r++] = i + 3;
+  int r = block_excl_scan(__popc(f), &tot);
+  for (int k = 0; k < 4; k++)
+    if ((f >> k) & 1u) sh_idx[r++] = (int)(tile * kCompactTile) + 4 * (int)threadIdx.x + k;
   if (threadIdx.x < 32) {
-    const unsigned long long e = tile_prefix(A.ctl.status, tile, (unsigned long long)tot, A.ctl.err);
+    const unsigned long long e = tile_prefix(ctl.status, tile, (unsigned long long)tot, ctl.err);
     if (threadIdx.x == 0) {
       excl_sh = e;
-      if (tile == n_tiles - 1) *A.n_events = (long long)e + tot;
+      if (tile == n_tiles - 1) *n_out = (long long)e + tot;
     }
   }
   __syncthreads();
   *count = tot;
-  for (int k = threadIdx.x; k < tot; k += kCompactThreads) sh_idx[k] += (int)(tile * kCompactTile);
-  __syncthreads();
   return (long long)excl_sh;
 }
 
@@ -340,7 +348,7 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact_samples(CompactArgs
   chain_wait();
   __shared__ int sh_idx[kCompactTile];
   int count;
-  const long long e0 = compact_tile(A, sh_idx, &count);
+  const long long e0 = compact_tile(A.flag, *A.n, A.n_events, A.ctl, sh_idx, &count);
   for (int r = threadIdx.x; r < count; r += kCompactThreads) {
     const long long i = sh_idx[r], e = e0 + r;
     const int gp = ev_gp[i];
@@ -381,7 +389,7 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact_items(CompactArgs A
   chain_wait();
   __shared__ int sh_idx[kCompactTile];
   int count;
-  const long long e0 = compact_tile(A, sh_idx, &count);
+  const long long e0 = compact_tile(A.flag, *A.n, A.n_events, A.ctl, sh_idx, &count);
   for (int r = threadIdx.x; r < count; r += kCompactThreads) {
     const long long i = sh_idx[r], e = grouped ? grouped[i] : e0 + r;
     if (e < 0) continue;
@@ -464,7 +472,7 @@ __device__ long long first_event_of(int k, long long E, const int* ev_gp, const 
 // count of earlier populations is the rank inside the population.  Per-set
 // counts come from the rank scans at the population boundaries (and are
 // stored in per_pop for the host); per-particle counts were summed into
-// per_pop by k_count_per_pop.  The slot and ID counters of each population
+// per_pop by k_pp_resolve.  The slot and ID counters of each population
 // advance here by the round's allocations: the apply kernels read only the
 // bases.  By one block; populations in tiles of blockDim.x.
 __device__ void alloc_bases(const PopDev* pops, int n_pop, long long E, const int* ev_gp, const int* gpair_pop,
@@ -615,16 +623,133 @@ __global__ void __launch_bounds__(256) k_resolve(ResolveArgs A) {
                 A.set_id_base, A.pp_slot_base, A.pp_id_base);
 }
 
-// need[q] of target operation q summed per population (op_pop[q])
-__global__ void k_count_per_pop(const int* need, const long long* n_items, const int* item_pop_of,
-                                int* per_pop) {
+// The bound on each target operation's removals (pp_remove_bound), scanned into
+// its place in the removal pool; their total to *total.  At most cap operations
+// are counted (a step graph's bound; the step does not run beyond it).
+__global__ void __launch_bounds__(256) k_pp_count(const PopDev* pops, const int* op_pop, const int* op_pair,
+                                                  const int* op_slot, const int* op_k, const long long* n_ops,
+                                                  long long cap, long long* rm_off, long long* total, TileCtl ctl) {
   chain_wait();
-  long long n = *n_items;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    if (!need[e]) continue;
-    atomicAdd(&per_pop[item_pop_of[e]], need[e]);
+  __shared__ unsigned long long excl_sh;
+  const long long Q = *n_ops < cap ? *n_ops : cap, n_tiles = (Q + 255) / 256;
+  const long long tile = take_tile(ctl);
+  if (tile < n_tiles) {
+    const long long q = tile * 256 + threadIdx.x;
+    int n = 0;
+    if (q < Q) {
+      Rng g(0, 0, 0, 0);
+      int n_extra = 0;
+      double prm = 0.0;
+      n = pp_remove_bound(pops[op_pop[q]], op_pair[q], op_slot[q], op_k[q], &g, &n_extra, &prm);
+      if (n < 0) n = 0;
+    }
+    long long tot;
+    const long long pre = block_excl_scan_ll(n, &tot);
+    if (threadIdx.x < 32) {
+      const unsigned long long x = tile_prefix(ctl.status, tile, (unsigned long long)tot, ctl.err);
+      if (threadIdx.x == 0) excl_sh = x;
+    }
+    __syncthreads();
+    if (q < Q) rm_off[q] = (long long)excl_sh + pre;
+    if (tile == n_tiles - 1 && threadIdx.x == 0) *total = (long long)excl_sh + tot;
+  } else if (n_tiles == 0 && tile == 0 && threadIdx.x == 0) {
+    *total = 0;
   }
+  last_block(ctl);
+}
+
+// Winners of the round's target operations, the ranks of the slots (and IDs:
+// as many) that their copies need, the needs per population, and the places of
+// the operations that lost, whose count goes to *n_lost: one launch for what
+// were five.
+__global__ void __launch_bounds__(256) k_pp_resolve(const PopDev* pops, int n_pop, const int* op_pop,
+                                                    const unsigned long long* op_key, const long long* n_ops,
+                                                    const PPResult* res, const int* rm_pool, uint8_t* win,
+                                                    long long* rank, int* per_pop, int* lost, long long* lost_off,
+                                                    long long* n_lost, TileCtl ctl) {
+  chain_wait();
+  __shared__ unsigned long long excl_sh;
+  const long long Q = *n_ops, n_tiles = (Q + 255) / 256;
+  const long long tile = take_tile(ctl);
+  if (tile < n_tiles) {
+    const long long q = tile * 256 + threadIdx.x;
+    bool ok = true;
+    int extra = 0;
+    if (q < Q) {
+      const int pop = op_pop[q];
+      const PopDev& P = pops[pop];
+      const PPResult& R = res[q];
+      const unsigned long long ck = claim_key(P, op_key[q]);
+      ok = !R.nofit;
+      if (R.merged) ok = ok && holds_slot(P, R.target, ck, true);
+      for (int z = 0; z < R.n_rm && ok; z++) ok = holds_slot(P, rm_pool[R.rm_off + z], ck, true);
+      win[q] = ok ? 1 : 0;
+      lost[q] = ok ? 0 : 1;
+      extra = (ok && R.merged && R.n_copies > 1) ? R.n_copies - 1 : 0;
+      if (extra) {
+        atomicAdd(&per_pop[2 * n_pop + pop], extra);
+        atomicAdd(&per_pop[3 * n_pop + pop], extra);
+      }
+    }
+    // at most 7 x 256 copies and 256 losers in a tile: one scan of both
+    int tot;
+    const int pre = block_excl_scan(extra | (ok ? 0 : 1 << 16), &tot);
+    if (threadIdx.x < 32) {
+      const unsigned long long agg = (unsigned long long)(tot & 0xffff) | ((unsigned long long)(tot >> 16) << 31);
+      const unsigned long long x = tile_prefix(ctl.status, tile, agg, ctl.err);
+      if (threadIdx.x == 0) excl_sh = x;
+    }
+    __syncthreads();
+    const long long s0 = (long long)(excl_sh & 0x7fffffffULL), l0 = (long long)(excl_sh >> 31);
+    if (q < Q) {
+      rank[q] = s0 + (pre & 0xffff);
+      lost_off[q] = l0 + (pre >> 16);
+    }
+    if (tile == n_tiles - 1 && threadIdx.x == 0) *n_lost = l0 + (tot >> 16);
+  } else if (n_tiles == 0 && tile == 0 && threadIdx.x == 0) {
+    *n_lost = 0;
+  }
+  last_block(ctl);
+}
+
+// walker places of the round's operations (kMaxCopies each), compacted in order
+__global__ void __launch_bounds__(kCompactThreads) k_compact_walkers(const uint8_t* flag, const long long* n_ops,
+                                                                     long long* n_walkers, TileCtl ctl,
+                                                                     const int* wk_slot, const int* wk_gp,
+                                                                     int* ppw_slot, int* ppw_gp) {
+  chain_wait();
+  __shared__ int sh_idx[kCompactTile];
+  int count;
+  const long long e0 = compact_tile(flag, *n_ops * kMaxCopies, n_walkers, ctl, sh_idx, &count);
+  for (int r = threadIdx.x; r < count; r += kCompactThreads) {
+    ppw_slot[e0 + r] = wk_slot[sh_idx[r]];
+    ppw_gp[e0 + r] = wk_gp[sh_idx[r]];
+  }
+  last_block(ctl);
+}
+
+// A later round's target operations of one population from the staging list,
+// in order, without the places that hold none
+__global__ void __launch_bounds__(kCompactThreads) k_compact_ops(const long long* n_staged, long long* n_ops,
+                                                                 TileCtl ctl, const int* pop, const int* pair,
+                                                                 const int* slot, const int* k,
+                                                                 const unsigned long long* key, int* pop_o,
+                                                                 int* pair_o, int* slot_o, int* k_o,
+                                                                 unsigned long long* key_o) {
+  chain_wait();
+  __shared__ int sh_idx[kCompactTile];
+  int count;
+  const long long e0 = compact_tile(pop, *n_staged, n_ops, ctl, sh_idx, &count);
+  for (int r = threadIdx.x; r < count; r += kCompactThreads) {
+    const int i = sh_idx[r];
+    const long long e = e0 + r;
+    pop_o[e] = pop[i];
+    pair_o[e] = pair[i];
+    slot_o[e] = slot[i];
+    k_o[e] = k[i];
+    key_o[e] = key[i];
+  }
+  last_block(ctl);
 }
 
 // particle upload: the caller's arrays were copied straight into slots
@@ -1304,7 +1429,7 @@ struct Ctx {
   Tune tune;
   Tuner tuner;
   // removal pool of the round's target operations
-  DevBuf<int> pp_rm_n, pp_rm_pool;
+  DevBuf<int> pp_rm_pool;
   DevBuf<uint8_t> pop_on;  // the populations a refresh covers
   // a batched round's lists grouped by population (group_by_pop)
   DevBuf<int> grp_hist, item_pop;
@@ -1312,7 +1437,6 @@ struct Ctx {
   // walkers of the round's operations, one place per operation and copy
   DevBuf<int> wk_slot, wk_gp;
   DevBuf<uint8_t> wk_flag;
-  DevBuf<long long> wk_off;
   DevBuf<long long> pp_rm_off, pp_rm_tot;
   // initial-condition sampler: staging of the modes, copy counts, radix select
   DevBuf<double> sample_buf;
@@ -1352,8 +1476,8 @@ struct Ctx {
   DevBuf<int> ch_y, ch_q;
   DevBuf<float> ch_pos;
   long long ch_chunks = 0;
-  DevBuf<int> need_slot_pp, need_id_pp, lost_pp;
-  DevBuf<long long> rank_slot_set, rank_id_set, rank_slot_pp, rank_id_pp, lost_off;
+  DevBuf<int> lost_pp;
+  DevBuf<long long> rank_slot_set, rank_id_set, rank_slot_pp, lost_off;
   DevBuf<int> op_pop, op_pair, op_slot, op_k, r_pop, r_pair, r_slot, r_k;
   DevBuf<unsigned long long> op_key, r_key;
   DevBuf<PPResult> pp_res;
@@ -1613,6 +1737,8 @@ void scan_multi(Ctx& c, std::initializer_list<ScanArg<T>> args, cudaStream_t st 
   launch_chained(c, k_scan_lb<T>, g, dim3(kScanThreads), 0, st, jobs, c.scan_status.p, (int)nb, c.scan_ctr.p,
                  c.scan_ctr.p + kScanMaxJobs, c.scan_err.p);
 }
+
+long long compact_tiles(long long n) { return std::max<long long>(1, (n + kCompactTile - 1) / kCompactTile); }
 
 // shared words of a tiled launch of at most `tiles` blocks
 TileCtl tile_ctl(Ctx& c, long long tiles, cudaStream_t st) {
@@ -2294,11 +2420,6 @@ void launch_items_kt(Ctx& c, int kt, bool flat, int n_gpairs, long long W, cudaS
   });
 }
 
-// the round's staged target operations: the redone ones, then one place per item
-__global__ void k_ops_span(long long* n_ops, const long long* n_items) {
-  chain_wait();
-  n_ops[0] += *n_items; }
-
 // Stable grouping by population of a batched context's per-round lists.
 // Slot and ID ranks come from one scan over a list, and the per-population
 // bases of k_alloc_bases assume that each population's entries lie together
@@ -2407,14 +2528,13 @@ void reserve_ops(Ctx& c, long long Q) {
   c.op_pop.reserve(q); c.op_pair.reserve(q); c.op_slot.reserve(q); c.op_k.reserve(q); c.op_key.reserve(q);
   c.pp_res.reserve(q);
   c.pp_vol.reserve(q * c.n_spec);
-  c.pp_rm_n.reserve(q + 1);
   c.pp_rm_off.reserve(q + 2);
   c.pp_rm_tot.reserve(1);
-  c.need_slot_pp.reserve(q + 1); c.need_id_pp.reserve(q + 1); c.win_pp.reserve(q + 1); c.lost_pp.reserve(q + 1);
-  c.lost_off.reserve(q + 2); c.rank_slot_pp.reserve(q + 2); c.rank_id_pp.reserve(q + 2);
+  c.win_pp.reserve(q + 1); c.lost_pp.reserve(q + 1);
+  c.lost_off.reserve(q + 2); c.rank_slot_pp.reserve(q + 2);
   c.grp_dest.reserve(q + 1);
   const size_t nw = q * kMaxCopies;
-  c.wk_slot.reserve(nw); c.wk_gp.reserve(nw); c.wk_flag.reserve(nw); c.wk_off.reserve(nw + 1);
+  c.wk_slot.reserve(nw); c.wk_gp.reserve(nw); c.wk_flag.reserve(nw);
   const size_t nh = std::max<size_t>(1, (q + kGrpTile - 1) / kGrpTile) * c.n_pop;
   c.grp_hist.reserve(nh);
   c.grp_off.reserve(nh + 1);
@@ -2426,23 +2546,29 @@ void reserve_redo(Ctx& c, long long Q) {
   c.r_pop.reserve(q); c.r_pair.reserve(q); c.r_slot.reserve(q); c.r_k.reserve(q); c.r_key.reserve(q);
 }
 
-// A later round's target operations (at most Q staged in r_*, n_dev[0] of
+// A later round's target operations (at most Q staged in r_*, n_dev[2] of
 // them): the redone ones, then one place per item (population -1 where the
 // item made none).  Grouped by population into op_*, which also drops the
 // empty places; n_dev[1] counts the operations kept.
 void launch_pp_group(Ctx& c, long long Q, cudaStream_t st) {
-  group_by_pop(c, c.n_dev.p, Q, c.r_pop.p, c.grp_dest.p, st, c.n_dev.p + 1);
-  launch_chained(c, k_scatter_ops, dim3(grid_for(Q, 256)), dim3(256), 0, st, c.n_dev.p, c.grp_dest.p, c.r_pop.p, c.r_pair.p, c.r_slot.p,
-                                                  c.r_k.p, c.r_key.p, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p,
-                                                  c.op_key.p);
+  if (c.n_pop == 1) {  // one population: only the empty places go
+    launch_chained(c, k_compact_ops, dim3((unsigned)compact_tiles(Q)), dim3(kCompactThreads), 0, st, c.n_dev.p + 2,
+                   c.n_dev.p + 1, tile_ctl(c, compact_tiles(Q), st), c.r_pop.p, c.r_pair.p, c.r_slot.p, c.r_k.p,
+                   c.r_key.p, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p, c.op_key.p);
+    return;
+  }
+  group_by_pop(c, c.n_dev.p + 2, Q, c.r_pop.p, c.grp_dest.p, st, c.n_dev.p + 1);
+  launch_chained(c, k_scatter_ops, dim3(grid_for(Q, 256)), dim3(256), 0, st, c.n_dev.p + 2, c.grp_dest.p, c.r_pop.p,
+                 c.r_pair.p, c.r_slot.p, c.r_k.p, c.r_key.p, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p,
+                 c.op_key.p);
 }
 
 // the bound on each target operation's removals, scanned into its place in
 // the removal pool (their total in pp_rm_tot); n_ops: their count
 void launch_pp_count(Ctx& c, long long Q, const long long* n_ops, cudaStream_t st) {
-  launch_chained(c, k_pp_count, dim3(grid_for(Q, 128)), dim3(128), 0, st, c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p,
-                 c.op_k.p, n_ops, Q, c.pp_rm_n.p);
-  scan_multi<int>(c, {ScanArg<int>{c.pp_rm_n.p, Q, n_ops, c.pp_rm_off.p, c.pp_rm_tot.p}}, st);
+  const long long tiles = std::max<long long>(1, (Q + 255) / 256);
+  launch_chained(c, k_pp_count, dim3((unsigned)tiles), dim3(256), 0, st, c.d_pops, c.op_pop.p, c.op_pair.p,
+                 c.op_slot.p, c.op_k.p, n_ops, Q, c.pp_rm_off.p, c.pp_rm_tot.p, tile_ctl(c, tiles, st));
 }
 
 // Every operation's removals fit the pool: one that did not would lose
@@ -2657,7 +2783,10 @@ __global__ void k_round_begin(uint32_t* d_round, long long* round_dev, int* per_
     round_dev[6] = round_dev[1];
     round_dev[7] = round_dev[5];
     round_dev[2] = round_dev[1] + round_dev[5];
-    n_dev[0] = round_dev[8];  // the target operations redone in this round
+    // the target operations redone in this round, and the places of its
+    // staging list: those, then one per item
+    n_dev[0] = round_dev[8];
+    n_dev[2] = round_dev[8] + round_dev[2];
     round_dev[0] = 0;
     round_dev[1] = 0;
     round_dev[3] = 0;
@@ -2815,14 +2944,10 @@ void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q, bool chain
   // Q bounds the round's target operations; their count is n_dev[1] (the
   // redone ones, then those that walks appended)
   if (Q > 0) {
-    launch_chained(c, k_pp_resolve, dim3(grid_for(Q, 256)), dim3(256), 0, st, c.d_pops, c.op_pop.p, c.op_key.p, c.n_dev.p + 1, c.pp_res.p,
-                                                   c.pp_rm_pool.p, c.win_pp.p, c.need_slot_pp.p, c.need_id_pp.p, c.lost_pp.p);
-    scan_multi<int>(c, {{c.need_slot_pp.p, Q, c.n_dev.p + 1, c.rank_slot_pp.p}, {c.need_id_pp.p, Q, c.n_dev.p + 1, c.rank_id_pp.p}},
-                    st);
-    launch_chained(c, k_count_per_pop, dim3(grid_for(Q, 256)), dim3(256), 0, st, c.need_slot_pp.p, c.n_dev.p + 1, c.op_pop.p,
-                                                      c.per_pop_i.p + 2 * c.n_pop);
-    launch_chained(c, k_count_per_pop, dim3(grid_for(Q, 256)), dim3(256), 0, st, c.need_id_pp.p, c.n_dev.p + 1, c.op_pop.p,
-                                                      c.per_pop_i.p + 3 * c.n_pop);
+    const long long tiles = std::max<long long>(1, (Q + 255) / 256);
+    launch_chained(c, k_pp_resolve, dim3((unsigned)tiles), dim3(256), 0, st, c.d_pops, c.n_pop, c.op_pop.p, c.op_key.p,
+                   c.n_dev.p + 1, c.pp_res.p, c.pp_rm_pool.p, c.win_pp.p, c.rank_slot_pp.p, c.per_pop_i.p, c.lost_pp.p,
+                   c.lost_off.p, c.round_dev.p + 8, tile_ctl(c, tiles, st));
   }
   {
     TuneScope ts(c, kTuneResolve, st);
@@ -2885,21 +3010,16 @@ void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q, bool chain
     }
   }
   if (Q > 0) {
-    const size_t nw = (size_t)Q * kMaxCopies;
-    launch_chained(c, k_pp_apply, dim3(grid_for(Q, 256)), dim3(256), 0, st, c.d_pops, c.op_pop.p, c.n_dev.p + 1, c.pp_res.p, c.pp_vol.p,
-                                                 c.pp_rm_pool.p, c.win_pp.p, c.rank_slot_pp.p, c.rank_id_pp.p,
-                                                 c.slot_base_pp.p, c.id_base_pp.p, c.pop_pair_base.p, c.op_k.p,
-                                                 c.wk_slot.p, c.wk_gp.p, c.wk_flag.p);
-    launch_chained(c, k_walkers_span, dim3(1), dim3(1), 0, st, c.n_dev.p + 1, c.round_dev.p + 9);
-    scan_multi<uint8_t>(c, {ScanArg<uint8_t>{c.wk_flag.p, (long long)nw, c.round_dev.p + 9, c.wk_off.p,
-                                             c.round_dev.p + 5}}, st);
-    launch_chained(c, k_compact_walkers, dim3(grid_for((long long)nw, 256)), dim3(256), 0, st, c.round_dev.p + 9, c.wk_flag.p, c.wk_off.p,
-                                                                    c.wk_slot.p, c.wk_gp.p, c.ppw_slot.p, c.ppw_gp.p);
-    scan_multi<int>(c, {ScanArg<int>{c.lost_pp.p, Q, c.n_dev.p + 1, c.lost_off.p, c.round_dev.p + 8}}, st);
+    launch_chained(c, k_pp_apply, dim3(grid_for(Q, 128)), dim3(128), 0, st, c.d_pops, c.op_pop.p, c.n_dev.p + 1,
+                   c.pp_res.p, c.pp_vol.p, c.pp_rm_pool.p, c.win_pp.p, c.rank_slot_pp.p, c.slot_base_pp.p,
+                   c.id_base_pp.p, c.pop_pair_base.p, c.op_k.p, c.wk_slot.p, c.wk_gp.p, c.wk_flag.p);
+    const long long tiles = compact_tiles(Q * kMaxCopies);
+    launch_chained(c, k_compact_walkers, dim3((unsigned)tiles), dim3(kCompactThreads), 0, st, c.wk_flag.p,
+                   c.n_dev.p + 1, c.round_dev.p + 5, tile_ctl(c, tiles, st), c.wk_slot.p, c.wk_gp.p, c.ppw_slot.p,
+                   c.ppw_gp.p);
   }
 }
 
-long long compact_tiles(long long n) { return std::max<long long>(1, (n + kCompactTile - 1) / kCompactTile); }
 
 CompactArgs compact_args(Ctx& c, const uint8_t* flag, const long long* n, long long bound, cudaStream_t st) {
   CompactArgs A;
@@ -2967,7 +3087,6 @@ void enqueue_round_head(Ctx& c, cudaStream_t st, const RoundBounds& b, long long
   }
   launch_items_kt(c, b.kt, b.flat, b.n_gpairs, b.W, st);
   if (Q > 0) {
-    launch_chained(c, k_ops_span, dim3(1), dim3(1), 0, st, c.n_dev.p, c.round_dev.p + 2);
     launch_pp_group(c, Q, st);
     launch_pp_count(c, Q, c.n_dev.p + 1, st);
   }
@@ -3258,11 +3377,11 @@ std::vector<long long> step_graph_key(const Ctx& c, const RoundBounds& b, long l
          {q_cap, qb_cap, (long long)c.op_pop.p, (long long)c.op_pair.p, (long long)c.op_slot.p, (long long)c.op_k.p,
           (long long)c.op_key.p, (long long)c.r_pop.p, (long long)c.r_pair.p, (long long)c.r_slot.p,
           (long long)c.r_k.p, (long long)c.r_key.p, (long long)c.pp_res.p, (long long)c.pp_vol.p,
-          (long long)c.pp_rm_n.p, (long long)c.pp_rm_off.p, (long long)c.pp_rm_tot.p, (long long)c.pp_rm_pool.p,
-          (long long)c.pp_rm_pool.n, (long long)c.need_slot_pp.p, (long long)c.need_id_pp.p, (long long)c.win_pp.p,
-          (long long)c.lost_pp.p, (long long)c.lost_off.p, (long long)c.rank_slot_pp.p, (long long)c.rank_id_pp.p,
+          (long long)c.pp_rm_off.p, (long long)c.pp_rm_tot.p, (long long)c.pp_rm_pool.p,
+          (long long)c.pp_rm_pool.n, (long long)c.win_pp.p,
+          (long long)c.lost_pp.p, (long long)c.lost_off.p, (long long)c.rank_slot_pp.p,
           (long long)c.grp_dest.p, (long long)c.grp_hist.p, (long long)c.grp_off.p, (long long)c.item_pop.p,
-          (long long)c.wk_slot.p, (long long)c.wk_gp.p, (long long)c.wk_flag.p, (long long)c.wk_off.p})
+          (long long)c.wk_slot.p, (long long)c.wk_gp.p, (long long)c.wk_flag.p})
       k.push_back(v);
   for (long long v : {(long long)c.report.dev, (long long)c.report_seq.p, (long long)c.n_dev.p, w_cap, (long long)max_pairs, (long long)c.prof, (long long)c.tune.threads[kTuneTest],
                       (long long)c.nwork_set.p, (long long)c.nwork_pp.p, (long long)c.work_off.p,
@@ -3478,7 +3597,7 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
     const long long qs = std::max(q_cap, qb_cap), hist = (std::max(qs, q_cap > 0 ? b.W : 0) / kGrpTile + 2) * c.n_pop;
     const long long lists = std::max(std::max(kMaxCopies * qs, hist), (long long)b.n_gpairs);
     const long long nb = std::max((c.sg_w + kScanTile - 1) / kScanTile, (lists + kScanTile - 1) / kScanTile);
-    c.scan_status.reserve((size_t)std::max(kScanMaxJobs * nb, std::max(c.sg_w, b.W) / kResolveMin + 2));
+    c.scan_status.reserve((size_t)std::max(std::max(kScanMaxJobs * nb, std::max(c.sg_w, b.W) / kResolveMin + 2), qs / 64 + 2));
     if (c.scan_status.n > c.scan_status_n) {
       CK(cudaMemsetAsync(c.scan_status.p, 0, sizeof(unsigned long long) * c.scan_status.n, c.stream));
       c.scan_status_n = c.scan_status.n;
@@ -3998,14 +4117,13 @@ int pmc_coag_gpu_destroy(pmc_coag_gpu_ctx* x) {
   cudaFree(c.d_pops);
   cudaFree(c.d_stat);
   cudaFree(c.d_round);
-  DevBuf<int>* bi[] = {&c.gpair_pop, &c.gpair_local, &c.need_slot_pp,
-                       &c.need_id_pp, &c.lost_pp, &c.op_pop, &c.op_pair, &c.op_slot, &c.op_k, &c.r_pop,
+  DevBuf<int>* bi[] = {&c.gpair_pop, &c.gpair_local, &c.lost_pp, &c.op_pop, &c.op_pair, &c.op_slot, &c.op_k, &c.r_pop,
                        &c.r_pair, &c.r_slot, &c.r_k, &c.per_pop_i, &c.slot_base_set, &c.slot_base_pp,
                        &c.ev_dest, &c.ev_len, &c.ev_head, &c.ev_app, &c.it_gp, &c.it_len, &c.it_head, &c.it_start,
                        &c.ch_y, &c.ch_q};
   for (auto* b : bi) b->release();
   DevBuf<long long>* bl[] = {&c.pop_pair_base, &c.nwork_set, &c.nwork_pp, &c.work_off, &c.pp_off,
-                             &c.rank_slot_set, &c.rank_id_set, &c.rank_slot_pp, &c.rank_id_pp, &c.lost_off,
+                             &c.rank_slot_set, &c.rank_id_set, &c.rank_slot_pp, &c.lost_off,
                              &c.id_base_set, &c.id_base_pp, &c.n_dev};
   for (auto* b : bl) b->release();
   DevBuf<unsigned long long>* bk[] = {&c.ev_key, &c.it_key, &c.op_key, &c.r_key};
@@ -4054,14 +4172,12 @@ int pmc_coag_gpu_destroy(pmc_coag_gpu_ctx* x) {
     if (ev) cudaEventDestroy(ev);
   c.graph_stats.release();
   c.sample_buf.release();
-  c.pp_rm_n.release();
   for (auto* b : {&c.grp_hist, &c.item_pop, &c.ppw_slot, &c.ppw_gp}) b->release();
   c.grp_off.release();
   c.grp_dest.release();
   c.wk_slot.release();
   c.wk_gp.release();
   c.wk_flag.release();
-  c.wk_off.release();
   c.pp_rm_pool.release();
   c.pp_rm_off.release();
   c.pp_rm_tot.release();

@@ -1790,9 +1790,9 @@ __device__ double pp_kernel(const PopDev& P, const RecD& qs, const RecD& qt, int
 
 // The first draws of a target operation: the number of removal samples,
 // which bounds the sources it can remove (sample_source_particle,
-// coagulation.F90:397).  k_pp_count stores that bound per operation;
-// its scan places every operation's removals in one pool, so an operation
-// can remove any number of sources.  Returns -1 for an operation that
+// coagulation.F90:397).  k_pp_count scans the bounds, which places every
+// operation's removals in one pool, so an operation can remove any number of
+// sources.  Returns -1 for an operation that
 // draws nothing (void, dead target, empty source cell).
 __device__ __forceinline__ int pp_remove_bound(const PopDev& P, int p, int t, int k, Rng* g_out, int* n_extra,
                                                double* prm_out) {
@@ -1812,22 +1812,6 @@ __device__ __forceinline__ int pp_remove_bound(const PopDev& P, int p, int t, in
   *g_out = g;
   *prm_out = prm_max;
   return n_remove;
-}
-
-__global__ void k_pp_count(const PopDev* pops, const int* op_pop, const int* op_pair, const int* op_slot,
-                           const int* op_k, const long long* n_ops, long long cap, int* rm_n) {
-  chain_wait();
-  long long Q = *n_ops;
-  if (Q > cap) Q = cap;  // a step graph's bound; the step does not run beyond it
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < Q;
-       q += (long long)gridDim.x * blockDim.x) {
-    const PopDev& P = pops[op_pop[q]];
-    Rng g(0, 0, 0, 0);
-    int n_extra = 0;
-    double prm = 0.0;
-    int n = pp_remove_bound(P, op_pair[q], op_slot[q], op_k[q], &g, &n_extra, &prm);
-    rm_n[q] = n > 0 ? n : 0;
-  }
 }
 
 // uniform number u (counted from 0) of the stream g: Rng::next's values by index
@@ -2191,50 +2175,11 @@ __global__ void __launch_bounds__(32 * kPPWarps) k_pp_ops(const PopDev* pops, co
   }
 }
 
-// phase 2a: winners and allocation needs of the target operations
-__global__ void k_pp_resolve(const PopDev* pops, const int* op_pop, const unsigned long long* op_key,
-                             const long long* n_ops, const PPResult* res, const int* rm_pool, uint8_t* win,
-                             int* need_slot, int* need_id, int* lost) {
-  chain_wait();
-  long long Q = *n_ops;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < Q;
-       q += (long long)gridDim.x * blockDim.x) {
-    const PopDev& P = pops[op_pop[q]];
-    const PPResult& R = res[q];
-    unsigned long long prio = op_key[q];
-    bool ok = !R.nofit;
-    if (R.merged) ok = ok && holds_slot(P, R.target, claim_key(P, prio), true);
-    for (int z = 0; z < R.n_rm; z++) ok = ok && holds_slot(P, rm_pool[R.rm_off + z], claim_key(P, prio), true);
-    win[q] = ok ? 1 : 0;
-    lost[q] = ok ? 0 : 1;
-    int extra = (ok && R.merged && R.n_copies > 1) ? R.n_copies - 1 : 0;
-    need_slot[q] = extra;
-    need_id[q] = extra;
-  }
-}
-
-// phase 2b: apply the winning target operations
-// walker places of the round's operations, compacted in order
-__global__ void k_walkers_span(const long long* n_ops, long long* n_places) {
-  chain_wait();
-  *n_places = *n_ops * kMaxCopies; }
-
-__global__ void k_compact_walkers(const long long* n_places, const uint8_t* flag, const long long* off,
-                                  const int* wk_slot, const int* wk_gp, int* ppw_slot, int* ppw_gp) {
-  chain_wait();
-  const long long n = *n_places;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    if (flag[i]) {
-      ppw_slot[off[i]] = wk_slot[i];
-      ppw_gp[off[i]] = wk_gp[i];
-    }
-}
-
-__global__ void k_pp_apply(const PopDev* pops, const int* op_pop, const long long* n_ops,
+// phase 2: apply the winning target operations (k_pp_resolve)
+__global__ void __launch_bounds__(128) k_pp_apply(const PopDev* pops, const int* op_pop, const long long* n_ops,
                            const PPResult* res, const double* res_vol, const int* rm_pool, const uint8_t* win,
-                           const long long* slot_rank, const long long* id_rank,
-                           const int* slot_base, const long long* id_base, const long long* pop_pair_base,
-                           const int* op_k, int* wk_slot, int* wk_gp, uint8_t* wk_flag) {
+                           const long long* rank, const int* slot_base, const long long* id_base,
+                           const long long* pop_pair_base, const int* op_k, int* wk_slot, int* wk_gp, uint8_t* wk_flag) {
   chain_wait();
   // the walkers an operation makes (its target, then its copies) go to the
   // operation's own kMaxCopies places, compacted afterwards in operation
@@ -2284,14 +2229,14 @@ __global__ void k_pp_apply(const PopDev* pops, const int* op_pop, const long lon
         refresh_slot(P, t);
         add_walker(t, 0);
         for (int z = 1; z < R.n_copies; z++) {
-          int dest = slot_base[pop] + (int)slot_rank[q] + (z - 1);
+          int dest = slot_base[pop] + (int)rank[q] + (z - 1);
           if (dest >= P.cap) {
             cap_fail(P.ctr, kCapCopySlot);
             break;
           }
           PMeta cm = R.meta;
           cm.grp = R.copy_group[z];
-          cm.id = id_base[pop] + id_rank[q] + (z - 1);
+          cm.id = id_base[pop] + rank[q] + (z - 1);
           store_particle(P, dest, v, cm);
           refresh_slot(P, dest);
           P.touched[dest] = gen;
