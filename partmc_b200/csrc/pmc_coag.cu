@@ -437,7 +437,7 @@ __global__ void k_build_ops(const PopDev* pops, const int* gpair_pop, const int*
 __global__ void k_build_redo(const PopDev* pops, const int* op_pop, const int* op_pair, const int* op_slot,
                              const int* op_k, const unsigned long long* op_key, const int* lost,
                              const long long* lost_off, const long long* n_ops, int* r_pop, int* r_pair, int* r_slot,
-                             int* r_k, unsigned long long* r_key) {
+                             int* r_k, unsigned long long* r_key, uint32_t begun) {
   const long long Q = *n_ops;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < Q;
        q += (long long)gridDim.x * blockDim.x) {
@@ -448,8 +448,10 @@ __global__ void k_build_redo(const PopDev* pops, const int* op_pop, const int* o
     r_pop[j] = op_pop[q];
     r_pair[j] = op_pair[q];
     // a target that an earlier operation or event of the round consumed
-    // (removed or rewrote) walks on from there instead: its redo is void
-    const bool consumed = t < 0 || t >= P.cap || !P.alive[t] || P.touched[t] == *P.gen_p;
+    // (removed or rewrote) walks on from there instead: its redo is void.  A
+    // slot is stamped with that round's generation, the one before a round
+    // that has begun
+    const bool consumed = t < 0 || t >= P.cap || !P.alive[t] || P.touched[t] == *P.gen_p - begun;
     r_slot[j] = consumed ? -1 : t;
     r_k[j] = op_k[q] + (1 << 24);  // fresh random stream for the redo
     r_key[j] = op_key[q];
@@ -2160,7 +2162,7 @@ size_t size_sort(Ctx& c, int max_cells) {
   return smem;
 }
 
-void launch_sort(Ctx& c, cudaStream_t st, int max_chunks, int max_cells) {
+void launch_sort(Ctx& c, cudaStream_t st, int max_chunks, int max_cells, const StepBegin& begin = StepBegin{}) {
   size_t smem = size_sort(c, max_cells);
   long long items = (long long)c.n_pop * max_chunks;
   int blocks = (int)std::min<long long>(c.sort_blocks, std::max<long long>(items, 1));
@@ -2175,7 +2177,7 @@ void launch_sort(Ctx& c, cudaStream_t st, int max_chunks, int max_cells) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   const PopDev* pops = c.d_pops;
-  CK(cudaLaunchKernelEx(&cfg, k_sort_all, pops, c.n_pop, max_chunks, max_cells));
+  CK(cudaLaunchKernelEx(&cfg, k_sort_all, pops, c.n_pop, max_chunks, max_cells, begin));
   note_launch();
 }
 
@@ -2813,8 +2815,7 @@ __global__ void k_pop_work(const long long* pop_pair_base, int n_pop, const long
 // graph stops and the host loop, which can grow both, carries on.  Rounds
 // with per-particle redo operations run from the host loop.
 
-__global__ void k_round_begin(uint32_t* d_round, long long* round_dev, int* per_pop, int n_per_pop, long long* n_dev) {
-  if (blockIdx.x != 0) return;
+__device__ void round_begin(uint32_t* d_round, long long* round_dev, int* per_pop, int n_per_pop, long long* n_dev) {
   if (threadIdx.x == 0) {
     d_round[0] += 1u;
     d_round[1] += 1u;
@@ -2837,16 +2838,21 @@ __global__ void k_round_begin(uint32_t* d_round, long long* round_dev, int* per_
   }
   for (int k = threadIdx.x; k < n_per_pop; k += blockDim.x) per_pop[k] = 0;
 }
+__global__ void k_round_begin(uint32_t* d_round, long long* round_dev, int* per_pop, int n_per_pop, long long* n_dev) {
+  round_begin(d_round, round_dev, per_pop, n_per_pop, n_dev);
+}
 
 // stats: [0] events that lost a claim, [1] events, [2] rounds, [3] 1 if the
 // graph stopped for lack of room (slots, sort chunks, or more items or target
 // operations than its later launches are bounded by) with work left (2: in the
 // middle of a round, k_pp_fits), [6] scans that gave up, [7] the largest number
 // of items of a later round, [8] of its target operations, at most, [9] target
-// operations, [10] those that lost a claim, [11] the largest removal bound
-__global__ void k_round_end(const long long* round_dev, long long* stats, const uint32_t* d_round, int max_rounds,
+// operations, [10] those that lost a claim, [11] the largest removal bound.
+// If the loop goes on, the next round begins here (per_pop null: it begins by
+// itself).
+__global__ void k_round_end(long long* round_dev, long long* stats, uint32_t* d_round, int max_rounds,
                             const PopDev* pops, PopCtr* ctrs, int n_pop, long long sort_slots, long long max_items,
-                            long long max_ops, const long long* n_dev, const unsigned long long* scan_err,
+                            long long max_ops, long long* n_dev, const unsigned long long* scan_err, int* per_pop,
                             cudaGraphConditionalHandle cond) {
   const long long E = round_dev[1], lost = round_dev[8], items = E + round_dev[5];
   // a step with target operations: at most one more per item
@@ -2862,19 +2868,23 @@ __global__ void k_round_end(const long long* round_dev, long long* stats, const 
   if (left && room && !more)
     for (int k = threadIdx.x; k < n_pop; k += blockDim.x)
       if (ctrs[k].status == 0) ctrs[k].status = kErrTimeout;
-  if (threadIdx.x != 0) return;
-  stats[0] += round_dev[0];
-  stats[1] += E;
-  stats[2] += 1;
-  stats[6] = (long long)*scan_err;
-  if (items > stats[7]) stats[7] = items;
-  if (ops > stats[8]) stats[8] = ops;
-  if (max_ops > 0) {
-    stats[9] += n_dev[1];
-    stats[10] += lost;
+  if (threadIdx.x == 0) {
+    stats[0] += round_dev[0];
+    stats[1] += E;
+    stats[2] += 1;
+    stats[6] = (long long)*scan_err;
+    if (items > stats[7]) stats[7] = items;
+    if (ops > stats[8]) stats[8] = ops;
+    if (max_ops > 0) {
+      stats[9] += n_dev[1];
+      stats[10] += lost;
+    }
+    if (left && !room) stats[3] = 1;
+    cudaGraphSetConditional(cond, more ? 1u : 0u);
   }
-  if (left && !room) stats[3] = 1;
-  cudaGraphSetConditional(cond, more ? 1u : 0u);
+  if (!more || !per_pop) return;
+  __syncthreads();  // the round's counts are read
+  round_begin(d_round, round_dev, per_pop, 4 * n_pop, n_dev);
 }
 
 // The removals of a later round's target operations fit their pool: the
@@ -2902,30 +2912,6 @@ __global__ void k_pp_fits(const long long* rm_tot, long long pool, long long* st
 // so the rest of the graph does nothing and the host runs the step the long
 // way.
 enum : long long { kNoGoGrid = 1, kNoGoOps = 2, kNoGoSamples = 4, kNoGoSlots = 8, kNoGoStops = 16, kNoGoPool = 32 };
-
-__global__ void k_step_begin(PopDev* pops, PopCtr* ctrs, int n_pop, uint32_t* d_round, long long* round_dev,
-                             int* per_pop, long long* stat, const long long* pop_pair_base, int n_gp,
-                             long long* nwork_set, long long* nwork_pp) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n_pop) {
-    PopCtr& r = ctrs[i];
-    r.tot_samp = r.tot_coag = r.kmax_warn = r.redraws = r.walk_tests = 0;
-    r.status = 0;
-    r.bad_site = 0;
-    r.bad_index = 0;
-    r.cap_site = 0;
-    pops[i].step += 1u;
-  }
-  if (i < 4 * n_pop) per_pop[i] = 0;
-  if (i < 12) round_dev[i] = 0;
-  if (i < kStatWords) stat[i] = 0;
-  const int gp = (int)pop_pair_base[n_pop] + i;  // the places past the last pair
-  if (gp < n_gp) nwork_set[gp] = nwork_pp[gp] = 0;
-  if (i == 0) {
-    d_round[0] = 0u;
-    d_round[1] += 1u;
-  }
-}
 
 __global__ void k_step_check(const PopDev* pops, int n_pop, const long long* pop_pair_base, long long* work_off,
                              long long* pp_off, int n_gp, long long w_cap, long long q_cap, const long long* rm_tot,
@@ -3154,10 +3140,11 @@ void enqueue_round_tail(Ctx& c, cudaStream_t st, const RoundBounds& b, long long
   resolve_apply(c, st, W, Q, true);
 }
 
-void launch_build_redo(Ctx& c, long long Q, cudaStream_t st) {
+// begun: 1 if the new round has begun already, 0 before k_round_begin
+void launch_build_redo(Ctx& c, long long Q, uint32_t begun, cudaStream_t st) {
   k_build_redo<<<grid_for(Q, 256), 256, 0, st>>>(c.d_pops, c.op_pop.p, c.op_pair.p, c.op_slot.p, c.op_k.p, c.op_key.p,
                                                  c.lost_pp.p, c.lost_off.p, c.n_dev.p + 1, c.r_pop.p, c.r_pair.p,
-                                                 c.r_slot.p, c.r_k.p, c.r_key.p);
+                                                 c.r_slot.p, c.r_k.p, c.r_key.p, begun);
   note_launch();
 }
 
@@ -3312,7 +3299,7 @@ GraphRun run_round_graph(Ctx& c, int kt, bool flat, int n_gpairs, long long e0) 
       enqueue_round_tail(c, c.cap_stream, b, 0);
       k_round_end<<<1, 128, 0, c.cap_stream>>>(c.round_dev.p, c.graph_stats.p, c.d_round, c.max_rounds, c.d_pops,
                                                c.d_ctrs, c.n_pop, (long long)b.max_chunks * kChunk, b.W, 0, c.n_dev.p,
-                                               c.scan_err.p, cond);
+                                               c.scan_err.p, nullptr, cond);
       note_launch();
     } catch (...) {
       cudaGraph_t dummy;
@@ -3447,12 +3434,20 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
   CK(cudaStreamBeginCaptureToGraph(st, c.sg_graph, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
   cudaGraph_t done = nullptr;
   try {
-    k_step_begin<<<std::max((4 * c.n_pop + 255) / 256, 4), 256, 0, st>>>(
-        c.d_pops, c.d_ctrs, c.n_pop, c.d_round, c.round_dev.p, c.per_pop_i.p, c.d_stat, c.pop_pair_base.p, n_gp,
-        c.nwork_set.p, c.nwork_pp.p);
-    note_launch();
     mark(0);
-    launch_sort(c, st, b.max_chunks, b.max_cells);
+    StepBegin begin;
+    begin.pops = c.d_pops;
+    begin.ctrs = c.d_ctrs;
+    begin.d_round = c.d_round;
+    begin.round_dev = c.round_dev.p;
+    begin.per_pop = c.per_pop_i.p;
+    begin.stat = c.d_stat;
+    begin.n_stat = kStatWords;
+    begin.pop_pair_base = c.pop_pair_base.p;
+    begin.n_gp = n_gp;
+    begin.nwork_set = c.nwork_set.p;
+    begin.nwork_pp = c.nwork_pp.p;
+    launch_sort(c, st, b.max_chunks, b.max_cells, begin);
     mark(1);
     launch_chained(c, k_pairs, dim3(dim3((max_pairs + 127) / 128, c.n_pop)), dim3(128), 0, st, c.d_pops, c.pop_pair_base.p, c.nwork_set.p,
                                                                    c.nwork_pp.p, 1);
@@ -3472,7 +3467,7 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
     launch_compact_samples(c, Wd, w_cap, st);
     resolve_apply(c, st, w_cap, q_cap, false);
     k_round_end<<<1, 128, 0, st>>>(c.round_dev.p, c.d_stat, c.d_round, c.max_rounds, c.d_pops, c.d_ctrs, c.n_pop,
-                                   sort_slots, b.W, qb_cap, c.n_dev.p, c.scan_err.p, cond);
+                                   sort_slots, b.W, qb_cap, c.n_dev.p, c.scan_err.p, c.per_pop_i.p, cond);
     note_launch();
     mark(4);
     c.sg_nodes0 = g_launches - n0;
@@ -3504,9 +3499,7 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
     CK(cudaStreamEndCapture(st, &done));
     const long long n1 = g_launches;
     CK(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    if (qb_cap > 0) launch_build_redo(c, qb_cap, st);
-    k_round_begin<<<1, 128, 0, st>>>(c.d_round, c.round_dev.p, c.per_pop_i.p, 4 * c.n_pop, c.n_dev.p);
-    note_launch();
+    if (qb_cap > 0) launch_build_redo(c, qb_cap, 1, st);  // the round has begun (k_round_end)
     c.fork = true;
     enqueue_round_head(c, st, b, qb_cap);
     if (qb_cap > 0) {
@@ -3522,7 +3515,7 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
     enqueue_round_tail(c, st, b, qb_cap);
     c.fork = false;
     k_round_end<<<1, 128, 0, st>>>(c.round_dev.p, c.d_stat, c.d_round, c.max_rounds, c.d_pops, c.d_ctrs, c.n_pop,
-                                   sort_slots, b.W, qb_cap, c.n_dev.p, c.scan_err.p, cond);
+                                   sort_slots, b.W, qb_cap, c.n_dev.p, c.scan_err.p, c.per_pop_i.p, cond);
     note_launch();
     c.sg_nodes = g_launches - n1;
   } catch (...) {
@@ -3552,7 +3545,7 @@ struct StepRun {
 // Run this step as the graph, if what it relies on holds: a valid sort and
 // current caches and bounds from the steps before, and no target operations
 // in the last one.  d_pops' copies keep their step count on the device
-// (k_step_begin adds one), so a step whose parameters are those of the last
+// (the sort's step_begin adds one), so a step whose parameters are those of the last
 // one pushes nothing.  One read-back, at the end.  The step the long way
 // takes six, with the copies and launches that wait on them: 0.351 ms a step
 // for 1e4 particles under the additive kernel, 0.160 with the graph; 0.860 and
@@ -3659,7 +3652,7 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
     c.sg_key = key;
   }
   if (c.dirty || !params_same) {
-    // k_step_begin advances the step
+    // the sort's step_begin advances the step
     for (auto& ph : c.pops) ph.h.step -= 1u;
     push_pops(c);
     for (auto& ph : c.pops) ph.h.step += 1u;
@@ -4001,7 +3994,7 @@ void step_rounds(Ctx& c, int kt, bool flat, int n_gpairs, long long Q, int round
     // the operations that lost are staged for this round before their
     // buffers, which they are read from, may grow
     if (Qb > 0) reserve_redo(c, Qb);
-    if (pp_lost > 0) launch_build_redo(c, last_qb, c.stream);
+    if (pp_lost > 0) launch_build_redo(c, last_qb, 0, c.stream);
     if (Qb > 0) reserve_ops(c, Qb);
     c.op_cap = Qb;
     // the walkers the last round's operations made are this round's to read

@@ -288,8 +288,49 @@ __device__ __forceinline__ void sort_rank_keys(int* keys, int lane, int* cnt) {
   }
 }
 
+// What a step captured as a graph starts with, done by the sort's first phase:
+// the populations' counters and step numbers, the round and claim generation,
+// the round's counts and the report cleared, and the places of the pair list
+// past the last pair emptied.  As kernels of their own, this and the round's
+// start took 3 to 4 us each (100 steps of 1e4 particles: 15.4 ms, 14.2 with
+// this and the round's start in k_round_end).  A
+// histogram error that phase 1 sets while another block clears the counters is
+// set again by phases 2 and 3.
+struct StepBegin {
+  PopDev* pops = nullptr;  // null: not the start of a step
+  PopCtr* ctrs = nullptr;
+  uint32_t* d_round = nullptr;
+  long long* round_dev = nullptr;
+  int* per_pop = nullptr;
+  long long* stat = nullptr;
+  int n_stat = 0;
+  const long long* pop_pair_base = nullptr;
+  int n_gp = 0;
+  long long *nwork_set = nullptr, *nwork_pp = nullptr;
+};
+
+__device__ __forceinline__ void step_begin(const StepBegin& B, int n_pop, int i0, int stride) {
+  for (int i = i0; i < n_pop; i += stride) {
+    PopCtr& r = B.ctrs[i];
+    r.tot_samp = r.tot_coag = r.kmax_warn = r.redraws = r.walk_tests = 0;
+    r.status = 0;
+    r.bad_site = 0;
+    r.bad_index = 0;
+    r.cap_site = 0;
+    B.pops[i].step += 1u;
+  }
+  for (int i = i0; i < 4 * n_pop; i += stride) B.per_pop[i] = 0;
+  for (int i = i0; i < 12; i += stride) B.round_dev[i] = 0;
+  for (int i = i0; i < B.n_stat; i += stride) B.stat[i] = 0;
+  for (int gp = (int)B.pop_pair_base[n_pop] + i0; gp < B.n_gp; gp += stride) B.nwork_set[gp] = B.nwork_pp[gp] = 0;
+  if (i0 == 0) {
+    B.d_round[0] = 0u;
+    B.d_round[1] += 1u;
+  }
+}
+
 __global__ void __launch_bounds__(kSortThreads, 6) k_sort_all(const PopDev* pops, int n_pop, int max_chunks,
-                                                           int max_cells) {
+                                                           int max_cells, StepBegin begin) {
   namespace cg = cooperative_groups;
   cg::grid_group grid = cg::this_grid();
   extern __shared__ int sm[];  // [kSortWarps][max_cells] counters, [max_cells] cell starts, [n_pop + 1] chunk_base
@@ -334,6 +375,8 @@ __global__ void __launch_bounds__(kSortThreads, 6) k_sort_all(const PopDev* pops
   int keys[kKeysPerThread];
   long long kept = -1;  // chunk item whose keys, ranks and warp counts are at hand
   // phase 1
+  if (begin.pops)
+    step_begin(begin, n_pop, (int)(blockIdx.x * blockDim.x + threadIdx.x), (int)(gridDim.x * blockDim.x));
   if (blockIdx.x == 0)
     for (int k = threadIdx.x; k < n_pop; k += blockDim.x) {
       pops[k].ctr->bmin = 1 << 30;
