@@ -194,15 +194,14 @@ int pmc_coag_gpu_rebalance(pmc_coag_gpu_ctx *ctx, int pop,
 
 /* Autotuning of the step's launch shapes (no counterpart in the reference).
  * Five launch sites have a threads-per-block choice: the pair tests, the
- * merge decisions and claim resolution, the walks, the chains, and the
- * apply.  pmc_coag_gpu_autotune(ctx, 1) makes the context's next steps
+ * claim resolution, the walks, the chains, and the apply.  pmc_coag_gpu_autotune(ctx, 1) makes the context's next steps
  * (ordinary pmc_coag_gpu_step / _step_batch calls) a coordinate search over
  * those choices: each site in turn tries its PMC_TUNE_CANDIDATES shapes for
  * PMC_TUNE_REPS steps each and keeps the best before moving on.  A shape's
  * score is the device time of the site's launches (CUDA events on the
  * library's stream) per million pair tests of its steps; during the search
- * the later rounds run from the host loop instead of the CUDA graph, so
- * that each launch can be timed.  The search takes PMC_TUNE_SITES *
+ * the steps run from the host loop instead of the CUDA graph, so that each
+ * launch can be timed.  The search takes PMC_TUNE_SITES *
  * PMC_TUNE_CANDIDATES * PMC_TUNE_REPS steps.  The particles do not depend
  * on the shapes or on the loop, so these steps are the caller's own.
  * pmc_coag_gpu_tune_state reports whether the search is still running, the
@@ -296,11 +295,13 @@ int pmc_coag_gpu_get_next_id(pmc_coag_gpu_ctx *ctx, int pop, int64_t *next_id);
 /* PMC_MODE_FP64 (default), PMC_MODE_MIXED or PMC_MODE_REPLAY. */
 int pmc_coag_gpu_set_mode(pmc_coag_gpu_ctx *ctx, int mode);
 
-/* Run the later rounds of a step (every round after the first: retried
- * events, walks of the particles the step made, chains) as one CUDA graph
- * whose loop condition is set on the device (enable = 1, the default), or
- * from a host loop (enable = 0).  Both give the same particles, bit for bit.
- * Rounds with per-particle (accelerated) redo operations use the host loop.
+/* Run a step as one CUDA graph, its later rounds (retried events, walks of
+ * the particles the step made, chains) a loop whose condition is set on the
+ * device (enable = 1, the default), or every launch from the host (enable =
+ * 0).  Both give the same particles, bit for bit.  The first steps of a
+ * population, and a step that outgrows the graph's bounds or changes the
+ * grid, run from the host (their later rounds as a graph where no
+ * per-particle operations run).
  * No counterpart in the reference (an execution choice). */
 int pmc_coag_gpu_set_graphs(pmc_coag_gpu_ctx *ctx, int enable);
 

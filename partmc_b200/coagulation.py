@@ -311,9 +311,8 @@ class AeroState:
         check(_lib.lib().pmc_coag_gpu_set_seed(self.ctx, pop, int(seed)), "pmc_coag_gpu_set_seed")
 
     def set_graphs(self, enable):
-        """The later rounds of a step (retries, walks, chains) as one
-        device-driven CUDA graph (default) or from a host loop; the particles
-        are the same either way."""
+        """A step as one device-driven CUDA graph (default) or launched from
+        the host; the particles are the same either way."""
         check(_lib.lib().pmc_coag_gpu_set_graphs(self.ctx, 1 if enable else 0), "pmc_coag_gpu_set_graphs")
 
     def set_weight(self, aero_weight_array):

@@ -951,7 +951,7 @@ __global__ void k_halve(PopDev P, int g, int c, uint32_t call) {
 // n_bin bins from d_min to d_max, each particle weighted by its number
 // concentration (aero_state_num_concs), per unit log diameter.  out holds
 // n_bin number values, then n_bin x n_spec species masses (kg m^-3).
-// A block takes kDistTile slots at a time and orders them by bin (counts and
+// A block takes TILE slots at a time and orders them by bin (counts and
 // ranks in shared memory).  A warp then goes over 64 of the ordered particles
 // with a lane per species (a particle's volumes are consecutive; HI: over 32
 // species, two a lane), eight particles' loads in flight, and sums a run of
@@ -965,27 +965,56 @@ __global__ void k_halve(PopDev P, int g, int c, uint32_t call) {
 // cluster first: 150 us, the blocks of a cluster wait for their slowest.)
 constexpr int kDistThreads = 512;
 constexpr int kDistTile = 2 * kDistThreads;
-template <bool HI>
+constexpr int kDistFewSpec = 8;
+
+// With at most kDistFewSpec species a thread per particle and its 1 + n_spec
+// atomics are the shorter way: 1e6 slots of 1 and 7 species take 84 and 105 us
+// a call, 123 and 128 in order of bins with a lane per species (most lanes
+// idle); 20 species 226 and 145.
+__global__ void __launch_bounds__(256) k_size_dist_few(PopDev P, int n_bin, double log_lo, double log_hi,
+                                                       double inv_width, double* out) {
+  extern __shared__ double hs[];  // [n_bin * (1 + n_spec)]
+  const int nv = n_bin * (1 + P.n_spec);
+  for (int k = threadIdx.x; k < nv; k += blockDim.x) hs[k] = 0.0;
+  __syncthreads();
+  const int n = P.ctr->n_slots;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    if (!P.alive[i]) continue;
+    const double r = vol2rad(P.benv.frac, P.vtot[i]);  // aero_particle_radius (fractal_vol2rad)
+    const int b = bin_find(n_bin, log_lo, log_hi, 2.0 * r);
+    if (b < 1 || b > n_bin) continue;
+    const double nc = num_conc_at_radius<double>(P.w, P.cls[i] - 1, r) * inv_width;
+    atomicAdd(&hs[b - 1], nc);
+    for (int s = 0; s < P.n_spec; s++)
+      atomicAdd(&hs[n_bin + (b - 1) * P.n_spec + s], nc * P.vol[vol_at(P, i, s)] * P.density[s]);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < nv; k += blockDim.x)
+    if (hs[k] != 0.0) atomicAdd(&out[k], hs[k]);
+}
+
+template <bool HI, int TILE>
 __global__ void __launch_bounds__(kDistThreads) k_size_dist(PopDev P, int n_bin, double log_lo, double log_hi,
                                                             double inv_width, double* out) {
+  constexpr int kPer = TILE / kDistThreads;
   extern __shared__ double hs[];  // [n_bin * (1 + n_spec)] sums, then the ordered slots
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, ns = P.n_spec;
   const int nv = n_bin * (1 + ns);
-  double* s_nc = hs + nv;                  // [kDistTile] number concentration, in bin order
-  int* s_slot = (int*)(s_nc + kDistTile);  // [kDistTile]
-  int* s_bin = s_slot + kDistTile;         // [kDistTile]
-  int* cnt = s_bin + kDistTile;            // [n_bin]
+  double* s_nc = hs + nv;                  // [TILE] number concentration, in bin order
+  int* s_slot = (int*)(s_nc + TILE);  // [TILE]
+  int* s_bin = s_slot + TILE;         // [TILE]
+  int* cnt = s_bin + TILE;            // [n_bin]
   for (int k = threadIdx.x; k < nv; k += blockDim.x) hs[k] = 0.0;
   const double den0 = lane < ns ? P.density[lane] : 0.0, den1 = HI && lane + 32 < ns ? P.density[lane + 32] : 0.0;
   const int n = P.ctr->n_slots;
   const int per = (n_bin + kDistThreads - 1) / kDistThreads;  // bins a thread scans
-  for (long long base = blockIdx.x * (long long)kDistTile; base < n; base += (long long)gridDim.x * kDistTile) {
+  for (long long base = blockIdx.x * (long long)TILE; base < n; base += (long long)gridDim.x * TILE) {
     for (int k = threadIdx.x; k < n_bin; k += blockDim.x) cnt[k] = 0;
     __syncthreads();
-    int b[2] = {0, 0}, rank[2];
-    double nc[2];
+    int b[kPer] = {}, rank[kPer];
+    double nc[kPer];
 #pragma unroll
-    for (int u = 0; u < 2; u++) {
+    for (int u = 0; u < kPer; u++) {
       const long long i = base + u * kDistThreads + threadIdx.x;
       if (!(i < n && P.alive[i])) continue;
       const double r = vol2rad(P.benv.frac, P.vtot[i]);  // aero_particle_radius (fractal_vol2rad)
@@ -1014,7 +1043,7 @@ __global__ void __launch_bounds__(kDistThreads) k_size_dist(PopDev P, int n_bin,
     }
     __syncthreads();
 #pragma unroll
-    for (int u = 0; u < 2; u++)
+    for (int u = 0; u < kPer; u++)
       if (b[u] > 0) {
         const int pos = cnt[b[u] - 1] + rank[u];
         s_slot[pos] = (int)base + u * kDistThreads + (int)threadIdx.x;
@@ -1378,10 +1407,10 @@ constexpr int kTuneCands = 3;
 // candidates per site (within each kernel's __launch_bounds__)
 constexpr int kTuneCand[kTuneSites][kTuneCands] = {
     {64, 128, 256},  // k_test: one pair test per thread
-    {64, 128, 256},  // k_decide and k_resolve_set: one event per thread
+    {64, 128, 256},  // k_resolve: one event per thread
     {64, 128, 256},  // k_items: one walk per thread
     {32, 64, 128},   // k_chain: one chain per thread
-    {64, 128, 256},  // k_apply_move and k_apply_set: one event per thread
+    {64, 128, 256},  // k_apply: one event per thread
 };
 constexpr int kTuneReps = 3;  // steps per candidate
 struct Tune {
@@ -3543,13 +3572,14 @@ struct StepRun {
 };
 
 // Run this step as the graph, if what it relies on holds: a valid sort and
-// current caches and bounds from the steps before, and no target operations
-// in the last one.  d_pops' copies keep their step count on the device
-// (the sort's step_begin adds one), so a step whose parameters are those of the last
-// one pushes nothing.  One read-back, at the end.  The step the long way
-// takes six, with the copies and launches that wait on them: 0.351 ms a step
-// for 1e4 particles under the additive kernel, 0.160 with the graph; 0.860 and
-// 0.689 for 1e6 particles of 20 species.
+// current caches and bounds from the steps before.  d_pops' copies keep their
+// step count on the device (the sort's step_begin adds one), so a step whose
+// parameters are those of the last one pushes nothing.  Its report comes by
+// stores to mapped host memory, without a copy or a synchronisation.  The step
+// the long way makes six read-backs, with the copies and launches that wait on
+// them: 0.351 ms a step for 1e4 particles under the additive kernel, 0.160 with
+// the graph when it came, 0.11 with its kernels as they are now; 0.860, 0.689
+// and 0.59 for 1e6 particles of 20 species.
 StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   StepRun out;
   if (!c.use_graph || c.tuner.on || !c.ctrs_fresh || c.last_w < 0) return out;
@@ -5038,12 +5068,26 @@ int pmc_coag_gpu_size_dist(pmc_coag_gpu_ctx* x, int pop, int n_bin, double d_min
   c.st_d.reserve(nv);
   CK(cudaMemsetAsync(c.st_d.p, 0, sizeof(double) * nv, c.stream));
   PopCtr r = read_ctr(c, pop);
-  if (r.n_slots > 0) {
-    const size_t smem = sizeof(double) * nv + kDistTile * (sizeof(double) + 2 * sizeof(int)) + sizeof(int) * n_bin;
-    auto k = c.n_spec > 32 ? k_size_dist<true> : k_size_dist<false>;
+  if (r.n_slots > 0 && c.n_spec <= kDistFewSpec) {
+    const size_t smem = sizeof(double) * nv;
+    if (smem > 48 * 1024)
+      CK(cudaFuncSetAttribute(k_size_dist_few, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_size_dist_few<<<std::min(grid_for(r.n_slots, 256), c.n_sm * 4), 256, smem, c.stream>>>(
+        ph.h, n_bin, log(d_min), log(d_max), (double)n_bin / (log(d_max) - log(d_min)), c.st_d.p);
+    note_launch();
+  } else if (r.n_slots > 0) {
+    // half tiles while two blocks an SM take them all: the call takes 63 us for
+    // 15,838 slots of 20 species (75 with whole tiles, too few blocks) and 65 for
+    // 120,000 (75); from 250,000 slots on, whole tiles are as fast or faster (76
+    // against 78; 138 against 150 for 1e6)
+    const bool half = r.n_slots <= 2LL * c.n_sm * (kDistTile / 2);
+    const int tile = half ? kDistTile / 2 : kDistTile;
+    const size_t smem = sizeof(double) * nv + tile * (sizeof(double) + 2 * sizeof(int)) + sizeof(int) * n_bin;
+    auto k = c.n_spec > 32 ? (half ? k_size_dist<true, kDistTile / 2> : k_size_dist<true, kDistTile>)
+                           : (half ? k_size_dist<false, kDistTile / 2> : k_size_dist<false, kDistTile>);
     if (smem > 48 * 1024) CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(4, (220 * 1024) / (smem + 1024)));
-    const long long tiles = (r.n_slots + kDistTile - 1) / kDistTile;
+    const long long tiles = (r.n_slots + tile - 1) / tile;
     k<<<(unsigned)std::min<long long>(tiles, (long long)c.n_sm * per_sm), kDistThreads, smem, c.stream>>>(
         ph.h, n_bin, log(d_min), log(d_max), (double)n_bin / (log(d_max) - log(d_min)), c.st_d.p);
     note_launch();

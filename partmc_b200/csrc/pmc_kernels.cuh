@@ -885,7 +885,7 @@ __device__ __forceinline__ Rng merge_rng(const PopDev& P, unsigned long long key
 // Per-set pair tests (maybe_coag_pair, coagulation.F90:712-759).  One thread
 // per sample w of the flattened (population, pair, sample) space; an
 // accepted sample records its slots and global pair.  Its merge decision is
-// drawn after the compaction (k_decide), so the FP64 decisions run in full
+// drawn in the compaction (k_compact_samples), so the FP64 decisions run in full
 // warps instead of in the few accepting lanes of each warp of tests.
 template <int KT, class T, bool FLAT>
 __global__ void __launch_bounds__(256) k_test(const PopDev* pops, const int* gpair_pop,

@@ -2,7 +2,7 @@
 //
 // Per-set events: coagulate_weighting + coagulate (coagulation.F90:810-985).
 // Per-particle (accelerated) path: sample_source_particle +
-// coag_target_with_source (coagulation.F90:333-582), one thread per target.
+// coag_target_with_source (coagulation.F90:333-582), one warp per target.
 // Every write to a particle slot is guarded by the slot's claim word: an
 // event or target operation is applied only if it holds the lowest priority
 // on every slot it writes or removes; otherwise it is retried (or dropped,
@@ -1353,7 +1353,7 @@ __global__ void __launch_bounds__(kChainThreads, 4) k_chain(ItemArgs A, ChainPoo
 // ev_app[e] events in order, each a coagulate (coagulation.F90:928-985) of
 // the walking particle with the next partner, with the merge decision
 // recomputed from the values and the stream the walk used.  One warp per
-// chain of the round's list (chain_list, filled by k_resolve_set); a chain's entries
+// chain of the round's list (chain_list, filled by k_resolve); a chain's entries
 // are taken a pool chunk at a time (kBatch events):
 //   1. lane k loads event k's partner (slot, pair, radius, scalar fields,
 //      species volumes) into shared memory;
