@@ -5325,7 +5325,9 @@ int pmc_coag_gpu_set_seed(pmc_coag_gpu_ctx* x, int pop, uint64_t seed) {
   PopHost& ph = x->c.pops[pop];
   ph.seed = seed;
   ph.h.seed = seed;
-  ph.step = 0;  // the population's streams start again at step 1
+  // the population's streams start again at step 1; a step graph counts on
+  // from the device's copy, which any call before the step may push
+  ph.step = ph.h.step = 0;
   x->c.dirty = true;
   return PMC_OK;
 }
