@@ -2754,7 +2754,7 @@ int replay_step_host(Ctx& c, long long* s_out, long long* k_out) {
   }
   ph.valid_sort = true;
   int nb = std::max(ph.n_bin, 1);
-  if (!replay_reserve(rb, ph.h.cap, nb * c.n_class, c.n_group * c.n_class, nb, c.n_class, c.n_group))
+  if (!replay_reserve(rb, ph.h.cap, nb * c.n_class, c.n_group * c.n_class, nb, c.n_class, c.n_group, c.stream))
     return PMC_ERR_CAPACITY;
   if (rb.n_cells != nb * c.n_class || !rb.valid) rebuild = true;
   push_pops(c);
@@ -4137,12 +4137,15 @@ static int do_init(int n_pop, int n_spec, const double* density, int i_water, in
   CK(cudaMalloc(&c.d_stat, sizeof(long long) * kStatWords + sizeof(PopCtr) * n_pop + 16));  // read in 16-byte words
   c.d_ctrs = (PopCtr*)(c.d_stat + kStatWords);
   CK(cudaMalloc(&c.d_round, 2 * sizeof(uint32_t)));  // round of the step, claim generation
-  CK(cudaMemset(c.d_round, 0, 2 * sizeof(uint32_t)));
+  // cleared in the order of the context's own stream, which does not wait for
+  // the default one: a clear queued there behind the caller's work would come
+  // after the first uploads
+  CK(cudaMemsetAsync(c.d_round, 0, 2 * sizeof(uint32_t), c.stream));
   c.scan_ctr.reserve(2 * kScanMaxJobs);  // tile counters, then finished-block counters
-  CK(cudaMemset(c.scan_ctr.p, 0, sizeof(unsigned) * c.scan_ctr.n));
+  CK(cudaMemsetAsync(c.scan_ctr.p, 0, sizeof(unsigned) * c.scan_ctr.n, c.stream));
   c.scan_err.reserve(1);
-  CK(cudaMemset(c.scan_err.p, 0, sizeof(unsigned long long) * c.scan_err.n));
-  CK(cudaMemset(c.d_ctrs, 0, sizeof(PopCtr) * n_pop));
+  CK(cudaMemsetAsync(c.scan_err.p, 0, sizeof(unsigned long long) * c.scan_err.n, c.stream));
+  CK(cudaMemsetAsync(c.d_ctrs, 0, sizeof(PopCtr) * n_pop, c.stream));
   for (int k = 0; k < n_pop; k++) {
     c.pops[k].seed = seeds ? seeds[k] : (uint64_t)(k + 1);
     init_pop(c, c.pops[k], 1024);
@@ -5350,7 +5353,10 @@ int pmc_coag_gpu_replay_set(pmc_coag_gpu_ctx* x, const double* u, int64_t n) {
   Ctx& c = x->c;
   GUARD_BEGIN
   c.replay_u.reserve((size_t)std::max<int64_t>(n, 1));
-  if (n > 0) CK(cudaMemcpy(c.replay_u.p, u, sizeof(double) * n, cudaMemcpyHostToDevice));
+  if (n > 0) {
+    CK(cudaMemcpyAsync(c.replay_u.p, u, sizeof(double) * n, cudaMemcpyHostToDevice, c.stream));
+    CK(cudaStreamSynchronize(c.stream));
+  }
   c.replay_n = n;
   c.replay_used = 0;
   return PMC_OK;

@@ -641,7 +641,7 @@ __global__ void k_replay_counts(RMapDev m, int* out) {
 }  // namespace
 
 bool replay_reserve(ReplayBuffers& rb, int cap, int n_cells, int n_gc, int n_bin, int n_class,
-                    int n_group) {
+                    int n_group, cudaStream_t stream) {
   size_t ints = 0;
   auto rm_ints = [&](int nc) { return (size_t)3 * cap + (size_t)nc + (size_t)nc * cap + 1; };
   ints = rm_ints(n_cells) + rm_ints(n_gc) + 8;
@@ -652,7 +652,7 @@ bool replay_reserve(ReplayBuffers& rb, int cap, int n_cells, int n_gc, int n_bin
     rb.mem = nullptr;
     return false;
   }
-  cudaMemset(rb.mem, 0, bytes);
+  cudaMemsetAsync(rb.mem, 0, bytes, stream);
   rb.bytes = bytes;
   rb.cap = cap;
   rb.n_cells = n_cells;

@@ -53,7 +53,7 @@ struct ReplayBuffers {
 // allocate (or keep) buffers for capacity cap and grids of n_cells size
 // cells and n_gc group cells; returns false on allocation failure
 bool replay_reserve(ReplayBuffers& rb, int cap, int n_cells, int n_gc, int n_bin, int n_class,
-                    int n_group);
+                    int n_group, cudaStream_t stream);
 void replay_free(ReplayBuffers& rb);
 // launch the single-thread replay of one mc_coag call on population `pop`
 void replay_launch(const PopDev* d_pops, int pop, const ReplayDev& rd, cudaStream_t stream);
