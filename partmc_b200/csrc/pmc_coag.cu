@@ -2937,17 +2937,19 @@ __global__ void k_pp_fits(const long long* rm_tot, long long pool, long long* st
 // occupied bins), the samples and target operations (none in a graph without
 // them) and their removals fit the buffers, every population's walks stop at
 // per-particle pairs exactly if it has target operations, and it has room for
-// a particle per sample and the copies.  If not, the totals are set to zero,
-// so the rest of the graph does nothing and the host runs the step the long
-// way.
-enum : long long { kNoGoGrid = 1, kNoGoOps = 2, kNoGoSamples = 4, kNoGoSlots = 8, kNoGoStops = 16, kNoGoPool = 32 };
+// a particle per sample and the copies, and no scan gave up (its offsets would
+// be wrong).  If not, the totals are set to zero, so the rest of the graph does
+// nothing and the host runs the step the long way, which reports such a scan
+// before a particle has changed.
+enum : long long { kNoGoGrid = 1, kNoGoOps = 2, kNoGoSamples = 4, kNoGoSlots = 8, kNoGoStops = 16, kNoGoPool = 32, kNoGoScan = 64 };
 
 __global__ void k_step_check(const PopDev* pops, int n_pop, const long long* pop_pair_base, long long* work_off,
                              long long* pp_off, int n_gp, long long w_cap, long long q_cap, const long long* rm_tot,
-                             long long pool, long long sort_slots, long long* n_dev, long long* stat) {
+                             long long pool, long long sort_slots, long long* n_dev, long long* stat,
+                             const unsigned long long* scan_err) {
   chain_wait();
   const long long W = work_off[n_gp], Q = pp_off[n_gp];
-  long long why = 0;
+  long long why = *scan_err ? kNoGoScan : 0;
   if (Q > q_cap) why |= kNoGoOps;
   if (W > w_cap) why |= kNoGoSamples;
   if (Q > 0 && q_cap > 0 && *rm_tot + 1 > pool) why |= kNoGoPool;
@@ -3487,7 +3489,7 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
       launch_pp_count(c, q_cap, c.pp_off.p + n_gp, st);
     }
     launch_chained(c, k_step_check, dim3(1), dim3(256), 0, st, c.d_pops, c.n_pop, c.pop_pair_base.p, c.work_off.p, c.pp_off.p, n_gp, w_cap, q_cap,
-                                    c.pp_rm_tot.p, (long long)c.pp_rm_pool.n, sort_slots, c.n_dev.p, c.d_stat);
+                                    c.pp_rm_tot.p, (long long)c.pp_rm_pool.n, sort_slots, c.n_dev.p, c.d_stat, c.scan_err.p);
     if (q_cap > 0) launch_pp_ops(c, b.kt, q_cap, st);
     mark(2);
     launch_test_kt(c, b.kt, b.flat, n_gp, w_cap, st);
@@ -4442,6 +4444,16 @@ static int finish_step(Ctx& c, long long* samp, long long* coag) {
   return status;
 }
 
+// After a step that an error ended: the host does not know how far the device
+// came, so the next step reads the counters, copies the populations to the
+// device, and restarts the claim generations (a word of a round that the host
+// did not count would win against the next step's).
+static void step_left(Ctx& c) {
+  c.ctrs_fresh = false;
+  c.dirty = true;
+  c.claim_gen = kGenLimit;
+}
+
 // the autotuner around one step: the candidate's shape before it; after it
 // (finish_step has synchronised the stream) the device time of the site's
 // launches and the step's pair tests
@@ -4558,8 +4570,13 @@ int pmc_coag_gpu_step_batch(pmc_coag_gpu_ctx* x, int kernel_type, const double* 
       ProfScope ps(c, 3, 1);
       c.replay.valid = false;  // the parallel step reorders and rewrites slots
       if (c.tuner.on) tune_before(c);
-      step_parallel(c, kernel_type, params_same);
-      status = finish_step(c, &s, &k);
+      try {
+        step_parallel(c, kernel_type, params_same);
+        status = finish_step(c, &s, &k);
+      } catch (...) {
+        step_left(c);
+        throw;
+      }
       if (c.tuner.on && status == 0) tune_after(c, s);
     }
     S += s;
@@ -5339,6 +5356,19 @@ int pmc_coag_gpu_set_graphs(pmc_coag_gpu_ctx* x, int enable) {
   if (!x || (enable != 0 && enable != 1)) return PMC_ERR_INVALID_ARG;
   x->c.use_graph = enable == 1;
   return PMC_OK;
+}
+
+// For the tests, not in the header: the next step finds a look-back that gave
+// up, as check_scan_err and the step's own checks would after a real one.
+int pmc_coag_gpu_test_scan_give_up(pmc_coag_gpu_ctx* x) {
+  if (!x) return PMC_ERR_INVALID_ARG;
+  Ctx& c = x->c;
+  GUARD_BEGIN
+  const unsigned long long one = 1ULL;
+  CK(cudaMemcpyAsync(c.scan_err.p, &one, sizeof(one), cudaMemcpyHostToDevice, c.stream));
+  CK(cudaStreamSynchronize(c.stream));
+  return PMC_OK;
+  GUARD_END
 }
 
 int pmc_coag_gpu_set_mode(pmc_coag_gpu_ctx* x, int mode) {
