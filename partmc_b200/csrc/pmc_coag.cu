@@ -1536,7 +1536,8 @@ struct Ctx {
   // round's k_items; their count is round_dev[5]
   DevBuf<int> ppw_slot, ppw_gp;  // read by a round's k_items, then written by its k_compact_walkers
   long long op_cap = 0;   // room in the target-operation arrays this round
-  bool pp_step = false;   // the step has target operations (per-particle path)
+  bool pp_step = false;   // the step has target operations (per-particle path), or one of the last kPPIdle had
+  int pp_idle = 0;        // graph steps since one that had
   // chain events of a round (ChainPool), in chunks
   DevBuf<int> ch_y, ch_q;
   DevBuf<float> ch_pos;
@@ -2935,15 +2936,16 @@ __global__ void k_pp_fits(const long long* rm_tot, long long pool, long long* st
 // WHILE node.  What round 0 needed the host for is checked on the device
 // (k_step_check): the grid is kept (aero_sorted_remake_if_needed's rule on the
 // occupied bins), the samples and target operations (none in a graph without
-// them) and their removals fit the buffers, every population's walks stop at
-// per-particle pairs exactly if it has target operations, and it has room for
-// a particle per sample and the copies, and no scan gave up (its offsets would
+// them) and their removals fit the buffers, every population has room for a
+// particle per sample and the copies, and no scan gave up (its offsets would
 // be wrong).  If not, the totals are set to zero, so the rest of the graph does
 // nothing and the host runs the step the long way, which reports such a scan
-// before a particle has changed.
-enum : long long { kNoGoGrid = 1, kNoGoOps = 2, kNoGoSamples = 4, kNoGoSlots = 8, kNoGoStops = 16, kNoGoPool = 32, kNoGoScan = 64 };
+// before a particle has changed.  A population's walks stop at per-particle
+// pairs if it has target operations in this step; that is set here too, so a
+// population whose operations come and go does not send the step the long way.
+enum : long long { kNoGoGrid = 1, kNoGoOps = 2, kNoGoSamples = 4, kNoGoSlots = 8, kNoGoPool = 16, kNoGoScan = 32 };
 
-__global__ void k_step_check(const PopDev* pops, int n_pop, const long long* pop_pair_base, long long* work_off,
+__global__ void k_step_check(PopDev* pops, int n_pop, const long long* pop_pair_base, long long* work_off,
                              long long* pp_off, int n_gp, long long w_cap, long long q_cap, const long long* rm_tot,
                              long long pool, long long sort_slots, long long* n_dev, long long* stat,
                              const unsigned long long* scan_err) {
@@ -2954,9 +2956,9 @@ __global__ void k_step_check(const PopDev* pops, int n_pop, const long long* pop
   if (W > w_cap) why |= kNoGoSamples;
   if (Q > 0 && q_cap > 0 && *rm_tot + 1 > pool) why |= kNoGoPool;
   for (int k = threadIdx.x; k < n_pop; k += blockDim.x) {
-    const PopDev& P = pops[k];
+    PopDev& P = pops[k];
     const GridDev& G = *P.grid;
-    const PopCtr& r = *P.ctr;
+    PopCtr& r = *P.ctr;
     if (G.n_bin >= 1) {
       const double gmin = G.edges[0], gmax = G.edges[G.n_bin];
       const double rmin = r.bmax < 0 ? gmax : G.edges[r.bmin], rmax = r.bmax < 0 ? gmin : G.edges[r.bmax + 1];
@@ -2966,7 +2968,7 @@ __global__ void k_step_check(const PopDev* pops, int n_pop, const long long* pop
     }
     const long long a = pop_pair_base[k], b = pop_pair_base[k + 1];
     const long long Wk = work_off[b] - work_off[a], Qk = pp_off[b] - pp_off[a];
-    if ((Qk > 0) != (P.walk_stops != 0)) why |= kNoGoStops;
+    P.walk_stops = r.walk_stops = Qk > 0 ? 1 : 0;
     const long long need = (long long)r.n_slots + Wk + (kMaxCopies - 1) * Qk;
     if (need > (long long)P.cap || (long long)r.n_slots > sort_slots) why |= kNoGoSlots;
   }
@@ -3563,6 +3565,8 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
   CK(cudaGraphInstantiate(&c.sg_exec, c.sg_graph, 0));
 }
 
+constexpr int kPPIdle = 8;  // steps
+
 struct StepRun {
   bool ran = false;   // round 0 ran on the device
   // 1: work is left, the host loop carries on after `rounds` rounds; 2: also
@@ -3708,7 +3712,9 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   long long stat[kStatWords];
   memcpy(stat, report, sizeof(stat));
   c.last_w = stat[5];
-  c.last_q = stat[12];
+  // target operations may come and go from step to step: their bounds follow
+  // a fall by an eighth a step, a rise at once
+  c.last_q = std::max(stat[12], c.last_q - c.last_q / 8);
   c.last_rm = std::max(c.last_rm, stat[11]);
   if (stat[4]) {
     c.ctrs_fresh = false;
@@ -3734,7 +3740,11 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   g_launches += c.sg_nodes0 + c.sg_nodes * (stat[2] - 1);
   c.claim_gen += (uint32_t)(stat[2] + (stat[3] == 2 ? 1 : 0));  // a round left in the middle has begun
   c.last_e0 = stat[7];
-  c.last_qb = stat[8];
+  c.last_qb = std::max(stat[8], c.last_qb - c.last_qb / 8);
+  for (int k = 0; k < c.n_pop; k++) c.pops[k].h.walk_stops = c.h_ctrs[k].walk_stops;
+  // without target operations for a while, back to the graph without them
+  c.pp_idle = stat[12] > 0 ? 0 : c.pp_idle + 1;
+  if (c.pp_idle >= kPPIdle && !stat[3]) c.pp_step = false;
   out.ran = true;
   out.rounds = stat[2];
   out.losers = stat[0];
@@ -3882,6 +3892,7 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
     // a population's walks stop when it has target operations of its own,
     // so it steps the same alone and in a batch
     c.pp_step = Q > 0;
+    c.pp_idle = 0;
     for (int k = 0; k < c.n_pop; k++) {
       const int stops = hw[3 + 2 * k + 1] > 0 ? 1 : 0;
       if (c.pops[k].h.walk_stops != stops) {

@@ -118,7 +118,7 @@ struct PopCtr {
   long long exact_tests;   // FP32 pair tests decided in FP64 (f32_decides), since the context was made
   long long n_removed;     // removal records appended since the host last read them
   int cap_site;            // first capacity limit a kernel hit (kCap*), 0 if none
-  int cap_pad;
+  int walk_stops;          // the population's PopDev::walk_stops in the last step run as a graph
 };
 
 // sites of the device capacity limits (PopCtr::cap_site)
