@@ -3697,9 +3697,16 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   c.report_count++;
   {
     // the report's sequence number; a look at the stream now and then, for an
-    // error or a graph that ended without it
+    // error or a graph that ended without it.  The wait spins, unless the
+    // process chose another (cudaSetDeviceFlags), as a stream synchronisation
+    // would
     const volatile unsigned* flag = (const volatile unsigned*)((const char*)c.report.p + 16 * (size_t)report_words(c));
+    unsigned sched = 0;
+    CK(cudaGetDeviceFlags(&sched));
+    sched &= cudaDeviceScheduleMask;
+    if (sched == cudaDeviceScheduleBlockingSync) CK(cudaStreamSynchronize(c.stream));
     for (long long spins = 1; *flag != c.report_count; spins++) {
+      if (sched == cudaDeviceScheduleYield) std::this_thread::yield();
       if (spins % 4096 != 0) continue;
       const cudaError_t e = cudaStreamQuery(c.stream);
       if (e == cudaErrorNotReady) continue;
