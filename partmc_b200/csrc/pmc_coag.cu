@@ -1475,6 +1475,7 @@ struct Ctx {
   cudaGraphExec_t rg_exec = nullptr;
   std::vector<long long> rg_key;
   std::vector<long long> rg_seen;  // the key of the previous step's later rounds
+  int rg_held = 0;                 // steps in a row that had it
   long long rg_nodes = 0, rg_builds = 0;
   DevBuf<long long> graph_stats;
   // the whole step as one graph (run_step_graph)
@@ -1607,13 +1608,22 @@ struct Ctx {
 // of 256; from the pool 3.3 and 0.4 ms.
 // One pool per device, shared by its contexts (the driver orders memory that
 // moves between their streams; a pool per context took 1 ms to create); it
-// keeps at most kPoolKeep bytes that are not in use past a synchronisation,
-// and the last context to go destroys it.
-constexpr uint64_t kPoolKeep = 4ULL << 30;
+// keeps at most kPoolKeep bytes that are not in use past a synchronisation
+// (a cudaMalloc of the process that would fail gets them: measured with 1 GiB
+// on a device with 49 MiB free), and the last context to go gives back all but
+// kPoolIdle.  For the process stay the pool itself with its first block (its
+// unit is 32 MiB), and one page of page-locked memory: the first such
+// allocation of a process maps a block that later small ones share (1 to 3 ms,
+// then 5 us each), and freeing the last unmaps it.  A program that makes a
+// context for each job paid for both every time: 6.8 ms for a context that
+// takes 1000 particles through 3 steps, now 3.6 (4.1 with nothing kept of the
+// pool; 3.5 with cudaMalloc and cudaFree).
+constexpr uint64_t kPoolKeep = 4ULL << 30, kPoolIdle = 32ULL << 20;
 
 struct DevicePools {
   std::mutex mu;
   std::vector<std::pair<cudaMemPool_t, int>> by_dev;  // pool, contexts
+  void* page = nullptr;  // page-locked
 };
 DevicePools& device_pools() {
   static DevicePools* p = new DevicePools();  // lives until the process ends: contexts may be destroyed at exit
@@ -1624,6 +1634,7 @@ cudaMemPool_t pool_acquire(int dev) {
   DevicePools& d = device_pools();
   std::lock_guard<std::mutex> l(d.mu);
   if ((int)d.by_dev.size() <= dev) d.by_dev.resize(dev + 1, {nullptr, 0});
+  if (!d.page) CK(cudaHostAlloc(&d.page, 4096, cudaHostAllocMapped));
   auto& e = d.by_dev[dev];
   if (!e.first) {
     cudaMemPoolProps mp = {};
@@ -1643,10 +1654,7 @@ void pool_release(int dev) {
   DevicePools& d = device_pools();
   std::lock_guard<std::mutex> l(d.mu);
   auto& e = d.by_dev[dev];
-  if (--e.second == 0) {
-    cudaMemPoolDestroy(e.first);
-    e.first = nullptr;
-  }
+  if (--e.second == 0) cudaMemPoolTrimTo(e.first, kPoolIdle);
 }
 
 void free_list(Ctx& c, std::vector<void*>& v) {
@@ -3211,9 +3219,9 @@ void free_redraw_graph(Ctx& c) {
 }
 
 // the item and event bound of the later rounds' graph for round-0 events
-// e0: a power of two, at least 4096, so that it holds from step to step
-long long graph_bound(long long e0) {
-  long long w = 4096;
+// e0: a power of two, at least `least`, so that it holds from step to step
+long long graph_bound(long long e0, long long least = 4096) {
+  long long w = least;
   while (w < e0) w *= 2;
   return w;
 }
@@ -3264,7 +3272,9 @@ struct GraphRun {
 };
 
 // Run the later rounds of this step as the graph (captured again when a
-// bound or an address changed and the change held for two steps in a row).
+// bound or an address changed and the change held for three steps in a row:
+// after two, the next step is a graph as a whole, unless the program's own
+// calls between steps keep it from that).
 // e0: the events of the round before.
 GraphRun run_round_graph(Ctx& c, int kt, bool flat, int n_gpairs, long long e0) {
   GraphRun out;
@@ -3302,11 +3312,12 @@ GraphRun run_round_graph(Ctx& c, int kt, bool flat, int n_gpairs, long long e0) 
   }
   if (c.dirty) push_pops(c);
   std::vector<long long> key = round_graph_key(c, b);
-  if (key != c.rg_key && key != c.rg_seen) {
-    // bounds or addresses new since the last step: capturing pays only when
+  if (key != c.rg_key) {
+    // bounds or addresses new since the last steps: capturing pays only when
     // they hold, so this step's later rounds run from the host loop
+    c.rg_held = key == c.rg_seen ? c.rg_held + 1 : 1;
     c.rg_seen = key;
-    return out;
+    if (c.rg_held < 3) return out;
   }
   if (key != c.rg_key) {
     free_redraw_graph(c);
@@ -3566,6 +3577,9 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
 }
 
 constexpr int kPPIdle = 8;  // steps
+// least bound of a step's target operations: their buffers take 2 KB an
+// operation with the copies and walkers they may make
+constexpr long long kLeastOps = 512;
 
 struct StepRun {
   bool ran = false;   // round 0 ran on the device
@@ -3614,7 +3628,7 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   long long q_cap = 0, qb_cap = 0;
   if (c.pp_step) {
     // room for twice as many when they outgrow it
-    const long long q = graph_bound(c.last_q + c.last_q / 4), qb = graph_bound(c.last_qb + c.last_qb / 4);
+    const long long q = graph_bound(c.last_q + c.last_q / 4, kLeastOps), qb = graph_bound(c.last_qb + c.last_qb / 4, kLeastOps);
     if (q > c.sg_q || 16 * q <= c.sg_q) c.sg_q = 2 * q;
     if (qb > c.sg_qb || 16 * qb <= c.sg_qb) c.sg_qb = 2 * qb;
     q_cap = c.sg_q;
