@@ -1378,6 +1378,7 @@ struct PopHost {
   std::vector<void*> fixed_allocs;
   uint64_t seed = 1;
   uint32_t step = 0;
+  uint32_t dev_step = 0;  // the step count of the device's copy of h
   int kmax_kt = 0;  // kernel type of the current k_max table
   bool own_w = false;  // weights set for this population alone
   // host copy kept slot by slot (pmc_coag_gpu_sync_host): refreshed in full
@@ -1858,6 +1859,7 @@ void push_pops(Ctx& c) {
     v[k] = c.pops[k].h;
     v[k].round_p = c.d_round;
     v[k].gen_p = c.d_round + 1;
+    c.pops[k].dev_step = v[k].step;
   }
   CK(cudaMemcpyAsync(c.d_pops, v.data(), sizeof(PopDev) * c.n_pop, cudaMemcpyHostToDevice, c.stream));
   c.dirty = false;
@@ -3701,13 +3703,18 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
     capture_step_graph(c, b, c.sg_w, max_pairs, q_cap, qb_cap);
     c.sg_key = key;
   }
-  if (c.dirty || !params_same) {
-    // the sort's step_begin advances the step
+  // the sort's step_begin advances the device's step counts, which have to be
+  // at the step before (a new seed restarts the host's; any call may have
+  // copied the population since)
+  bool counts = true;
+  for (const auto& ph : c.pops) counts = counts && ph.dev_step + 1u == ph.h.step;
+  if (c.dirty || !params_same || !counts) {
     for (auto& ph : c.pops) ph.h.step -= 1u;
     push_pops(c);
     for (auto& ph : c.pops) ph.h.step += 1u;
   }
   CK(cudaGraphLaunch(c.sg_exec, c.stream));
+  for (auto& ph : c.pops) ph.dev_step++;
   c.report_count++;
   {
     // the report's sequence number; a look at the stream now and then, for an
@@ -5377,9 +5384,7 @@ int pmc_coag_gpu_set_seed(pmc_coag_gpu_ctx* x, int pop, uint64_t seed) {
   PopHost& ph = x->c.pops[pop];
   ph.seed = seed;
   ph.h.seed = seed;
-  // the population's streams start again at step 1; a step graph counts on
-  // from the device's copy, which any call before the step may push
-  ph.step = ph.h.step = 0;
+  ph.step = 0;  // the population's streams start again at step 1
   x->c.dirty = true;
   return PMC_OK;
 }
