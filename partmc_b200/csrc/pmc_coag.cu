@@ -1371,7 +1371,6 @@ struct PopHost {
   bool valid_sort = false;
   int n_bin = 0;
   std::vector<double> edges, centers;
-  std::vector<PairDesc> pair_desc;
   // owned allocations (freed on relayout / destroy)
   std::vector<void*> slot_allocs;
   std::vector<void*> sort_allocs;
@@ -1786,6 +1785,16 @@ struct ScanArg {
   long long* total_out = nullptr;
 };
 
+// room for n look-back words; fresh memory is cleared once
+void reserve_scan_status(Ctx& c, size_t n, cudaStream_t st) {
+  if (n > c.scan_status.n) c.scan_status_n = 0;  // also if this fails
+  c.scan_status.reserve(n);
+  if (c.scan_status.n > c.scan_status_n) {
+    CK(cudaMemsetAsync(c.scan_status.p, 0, sizeof(unsigned long long) * c.scan_status.n, st));
+    c.scan_status_n = c.scan_status.n;
+  }
+}
+
 template <class T>
 void scan_multi(Ctx& c, std::initializer_list<ScanArg<T>> args, cudaStream_t st = nullptr) {
   if (!st) st = c.stream;
@@ -1803,11 +1812,7 @@ void scan_multi(Ctx& c, std::initializer_list<ScanArg<T>> args, cudaStream_t st 
   }
   if (k == 0) return;
   if (nb > (1LL << 30)) cap_throw("scan longer than its tile limit");
-  c.scan_status.reserve((size_t)kScanMaxJobs * nb);
-  if (c.scan_status.n > c.scan_status_n) {  // fresh memory: clear it once
-    CK(cudaMemsetAsync(c.scan_status.p, 0, sizeof(unsigned long long) * c.scan_status.n, st));
-    c.scan_status_n = c.scan_status.n;
-  }
+  reserve_scan_status(c, (size_t)kScanMaxJobs * nb, st);
   dim3 g((unsigned)nb, (unsigned)k);
   launch_chained(c, k_scan_lb<T>, g, dim3(kScanThreads), 0, st, jobs, c.scan_status.p, (int)nb, c.scan_ctr.p,
                  c.scan_ctr.p + kScanMaxJobs, c.scan_err.p);
@@ -1818,11 +1823,7 @@ long long compact_tiles(long long n) { return std::max<long long>(1, (n + kCompa
 // shared words of a tiled launch of at most `tiles` blocks
 TileCtl tile_ctl(Ctx& c, long long tiles, cudaStream_t st) {
   if (tiles > (1LL << 30)) cap_throw("scan longer than its tile limit");
-  c.scan_status.reserve((size_t)std::max<long long>(tiles, 1));
-  if (c.scan_status.n > c.scan_status_n) {  // fresh memory: clear it once
-    CK(cudaMemsetAsync(c.scan_status.p, 0, sizeof(unsigned long long) * c.scan_status.n, st));
-    c.scan_status_n = c.scan_status.n;
-  }
+  reserve_scan_status(c, (size_t)std::max<long long>(tiles, 1), st);
   return TileCtl{c.scan_status.p, c.scan_ctr.p, c.scan_ctr.p + kScanMaxJobs, c.scan_err.p};
 }
 
@@ -1892,10 +1893,9 @@ void write_ctr(Ctx& c, int k, const PopCtr& r) {
   CK(cudaStreamSynchronize(c.stream));
 }
 
-// allocate the slot arrays of a population with capacity cap
-void alloc_slots(Ctx& c, PopHost& ph, int cap) {
-  PopDev& h = ph.h;
-  std::vector<void*>& o = ph.slot_allocs;
+// allocate slot arrays of capacity cap into h, owned by o: all of them, or an
+// error and none
+void alloc_slots(Ctx& c, PopDev& h, std::vector<void*>& o, int cap) try {
   h.cap = cap;
   h.vol = dalloc<double>(c, o, (size_t)cap * c.n_spec);
   h.vtot = dalloc<double>(c, o, cap);
@@ -1930,41 +1930,40 @@ void alloc_slots(Ctx& c, PopHost& ph, int cap) {
   CK(cudaMemsetAsync(h.rclaim, 0xff, sizeof(unsigned long long) * cap, c.stream));
   CK(cudaMemsetAsync(h.touched, 0xff, sizeof(uint32_t) * cap, c.stream));        // no generation
   c.dirty = true;
+} catch (...) {
+  free_list(c, o);
+  throw;
 }
 
-// sort structures that depend on the grid and the slot count
-void alloc_sort(Ctx& c, PopHost& ph) {
-  PopDev& h = ph.h;
-  free_list(c, ph.sort_allocs);
-  std::vector<void*>& o = ph.sort_allocs;
-  int nb = std::max(ph.n_bin, 1);
+// sort structures of a grid of n_bin bins into h, owned by o
+void fill_sort(Ctx& c, PopDev& h, std::vector<void*>& o, int n_bin) {
+  int nb = std::max(n_bin, 1);
   h.n_cells = nb * c.n_class;
-  ph.chunk_hist_cap = 0;  // reallocated by the sort when needed
-  h.chunk_hist = nullptr;
+  h.chunk_hist = nullptr;  // allocated by the sort when needed
   h.chunk_hist_len = 0;
   h.cell_count = dalloc<int>(c, o, h.n_cells);
   h.cell_start = dalloc<int>(c, o, h.n_cells + 1);
   h.kmax_tab = dalloc<double>(c, o, (size_t)nb * nb);
   // pairs in the reference's loop order (coagulation.F90:74-94)
-  ph.pair_desc.clear();
+  std::vector<PairDesc> pair_desc;
   for (int c1 = 0; c1 < c.n_class; c1++)
     for (int c2 = 0; c2 <= c1; c2++)
-      for (int b1 = 0; b1 < ph.n_bin; b1++)
-        for (int b2 = (c1 == c2 ? b1 : 0); b2 < ph.n_bin; b2++) {
+      for (int b1 = 0; b1 < n_bin; b1++)
+        for (int b2 = (c1 == c2 ? b1 : 0); b2 < n_bin; b2++) {
           PairDesc d;
           d.b1 = (int16_t)b1;
           d.b2 = (int16_t)b2;
           d.c1 = (int8_t)c1;
           d.c2 = (int8_t)c2;
           d.pad0 = d.pad1 = 0;
-          ph.pair_desc.push_back(d);
+          pair_desc.push_back(d);
         }
-  h.n_pairs = (int)ph.pair_desc.size();
+  h.n_pairs = (int)pair_desc.size();
   if (h.n_pairs >= (1 << 20)) cap_throw("more than 2^20 bin pairs");  // pair numbers in keys and random streams
   // the pairs of each cell in loop order, for walks
   {
     std::vector<int> off(h.n_cells + 1, 0), list;
-    for (const PairDesc& d : ph.pair_desc) {
+    for (const PairDesc& d : pair_desc) {
       off[d.b1 + nb * d.c1 + 1]++;
       if (d.b2 + nb * d.c2 != d.b1 + nb * d.c1) off[d.b2 + nb * d.c2 + 1]++;
     }
@@ -1972,7 +1971,7 @@ void alloc_sort(Ctx& c, PopHost& ph) {
     list.assign(std::max(off[h.n_cells], 1), 0);
     std::vector<int> fill(off.begin(), off.end() - 1);
     for (int p = 0; p < h.n_pairs; p++) {
-      const PairDesc& d = ph.pair_desc[p];
+      const PairDesc& d = pair_desc[p];
       int a = d.b1 + nb * d.c1, b = d.b2 + nb * d.c2;
       list[fill[a]++] = p;
       if (b != a) list[fill[b]++] = p;
@@ -2000,20 +1999,38 @@ void alloc_sort(Ctx& c, PopHost& ph) {
     h.cp_off = d_off;
     h.cp_list = d_list;
   }
-  PairDesc* pd = dalloc<PairDesc>(c, o, std::max<size_t>(ph.pair_desc.size(), 1));
-  if (!ph.pair_desc.empty())
-    CK(cudaMemcpyAsync(pd, ph.pair_desc.data(), sizeof(PairDesc) * ph.pair_desc.size(),
+  PairDesc* pd = dalloc<PairDesc>(c, o, std::max<size_t>(pair_desc.size(), 1));
+  if (!pair_desc.empty())
+    CK(cudaMemcpyAsync(pd, pair_desc.data(), sizeof(PairDesc) * pair_desc.size(),
                        cudaMemcpyHostToDevice, c.stream));
   h.pair_desc = pd;
-  h.pair = dalloc<PairState>(c, o, std::max<size_t>(ph.pair_desc.size(), 1));
+  h.pair = dalloc<PairState>(c, o, std::max<size_t>(pair_desc.size(), 1));
   h.kmax_valid = 0;
   h.pair_setup_valid = 0;
+}
+
+// the population's sort structures for n_bin bins: new ones in the old ones'
+// place, or an error and the old ones stay
+void alloc_sort(Ctx& c, PopHost& ph, int n_bin) {
+  PopDev h = ph.h;
+  std::vector<void*> o;
+  try {
+    fill_sort(c, h, o, n_bin);
+  } catch (...) {
+    free_list(c, o);
+    throw;
+  }
+  ph.h = h;
+  o.swap(ph.sort_allocs);
+  free_list(c, o);
+  ph.n_bin = n_bin;
+  ph.chunk_hist_cap = 0;
   c.dirty = true;
 }
 
 // bin_grid_make (log) on the host, with glibc's log/exp like the reference
 void make_grid(Ctx& c, PopHost& ph, int n_bin, double rmin, double rmax) {
-  ph.n_bin = n_bin;
+  alloc_sort(c, ph, n_bin);
   ph.edges.assign(n_bin + 1, 0.0);
   ph.centers.assign(std::max(n_bin, 1), 0.0);
   if (n_bin > 0) {
@@ -2048,7 +2065,6 @@ void make_grid(Ctx& c, PopHost& ph, int n_bin, double rmin, double rmax) {
     for (int i = 0; i < n_bin; i++) g.centers[i] = ph.centers[i];
   }
   CK(cudaMemcpyAsync(ph.h.grid, &g, sizeof(GridDev), cudaMemcpyHostToDevice, c.stream));  // staged before it returns
-  alloc_sort(c, ph);
 }
 
 void set_params(Ctx& c, PopHost& ph) {
@@ -2080,36 +2096,43 @@ void init_pop(Ctx& c, PopHost& ph, int cap) {
   CK(cudaMemcpyAsync(dens, c.density.data(), sizeof(double) * c.n_spec, cudaMemcpyHostToDevice, c.stream));
   ph.h.density = dens;
   set_params(c, ph);
-  alloc_slots(c, ph, cap);
+  alloc_slots(c, ph.h, ph.slot_allocs, cap);
   PopCtr z{};
   ph.rm_count = 0;  // the population's removal records start empty
   z.next_id = 1;
   z.bmin = 1 << 30;
   z.bmax = -1;
   write_ctr(c, (int)(&ph - c.pops.data()), z);
-  ph.n_bin = 0;
   GridDev g{};
   CK(cudaMemcpyAsync(ph.h.grid, &g, sizeof(GridDev), cudaMemcpyHostToDevice, c.stream));
-  alloc_sort(c, ph);
+  alloc_sort(c, ph, 0);
 }
 
-// grow (compact = false, slot numbers kept) or compact (slot order kept)
+// grow (compact = false, slot numbers kept) or compact (slot order kept); on an
+// error the population keeps its arrays
 void relayout(Ctx& c, int k, int new_cap, bool compact) {
   PopHost& ph = c.pops[k];
   PopCtr r = read_ctr(c, k);
-  PopDev old = ph.h;
-  std::vector<void*> old_allocs;
-  old_allocs.swap(ph.slot_allocs);
-  alloc_slots(c, ph, new_cap);
-  std::vector<void*> tmp;
-  long long* off = dalloc<long long>(c, tmp, (size_t)r.n_slots + 1);
+  PopDev h = ph.h;
+  std::vector<void*> allocs, tmp;
   long long n_live = r.n_slots;
-  if (compact) n_live = scan(c, old.alive, r.n_slots, off, true);
-  if (r.n_slots > 0)
-    k_relayout<<<grid_for(r.n_slots, 256), 256, 0, c.stream>>>(old, ph.h, off, r.n_slots,
-                                                               compact ? 1 : 0); note_launch();
+  try {
+    alloc_slots(c, h, allocs, new_cap);
+    long long* off = dalloc<long long>(c, tmp, (size_t)r.n_slots + 1);
+    if (compact) n_live = scan(c, ph.h.alive, r.n_slots, off, true);
+    if (r.n_slots > 0) {
+      k_relayout<<<grid_for(r.n_slots, 256), 256, 0, c.stream>>>(ph.h, h, off, r.n_slots, compact ? 1 : 0);
+      note_launch();
+    }
+  } catch (...) {
+    free_list(c, tmp);
+    free_list(c, allocs);
+    throw;
+  }
+  ph.h = h;
+  allocs.swap(ph.slot_allocs);
   free_list(c, tmp);
-  free_list(c, old_allocs);
+  free_list(c, allocs);
   if (compact) {
     r.n_slots = (int)n_live;
     ph.mirror_full = true;  // slots renumbered
@@ -3306,11 +3329,7 @@ GraphRun run_round_graph(Ctx& c, int kt, bool flat, int n_gpairs, long long e0) 
   c.graph_stats.reserve(kStatWords);
   {
     const long long nb = (b.W + kScanTile - 1) / kScanTile;
-    c.scan_status.reserve((size_t)std::max(kScanMaxJobs * nb, b.W / kResolveMin + 2));
-    if (c.scan_status.n > c.scan_status_n) {
-      CK(cudaMemsetAsync(c.scan_status.p, 0, sizeof(unsigned long long) * c.scan_status.n, c.stream));
-      c.scan_status_n = c.scan_status.n;
-    }
+    reserve_scan_status(c, (size_t)std::max(kScanMaxJobs * nb, b.W / kResolveMin + 2), c.stream);
   }
   if (c.dirty) push_pops(c);
   std::vector<long long> key = round_graph_key(c, b);
@@ -3411,6 +3430,7 @@ int padded_pairs(long long n) { return (int)((n + 1023) / 1024 * 1024); }
 // global pair list, uploaded when its layout changes
 void upload_pair_layout(Ctx& c, const std::vector<long long>& base) {
   if (base == c.base_cached) return;
+  c.base_cached.clear();  // if a buffer does not fit
   const int n = padded_pairs(base[c.n_pop]);
   std::vector<int> gp_pop(std::max(n, 1), 0), gp_loc(std::max(n, 1), 0);
   for (int k = 0; k < c.n_pop; k++)
@@ -3656,10 +3676,10 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   reserve_round(c, b.W);
   c.pp_rm_tot.reserve(1);
   if (!c.report.p) {
-    c.report.reserve(16 * (size_t)report_words(c) + 64);
-    memset(c.report.p, 0, c.report.bytes);
     c.report_seq.reserve(1);
     CK(cudaMemsetAsync(c.report_seq.p, 0, sizeof(unsigned) * c.report_seq.n, c.stream));
+    c.report.reserve(16 * (size_t)report_words(c) + 64);
+    memset(c.report.p, 0, c.report.bytes);
   }
   if (q_cap > 0) {
     const long long q = std::max(q_cap, qb_cap);
@@ -3681,11 +3701,8 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
     const long long qs = std::max(q_cap, qb_cap), hist = (std::max(qs, q_cap > 0 ? b.W : 0) / kGrpTile + 2) * c.n_pop;
     const long long lists = std::max(std::max(kMaxCopies * qs, hist), (long long)b.n_gpairs);
     const long long nb = std::max((c.sg_w + kScanTile - 1) / kScanTile, (lists + kScanTile - 1) / kScanTile);
-    c.scan_status.reserve((size_t)std::max(std::max(kScanMaxJobs * nb, std::max(c.sg_w, b.W) / kResolveMin + 2), qs / 64 + 2));
-    if (c.scan_status.n > c.scan_status_n) {
-      CK(cudaMemsetAsync(c.scan_status.p, 0, sizeof(unsigned long long) * c.scan_status.n, c.stream));
-      c.scan_status_n = c.scan_status.n;
-    }
+    reserve_scan_status(
+        c, (size_t)std::max(std::max(kScanMaxJobs * nb, std::max(c.sg_w, b.W) / kResolveMin + 2), qs / 64 + 2), c.stream);
   }
   c.op_cap = qb_cap;
   if (c.prof)
@@ -4311,11 +4328,25 @@ int pmc_coag_gpu_upload(pmc_coag_gpu_ctx* x, int pop, int n_part, const double* 
   GUARD_BEGIN
   PopHost& ph = c.pops[pop];
   int cap = std::max(1024, n_part + n_part / 2 + 64);
-  if (cap > ph.h.cap || cap < ph.h.cap / 4) {
-    free_list(c, ph.slot_allocs);
-    alloc_slots(c, ph, cap);
-  }
   PopCtr r = read_ctr(c, pop);
+  if (cap > ph.h.cap || cap < ph.h.cap / 4) {
+    // the old arrays go first: there may not be room for both.  If the new ones
+    // do not fit, the population is left empty, without slots
+    free_list(c, ph.slot_allocs);
+    PopDev h = ph.h;
+    ph.h.cap = 0;
+    try {
+      alloc_slots(c, h, ph.slot_allocs, cap);
+    } catch (...) {
+      r.n_slots = r.n_live = 0;
+      write_ctr(c, pop, r);
+      ph.valid_sort = ph.caches_valid = c.replay.valid = false;
+      ph.mirror_full = true;
+      push_pops(c);
+      throw;
+    }
+    ph.h = h;
+  }
   CK(cudaMemsetAsync(ph.h.alive, 0, ph.h.cap, c.stream));
   CK(cudaMemsetAsync(ph.h.changed, 0, ph.h.cap, c.stream));
   ph.mirror_full = true;  // a host copy kept slot by slot must be refreshed in full
@@ -4356,12 +4387,16 @@ int pmc_coag_gpu_upload(pmc_coag_gpu_ctx* x, int pop, int n_part, const double* 
   ph.valid_sort = false;
   ph.caches_valid = false;
   c.replay.valid = false;
-  ph.n_bin = 0;
+  try {
+    alloc_sort(c, ph, 0);
+  } catch (...) {
+    push_pops(c);  // the slot arrays may be new
+    throw;
+  }
   {
     GridDev g{};
     CK(cudaMemcpyAsync(ph.h.grid, &g, sizeof(GridDev), cudaMemcpyHostToDevice, c.stream));
   }
-  alloc_sort(c, ph);
   push_pops(c);
   CK(cudaStreamSynchronize(c.stream));
   return PMC_OK;
