@@ -1482,6 +1482,7 @@ struct Ctx {
   cudaGraph_t sg_graph = nullptr;
   cudaGraphExec_t sg_exec = nullptr;
   std::vector<long long> sg_key, sg_seen;
+  int sg_pause = 0;                  // steps left that go the long way (kGraphPause)
   long long sg_w = 0, sg_e = 0;      // samples and items it holds room for
   long long sg_q = 0, sg_qb = 0;     // target operations of round 0 and of a later round
   long long sg_nodes0 = 0, sg_nodes = 0;  // launches of its round 0 and of one later round
@@ -3599,9 +3600,22 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
 }
 
 constexpr int kPPIdle = 8;  // steps
+constexpr int kGraphPause = 32;  // steps the long way after bounds that did not fit the device
 // least bound of a step's target operations: their buffers take 2 KB an
 // operation with the copies and walkers they may make
 constexpr long long kLeastOps = 512;
+
+// a step's buffers that hold nothing between steps
+void release_step_buffers(Ctx& c) {
+  auto release = [](auto&... b) { (b.release(), ...); };
+  release(c.flag, c.ev, c.ev_gp, c.ev_key, c.ev_c, c.gp_c, c.ev_pos, c.ev_dest, c.win_set, c.dec_set, c.ev_len,
+          c.ev_head, c.ev_app, c.ev_done, c.ev_term, c.chain_list, c.rank_slot_set, c.rank_id_set, c.ch_y, c.ch_q,
+          c.ch_pos);
+  release(c.it_flag, c.it_key, c.it_c, c.it_gp, c.it_pos, c.it_len, c.it_head, c.it_done, c.it_start, c.it_dec,
+          c.it_gused, c.it_term);
+  release(c.op_pop, c.op_pair, c.op_slot, c.op_k, c.op_key, c.r_pop, c.r_pair, c.r_slot, c.r_k, c.r_key, c.pp_res,
+          c.pp_vol, c.pp_rm_off, c.pp_rm_pool, c.wk_slot, c.wk_gp, c.wk_flag, c.ppw_slot, c.ppw_gp);
+}
 
 struct StepRun {
   bool ran = false;   // round 0 ran on the device
@@ -3625,6 +3639,10 @@ struct StepRun {
 StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   StepRun out;
   if (!c.use_graph || c.tuner.on || !c.ctrs_fresh || c.last_w < 0) return out;
+  if (c.sg_pause > 0) {
+    c.sg_pause--;
+    return out;
+  }
   if (c.claim_gen + 1 + (uint32_t)c.max_rounds + 2u >= kGenLimit) return out;  // the generations restart
   if (c.base_cached.size() != (size_t)c.n_pop + 1) return out;
   RoundBounds b;
@@ -3662,63 +3680,79 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   b.max_cells = (max_cells_of(c) + 15) / 16 * 16;
   b.max_chunks = (int)((slots + 4 * b.W + kMaxCopies * qb_cap + kChunk - 1) / kChunk);
   b.max_chunks = (b.max_chunks + 15) / 16 * 16;
-  prepare_chunks(c, (long long)b.max_chunks * kChunk - min_slots);
-  size_sort(c, b.max_cells);
-  // every buffer at its final size before the addresses are taken
-  const size_t ng = (size_t)b.n_gpairs + 1;
-  c.nwork_set.reserve(ng);
-  c.nwork_pp.reserve(ng);
-  c.work_off.reserve(ng);
-  c.pp_off.reserve(ng);
-  const size_t ws = (size_t)c.sg_w;
-  c.flag.reserve(ws + 1); c.ev.reserve(ws + 1); c.ev_gp.reserve(ws + 1);
-  reserve_events(c, std::max(c.sg_w + kMaxCopies * q_cap, b.W));
-  reserve_round(c, b.W);
-  c.pp_rm_tot.reserve(1);
-  if (!c.report.p) {
-    c.report_seq.reserve(1);
-    CK(cudaMemsetAsync(c.report_seq.p, 0, sizeof(unsigned) * c.report_seq.n, c.stream));
-    c.report.reserve(16 * (size_t)report_words(c) + 64);
-    memset(c.report.p, 0, c.report.bytes);
-  }
-  if (q_cap > 0) {
-    const long long q = std::max(q_cap, qb_cap);
-    reserve_ops(c, q);
-    reserve_redo(c, q);
-    c.ppw_slot.reserve((size_t)(kMaxCopies * (q + 1)));
-    c.ppw_gp.reserve((size_t)(kMaxCopies * (q + 1)));
-    if (c.n_pop > 1) {
-      c.item_pop.reserve((size_t)b.W + 1);
-      c.grp_dest.reserve((size_t)b.W + 1);
-      const size_t nh = (size_t)((b.W + kGrpTile - 1) / kGrpTile) * c.n_pop;
-      c.grp_hist.reserve(nh);
-      c.grp_off.reserve(nh + 1);
+  auto prepare = [&]() -> bool {
+    prepare_chunks(c, (long long)b.max_chunks * kChunk - min_slots);
+    size_sort(c, b.max_cells);
+    // every buffer at its final size before the addresses are taken
+    const size_t ng = (size_t)b.n_gpairs + 1;
+    c.nwork_set.reserve(ng);
+    c.nwork_pp.reserve(ng);
+    c.work_off.reserve(ng);
+    c.pp_off.reserve(ng);
+    const size_t ws = (size_t)c.sg_w;
+    c.flag.reserve(ws + 1); c.ev.reserve(ws + 1); c.ev_gp.reserve(ws + 1);
+    reserve_events(c, std::max(c.sg_w + kMaxCopies * q_cap, b.W));
+    reserve_round(c, b.W);
+    c.pp_rm_tot.reserve(1);
+    if (!c.report.p) {
+      c.report_seq.reserve(1);
+      CK(cudaMemsetAsync(c.report_seq.p, 0, sizeof(unsigned) * c.report_seq.n, c.stream));
+      c.report.reserve(16 * (size_t)report_words(c) + 64);
+      memset(c.report.p, 0, c.report.bytes);
     }
-    // twice the largest bound seen, so that it seldom grows
-    if (2 * c.last_rm + 1024 > (long long)c.pp_rm_pool.n) c.pp_rm_pool.reserve((size_t)(4 * c.last_rm + 65536));
-  }
-  {
-    const long long qs = std::max(q_cap, qb_cap), hist = (std::max(qs, q_cap > 0 ? b.W : 0) / kGrpTile + 2) * c.n_pop;
-    const long long lists = std::max(std::max(kMaxCopies * qs, hist), (long long)b.n_gpairs);
-    const long long nb = std::max((c.sg_w + kScanTile - 1) / kScanTile, (lists + kScanTile - 1) / kScanTile);
-    reserve_scan_status(
-        c, (size_t)std::max(std::max(kScanMaxJobs * nb, std::max(c.sg_w, b.W) / kResolveMin + 2), qs / 64 + 2), c.stream);
-  }
-  c.op_cap = qb_cap;
-  if (c.prof)
-    for (auto& ev : c.sg_ev)
-      if (!ev) CK(cudaEventCreate(&ev));
-  const std::vector<long long> key = step_graph_key(c, b, c.sg_w, max_pairs, q_cap, qb_cap);
-  if (key != c.sg_key) {
-    // captured when the bounds and addresses hold for two steps; at once where
-    // a step the long way costs several captures (about 1 ms each)
-    if (key != c.sg_seen && !c.pp_step) {
-      c.sg_seen = key;
-      return out;
+    if (q_cap > 0) {
+      const long long q = std::max(q_cap, qb_cap);
+      reserve_ops(c, q);
+      reserve_redo(c, q);
+      c.ppw_slot.reserve((size_t)(kMaxCopies * (q + 1)));
+      c.ppw_gp.reserve((size_t)(kMaxCopies * (q + 1)));
+      if (c.n_pop > 1) {
+        c.item_pop.reserve((size_t)b.W + 1);
+        c.grp_dest.reserve((size_t)b.W + 1);
+        const size_t nh = (size_t)((b.W + kGrpTile - 1) / kGrpTile) * c.n_pop;
+        c.grp_hist.reserve(nh);
+        c.grp_off.reserve(nh + 1);
+      }
+      // twice the largest bound seen, so that it seldom grows
+      if (2 * c.last_rm + 1024 > (long long)c.pp_rm_pool.n) c.pp_rm_pool.reserve((size_t)(4 * c.last_rm + 65536));
     }
+    {
+      const long long qs = std::max(q_cap, qb_cap), hist = (std::max(qs, q_cap > 0 ? b.W : 0) / kGrpTile + 2) * c.n_pop;
+      const long long lists = std::max(std::max(kMaxCopies * qs, hist), (long long)b.n_gpairs);
+      const long long nb = std::max((c.sg_w + kScanTile - 1) / kScanTile, (lists + kScanTile - 1) / kScanTile);
+      reserve_scan_status(
+          c, (size_t)std::max(std::max(kScanMaxJobs * nb, std::max(c.sg_w, b.W) / kResolveMin + 2), qs / 64 + 2), c.stream);
+    }
+    c.op_cap = qb_cap;
+    if (c.prof)
+      for (auto& ev : c.sg_ev)
+        if (!ev) CK(cudaEventCreate(&ev));
+    const std::vector<long long> key = step_graph_key(c, b, c.sg_w, max_pairs, q_cap, qb_cap);
+    if (key != c.sg_key) {
+      // captured when the bounds and addresses hold for two steps; at once where
+      // a step the long way costs several captures (about 1 ms each)
+      if (key != c.sg_seen && !c.pp_step) {
+        c.sg_seen = key;
+        return false;
+      }
+      CK(cudaStreamSynchronize(c.stream));  // a graph's report comes before its end
+      free_step_graph(c);
+      capture_step_graph(c, b, c.sg_w, max_pairs, q_cap, qb_cap);
+      c.sg_key = key;
+    }
+    return true;
+  };
+  try {
+    if (!prepare()) return out;
+  } catch (const Fail&) {
+    // the bounds do not fit the device: the long way needs less (an error that
+    // stays is its to report)
+    cudaGetLastError();
     free_step_graph(c);
-    capture_step_graph(c, b, c.sg_w, max_pairs, q_cap, qb_cap);
-    c.sg_key = key;
+    c.sg_seen.clear();
+    release_step_buffers(c);
+    c.sg_pause = kGraphPause;
+    return out;
   }
   // the sort's step_begin advances the device's step counts, which have to be
   // at the step before (a new seed restarts the host's; any call may have

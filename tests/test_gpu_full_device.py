@@ -1,5 +1,5 @@
 """A device with little memory left: a call whose memory does not fit is refused
-and the populations stay usable."""
+and the populations stay usable; a step that fits without its graph runs."""
 import numpy as np
 import pytest
 
@@ -89,5 +89,34 @@ def test_upload_that_does_not_fit(gpu_lib):
         s.add_particles(pop.vol, pop.group)
         s.set_seed(5)
         res.append(([f(1.0) for _ in range(5)], s.particles()))
+    assert res[0][0] == res[1][0]
+    same(res[0][1], res[1][1])
+
+
+def test_step_whose_graph_does_not_fit(gpu_lib):
+    """A step graph's bounds are the power of two above 1.25 of the last step's
+    samples, its host-run step's the one above the samples: with 1.7 to 2.1
+    million samples the graph's buffers take 2 GB, twice the others, which the
+    device has no room for here."""
+    import partmc_b200 as pm
+    import torch
+    from partmc_b200 import aero_dist
+    pop = aero_dist.brown_bimodal(2000000, seed=2)
+    env = pm.EnvState(288.0, 1e5)
+    res = []
+    for full in (False, True):
+        st = pm.AeroState(pop.aero_data, pop.awa, seed=3)
+        st.add_particles(pop.vol, pop.group)
+        counts = [pm.mc_coag(pm.COAG_KERNEL_TYPE_BROWN, env, pop.aero_data, st, dt) for dt in (600.0, 37000.0)]
+        assert 2 ** 21 / 1.25 < counts[1][0] < 2.05 * 2 ** 20
+        if full:
+            with Full(300 << 20):
+                counts += [pm.mc_coag(pm.COAG_KERNEL_TYPE_BROWN, env, pop.aero_data, st, 20000.0) for _ in range(2)]
+        else:
+            counts += [pm.mc_coag(pm.COAG_KERNEL_TYPE_BROWN, env, pop.aero_data, st, 20000.0) for _ in range(2)]
+        counts += [pm.mc_coag(pm.COAG_KERNEL_TYPE_BROWN, env, pop.aero_data, st, 600.0) for _ in range(40)]
+        res.append((counts, st.particles()))
+        del st
+        torch.cuda.synchronize()
     assert res[0][0] == res[1][0]
     same(res[0][1], res[1][1])
