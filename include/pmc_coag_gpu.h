@@ -299,9 +299,11 @@ int pmc_coag_gpu_set_mode(pmc_coag_gpu_ctx *ctx, int mode);
  * the particles the step made, chains) a loop whose condition is set on the
  * device (enable = 1, the default), or every launch from the host (enable =
  * 0).  Both give the same particles, bit for bit.  The first steps of a
- * population, and a step that outgrows the graph's bounds or changes the
- * grid, run from the host (their later rounds as a graph where no
- * per-particle operations run).
+ * population, a step that outgrows the graph's bounds or changes the grid or
+ * the environment, and the step after a call that changes a population's
+ * particles or counters (uploads, rebalancing, sampling, weights, IDs,
+ * reading removal records) run from the host, their later rounds as a graph
+ * where no per-particle operations run and the calls come back step for step.
  * No counterpart in the reference (an execution choice). */
 int pmc_coag_gpu_set_graphs(pmc_coag_gpu_ctx *ctx, int enable);
 

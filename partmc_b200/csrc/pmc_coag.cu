@@ -1487,7 +1487,6 @@ struct Ctx {
   long long sg_q = 0, sg_qb = 0;     // target operations of round 0 and of a later round
   long long sg_nodes0 = 0, sg_nodes = 0;  // launches of its round 0 and of one later round
   cudaEvent_t sg_ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // when profiling: sort, tests, later rounds
-  bool sg_prof = false;              // the captured graph records them
   long long* d_stat = nullptr;       // kStatWords words before the counter blocks, read back with them
   // the last step's samples, largest items and target operations of a later
   // round, target operations of round 0 and largest removal bound
@@ -2193,9 +2192,9 @@ __global__ void k_radius_minmax_masked(const PopDev* pops, const uint8_t* on) {
 }
 
 
-// chunk counts from the host's copy of the slot counts
-// chunk histograms for the current slot counts plus extra slots per
-// population (the growth a device-driven loop may add before the host looks)
+// chunk counts and histograms for the host's copy of the slot counts plus extra
+// slots per population (the growth a device-driven loop may add before the
+// host looks)
 void prepare_chunks(Ctx& c, long long extra = 0) {
   for (int k = 0; k < c.n_pop; k++) {
     PopHost& ph = c.pops[k];
@@ -2211,9 +2210,7 @@ void prepare_chunks(Ctx& c, long long extra = 0) {
   }
 }
 
-// one cooperative launch of k_sort_all on a persistent grid of co-resident
-// blocks, for chunk and cell counts up to max_chunks and max_cells
-// co-resident blocks of the sort for max_cells cells (its shared memory)
+// co-resident blocks of the sort for max_cells cells, and its shared memory
 size_t size_sort(Ctx& c, int max_cells) {
   size_t smem = sizeof(int) * ((kSortWarps + 1) * (size_t)max_cells + (c.n_pop <= kSortMapPops ? c.n_pop + 1 : 0));
   if (smem != c.sort_smem) {
@@ -2226,6 +2223,8 @@ size_t size_sort(Ctx& c, int max_cells) {
   return smem;
 }
 
+// one cooperative launch of k_sort_all on a persistent grid of co-resident
+// blocks, for chunk and cell counts up to max_chunks and max_cells
 void launch_sort(Ctx& c, cudaStream_t st, int max_chunks, int max_cells, const StepBegin& begin = StepBegin{}) {
   size_t smem = size_sort(c, max_cells);
   long long items = (long long)c.n_pop * max_chunks;
@@ -2528,7 +2527,7 @@ void launch_items_kt(Ctx& c, int kt, bool flat, int n_gpairs, long long W, cudaS
 
 // Stable grouping by population of a batched context's per-round lists.
 // Slot and ID ranks come from one scan over a list, and the per-population
-// bases of k_alloc_bases assume that each population's entries lie together
+// bases of alloc_bases assume that each population's entries lie together
 // and in population order.  Round 0's samples and target operations are
 // built that way; later rounds add entries from every population at the end
 // (the walkers of target operations, and the target operations that walks
@@ -2876,8 +2875,10 @@ __global__ void k_pop_work(const long long* pop_pair_base, int n_pop, const long
 // statistics and sets the loop condition: events in this round, fewer than
 // max_rounds rounds, and room in every population for the next round's new
 // slots, in the slot arrays and in the sort's chunks.  Without room the
-// graph stops and the host loop, which can grow both, carries on.  Rounds
-// with per-particle redo operations run from the host loop.
+// graph stops and the host loop, which can grow both, carries on.  A step
+// graph's rounds take target operations too, their tail an IF node
+// (k_pp_fits); in a step that the host begins, rounds with target operations
+// run from the host loop.
 
 __device__ void round_begin(uint32_t* d_round, long long* round_dev, int* per_pop, int n_per_pop, long long* n_dev) {
   if (threadIdx.x == 0) {
@@ -3029,8 +3030,8 @@ __global__ void __launch_bounds__(1024) k_step_report(const uint4* stat, int n16
 }
 
 // Resolve and apply the events of a round (E at round_dev[1], at most W) and,
-// with Q > 0 (host loop only), its Q target operations.  chains: the round may
-// have chains (every round but the first).
+// with Q > 0, its target operations (n_dev[1] of them, at most Q).  chains: the
+// round may have chains (every round but the first).
 void resolve_apply(Ctx& c, cudaStream_t st, long long W, long long Q, bool chains) {
   long long* Ed = c.round_dev.p + 1;
   ChainPool pool = chain_pool(c);
@@ -3456,12 +3457,12 @@ void free_step_graph(Ctx& c) {
   c.sg_key.clear();
 }
 
-// what the step graph's captured launches depend on, beyond round_graph_key
 // 16-byte words of the step graph's report
 int report_words(const Ctx& c) {
   return (int)((sizeof(long long) * kStatWords + sizeof(PopCtr) * c.n_pop + 15) / 16);
 }
 
+// what the step graph's captured launches depend on, beyond round_graph_key
 std::vector<long long> step_graph_key(const Ctx& c, const RoundBounds& b, long long w_cap, int max_pairs,
                                       long long q_cap, long long qb_cap) {
   std::vector<long long> k = round_graph_key(c, b);
@@ -3730,7 +3731,8 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
     const std::vector<long long> key = step_graph_key(c, b, c.sg_w, max_pairs, q_cap, qb_cap);
     if (key != c.sg_key) {
       // captured when the bounds and addresses hold for two steps; at once where
-      // a step the long way costs several captures (about 1 ms each)
+      // a step the long way, with its host-driven rounds, costs several captures
+      // (0.2 to 0.3 ms each)
       if (key != c.sg_seen && !c.pp_step) {
         c.sg_seen = key;
         return false;
@@ -3883,7 +3885,7 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
   // round_dev: [0] losers, [1] events, [2] items, [3] chain chunks, [4] chains,
   // [5] walkers of target operations, [6] items that are events, [7] items
   // that are such walkers, [8] target operations that lost a claim,
-  // [9] places of their walkers, [10] chains that k_chain carries on
+  // [10] chains that k_chain carries on
   c.round_dev.reserve(12);
   int max_pairs = 1, nb_max = 1, max_cap = 1;
   for (int k = 0; k < c.n_pop; k++) {
@@ -3966,10 +3968,10 @@ void step_parallel(Ctx& c, int kt, bool params_same) {
       hw[3] = W;
       hw[4] = Q;
     }
-    // a step with target operations runs its later rounds from the host,
-    // where walks that reach a per-particle pair's target cell stop for one;
-    // a population's walks stop when it has target operations of its own,
-    // so it steps the same alone and in a batch
+    // in a step with target operations walks that reach a per-particle pair's
+    // target cell stop for one; a population's walks stop when it has target
+    // operations of its own, so it steps the same alone and in a batch (in a
+    // step graph k_step_check sets this)
     c.pp_step = Q > 0;
     c.pp_idle = 0;
     for (int k = 0; k < c.n_pop; k++) {

@@ -17,8 +17,8 @@
 //             priority (its position in the reference's loop order);
 //   resolve   an accepted sample that holds both claims is applied
 //             (coagulate / coagulate_weighting, coagulation.F90:810-985).
-// Later rounds (k_items, one thread per event of the round before) carry on
-// the sequential loop's order:
+// Later rounds (k_items: a warp, or with more of them a thread, per event of
+// the round before) carry on the sequential loop's order:
 //   - an event that lost a claim is retried unchanged if neither of its
 //     particles was consumed, and dropped if one was: in the sequential loop
 //     a test never meets a particle that an earlier event removed, so the

@@ -1685,10 +1685,9 @@ __global__ void __launch_bounds__(32) k_apply_chain(const PopDev* pops, const in
 // pairs on the per-particle path add nothing.  One block per cell, its
 // threads over the cell's pairs, a block-wide scan in a fixed order.
 // P.walk_stops: 1 when the population's round 0 has target operations (the
-// step's later rounds then run from the host and take the operations that
-// walks stop for); with 0, its per-particle pairs (whose target cells were
-// all empty at the step's start) are walked at the per-set rate like any
-// pair.
+// step's later rounds then take the operations that walks stop for); with 0,
+// its per-particle pairs (whose target cells were all empty at the step's
+// start) are walked at the per-set rate like any pair.
 __global__ void __launch_bounds__(128) k_walk_rates(const PopDev* pops) {
   chain_wait();
   const PopDev& P = pops[blockIdx.y];

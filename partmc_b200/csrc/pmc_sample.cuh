@@ -252,11 +252,10 @@ __global__ void k_select_hist(PopDev P, int g, int c, uint32_t call, SelectState
   }
 }
 
-// one block of 1024 threads: thread t owns bins [64 t, 64 t + 64)
-// A warp takes 2048 bins of the digit, 64 a lane in registers (16 words of 16
-// bytes, read in order across the warp); the warp whose bins hold the wanted
-// rank finds the bin by warp scans.  A thread's 64 bins one after another,
-// read with a stride of 256 bytes, took 72 us; now 21.
+// One block of 1024 threads.  A warp takes 2048 bins of the digit, 64 a lane in
+// registers (16 words of 16 bytes, read in order across the warp); the warp
+// whose bins hold the wanted rank finds the bin by warp scans.  A thread's 64
+// bins one after another, read with a stride of 256 bytes, took 72 us; now 21.
 __global__ void __launch_bounds__(1024) k_select_pick(SelectState* S, int shift) {
   constexpr unsigned kFull = 0xffffffffu;
   __shared__ long long before_sh[33];
