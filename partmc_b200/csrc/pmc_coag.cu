@@ -1375,6 +1375,7 @@ struct PopHost {
   std::vector<void*> slot_allocs;
   std::vector<void*> sort_allocs;
   std::vector<void*> fixed_allocs;
+  PopDev none{};  // its sort structures, those of no bins, stay for good (fixed_allocs)
   uint64_t seed = 1;
   uint32_t step = 0;
   uint32_t dev_step = 0;  // the step count of the device's copy of h
@@ -2009,23 +2010,58 @@ void fill_sort(Ctx& c, PopDev& h, std::vector<void*>& o, int n_bin) {
   h.pair_setup_valid = 0;
 }
 
-// the population's sort structures for n_bin bins: new ones in the old ones'
-// place, or an error and the old ones stay
+// the sort structures of src (fill_sort) as dst's
+void take_sort(PopDev& dst, const PopDev& src) {
+  dst.n_cells = src.n_cells;
+  dst.chunk_hist = src.chunk_hist;
+  dst.chunk_hist_len = src.chunk_hist_len;
+  dst.cell_count = src.cell_count;
+  dst.cell_start = src.cell_start;
+  dst.kmax_tab = src.kmax_tab;
+  dst.n_pairs = src.n_pairs;
+  dst.cp_off = src.cp_off;
+  dst.cp_list = src.cp_list;
+  dst.cp_cum = src.cp_cum;
+  dst.cp_ent = src.cp_ent;
+  dst.cp_nstop = src.cp_nstop;
+  dst.cp_tab = src.cp_tab;
+  dst.cp_coarse = src.cp_coarse;
+  dst.n_coarse = src.n_coarse;
+  dst.pair_desc = src.pair_desc;
+  dst.pair = src.pair;
+  dst.kmax_valid = 0;
+  dst.pair_setup_valid = 0;
+}
+
+// no grid, with the sort structures that stay
+void no_grid(Ctx& c, PopHost& ph) {
+  free_list(c, ph.sort_allocs);
+  take_sort(ph.h, ph.none);
+  ph.n_bin = 0;
+  ph.chunk_hist_cap = 0;
+  c.dirty = true;
+  GridDev g{};
+  CK(cudaMemcpyAsync(ph.h.grid, &g, sizeof(GridDev), cudaMemcpyHostToDevice, c.stream));  // staged before it returns
+}
+
+// the population's sort structures for n_bin bins, or an error and no grid
+// (the old ones go first: the pool then hands out the same blocks; new ones
+// first made an upload and an emptying of one of 256 populations 15 us longer)
 void alloc_sort(Ctx& c, PopHost& ph, int n_bin) {
+  no_grid(c, ph);
+  if (n_bin == 0) return;
   PopDev h = ph.h;
   std::vector<void*> o;
   try {
     fill_sort(c, h, o, n_bin);
   } catch (...) {
     free_list(c, o);
+    ph.valid_sort = ph.caches_valid = false;
     throw;
   }
-  ph.h = h;
-  o.swap(ph.sort_allocs);
-  free_list(c, o);
+  take_sort(ph.h, h);
+  ph.sort_allocs = o;
   ph.n_bin = n_bin;
-  ph.chunk_hist_cap = 0;
-  c.dirty = true;
 }
 
 // bin_grid_make (log) on the host, with glibc's log/exp like the reference
@@ -2103,9 +2139,9 @@ void init_pop(Ctx& c, PopHost& ph, int cap) {
   z.bmin = 1 << 30;
   z.bmax = -1;
   write_ctr(c, (int)(&ph - c.pops.data()), z);
-  GridDev g{};
-  CK(cudaMemcpyAsync(ph.h.grid, &g, sizeof(GridDev), cudaMemcpyHostToDevice, c.stream));
-  alloc_sort(c, ph, 0);
+  ph.none = ph.h;
+  fill_sort(c, ph.none, o, 0);
+  no_grid(c, ph);
 }
 
 // grow (compact = false, slot numbers kept) or compact (slot order kept); on an
@@ -4423,16 +4459,7 @@ int pmc_coag_gpu_upload(pmc_coag_gpu_ctx* x, int pop, int n_part, const double* 
   ph.valid_sort = false;
   ph.caches_valid = false;
   c.replay.valid = false;
-  try {
-    alloc_sort(c, ph, 0);
-  } catch (...) {
-    push_pops(c);  // the slot arrays may be new
-    throw;
-  }
-  {
-    GridDev g{};
-    CK(cudaMemcpyAsync(ph.h.grid, &g, sizeof(GridDev), cudaMemcpyHostToDevice, c.stream));
-  }
+  no_grid(c, ph);
   push_pops(c);
   CK(cudaStreamSynchronize(c.stream));
   return PMC_OK;
