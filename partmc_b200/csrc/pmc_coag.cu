@@ -3282,9 +3282,9 @@ void free_redraw_graph(Ctx& c) {
 }
 
 // the item and event bound of the later rounds' graph for round-0 events
-// e0: a power of two, at least `least`, so that it holds from step to step
-long long graph_bound(long long e0, long long least = 4096) {
-  long long w = least;
+// e0: a power of two, at least 4096, so that it holds from step to step
+long long graph_bound(long long e0) {
+  long long w = 4096;
   while (w < e0) w *= 2;
   return w;
 }
@@ -3638,9 +3638,6 @@ void capture_step_graph(Ctx& c, const RoundBounds& b, long long w_cap, int max_p
 
 constexpr int kPPIdle = 8;  // steps
 constexpr int kGraphPause = 32;  // steps the long way after bounds that did not fit the device
-// least bound of a step's target operations: their buffers take 2 KB an
-// operation with the copies and walkers they may make
-constexpr long long kLeastOps = 512;
 
 // a step's buffers that hold nothing between steps
 void release_step_buffers(Ctx& c) {
@@ -3705,7 +3702,7 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   long long q_cap = 0, qb_cap = 0;
   if (c.pp_step) {
     // room for twice as many when they outgrow it
-    const long long q = graph_bound(c.last_q + c.last_q / 4, kLeastOps), qb = graph_bound(c.last_qb + c.last_qb / 4, kLeastOps);
+    const long long q = graph_bound(c.last_q + c.last_q / 4), qb = graph_bound(c.last_qb + c.last_qb / 4);
     if (q > c.sg_q || 16 * q <= c.sg_q) c.sg_q = 2 * q;
     if (qb > c.sg_qb || 16 * qb <= c.sg_qb) c.sg_qb = 2 * qb;
     q_cap = c.sg_q;
@@ -3830,8 +3827,8 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   memcpy(stat, report, sizeof(stat));
   c.last_w = stat[5];
   // target operations may come and go from step to step: their bounds follow
-  // a fall by an eighth a step, a rise at once
-  c.last_q = std::max(stat[12], c.last_q - c.last_q / 8);
+  // a fall by half a step, a rise at once
+  c.last_q = std::max(stat[12], c.last_q / 2);
   c.last_rm = std::max(c.last_rm, stat[11]);
   if (stat[4]) {
     c.ctrs_fresh = false;
@@ -3857,7 +3854,7 @@ StepRun run_step_graph(Ctx& c, int kt, bool params_same) {
   g_launches += c.sg_nodes0 + c.sg_nodes * (stat[2] - 1);
   c.claim_gen += (uint32_t)(stat[2] + (stat[3] == 2 ? 1 : 0));  // a round left in the middle has begun
   c.last_e0 = stat[7];
-  c.last_qb = std::max(stat[8], c.last_qb - c.last_qb / 8);
+  c.last_qb = std::max(stat[8], c.last_qb / 2);
   for (int k = 0; k < c.n_pop; k++) c.pops[k].h.walk_stops = c.h_ctrs[k].walk_stops;
   // without target operations for a while, back to the graph without them
   c.pp_idle = stat[12] > 0 ? 0 : c.pp_idle + 1;
