@@ -1635,7 +1635,10 @@ cudaMemPool_t pool_acquire(int dev) {
   DevicePools& d = device_pools();
   std::lock_guard<std::mutex> l(d.mu);
   if ((int)d.by_dev.size() <= dev) d.by_dev.resize(dev + 1, {nullptr, 0});
-  if (!d.page) CK(cudaHostAlloc(&d.page, 4096, cudaHostAllocMapped));
+  if (!d.page && cudaHostAlloc(&d.page, 4096, cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();  // a saving only
+    d.page = nullptr;
+  }
   auto& e = d.by_dev[dev];
   if (!e.first) {
     cudaMemPoolProps mp = {};
